@@ -26,6 +26,8 @@
 #include <type_traits>
 #include <vector>
 
+#include <cuda_fp16.h>
+
 #include "tcr_common.cuh"
 #include "tcr_scan.cuh"
 #include "tcr_sort.cuh"
@@ -128,7 +130,7 @@ struct Scratch {
     int64_t* info;          // [8] see tcr_count
     int32_t* num_flagged;   // [1]
     int32_t* exact_clouds;  // [1] clouds whose every pair takes the exact test
-    int32_t* num_exact;     // [1] units the count walk re-tested with exact decisions
+    int32_t* num_exact;     // [1] pairs inside the count walk's band, decided exactly
     int32_t* unit_cap;      // [1] queries per work unit of this search (set by the count phase)
     unsigned long long* cursor;  // [1] staging fill
     float4* pack;           // [max(nq,nr)] packed input points before sorting
@@ -649,12 +651,14 @@ __device__ __forceinline__ void map_insert(unsigned long long* map, int64_t cap,
 }
 
 __device__ __forceinline__ int32_t map_find(const unsigned long long* __restrict__ map, int64_t cap, int32_t lin) {
-    uint64_t slot = mix32((uint32_t)lin) & (cap - 1);
-    for (int64_t probe = 0; probe < cap; ++probe) {
-        unsigned long long e = __ldg(&map[slot]);
-        if (e == ~0ull) return -1;
-        if ((uint32_t)(e >> 32) == (uint32_t)lin) return (int32_t)(uint32_t)e;
-        slot = (slot + 1) & (cap - 1);
+    const uint32_t mask = (uint32_t)(cap - 1);  // capacities are at most 2^32
+    uint32_t slot = mix32((uint32_t)lin) & mask;
+    for (uint32_t probe = 0; probe <= mask; ++probe) {
+        const uint2 e = __ldg(reinterpret_cast<const uint2*>(map) + slot);  // (cell, lin)
+        if (e.y == (uint32_t)lin && (int32_t)e.x >= 0) return (int32_t)e.x;
+        if (e.x == 0xffffffffu && e.y == 0xffffffffu) return -1;
+        if (probe == 0xffffffffu) return -1;
+        slot = (slot + 1) & mask;
     }
     return -1;
 }
@@ -1019,6 +1023,16 @@ __device__ __noinline__ bool f64_pair_decide(F64Walk f, int dim, int mask, int m
     return f64_pair_test(dim, mask, mode, f.ext, xi, f.qsup ? f.qsup[qi] : 0.0, xj, c.w);
 }
 
+// The tensor-core test's constants (see split_pair): the band relative to the largest product, the
+// largest scaled support it takes, the scaled distance beyond which a candidate sends its unit to
+// fix_unit, the scaled place of the lanes past a unit's candidates (farther than any support), and the
+// norm of a query row that must never hit.
+constexpr float kMmaBand = 4e-6f;
+constexpr float kMmaSupport = 4.0f;
+constexpr float kMmaReach = 16.0f;
+constexpr float kMmaPad = 15.0f;
+constexpr float kMmaFar = 60000.0f;
+
 // The unit's cloud, as the walk kernels read it (shared memory, warp-uniform).
 struct UnitCtx {
     int32_t cloud, dim, periodic_mask, dedupe;
@@ -1029,8 +1043,15 @@ struct UnitCtx {
     float dmin[3], hcell[3], ext[3];
     float rmax, qmax;        // largest reference / query support (band of the fast test)
     float f64_err;           // float64 inputs: bound on the error of a float32 coordinate difference
-    int32_t shift_ok;        // periodic dims all hold >= 6 cells: candidates across a seam are shifted
+    int32_t shift_ok;        // the periodic dims hold enough cells: candidates across a seam are shifted
     float shift_delta;       // bound on the error a shift adds to a difference
+    // the tensor-core test: power-of-two scale that puts the largest cell edge (scale_cell) in [1, 2), the
+    // half width of the band its result must leave (in scaled units; mma_seam more for shifted
+    // candidates), and whether every support is in its range
+    float scale, scale_cell, mma_band, mma_seam;
+    int32_t mma_ok;
+    int32_t plain_cells;  // every point lies in the grid and linear indices do not wrap: an in-range cell's linear
+                          // index names that cell only, so its bucket needs no check
     int64_t map_base, map_cap;
 };
 
@@ -1069,7 +1090,8 @@ struct WalkArgs {
     int32_t* rec;                 // [units] offset of each unit's record in the staging list, -1 if not staged
     int32_t* flagged;             // [units] units to re-walk in the emit pass
     int32_t* num_flagged;
-    int32_t* num_exact;           // units re-tested with exact decisions
+    int32_t* num_exact;           // pairs inside the product's band, decided after the walk
+    int4* band_pairs;             // [nq] (sorted query, sorted reference, mask word of the staging list, bit)
     unsigned long long* cursor;   // staging list fill
     int32_t* stage;               // staging list
     int64_t stage_cap;
@@ -1106,15 +1128,18 @@ __device__ __forceinline__ void load_unit_ctx(UnitCtx& u, const WalkArgs& a, int
     u.rmax = key_float(g.ref_stats.max_key);
     u.qmax = q.qmax;
     // Points of a stencil cell across the periodic seam can be moved by +-ext while staged, so
-    // the fast test needs no wrap: with >= 6 cells on every periodic dimension no candidate is near
-    // half the extent away, so the reference's moduloOp wraps exactly the shifted cells.  A shift
+    // the fast test needs no wrap: with >= 5 cells on every periodic dimension no candidate of the stencil
+    // (at most two cells away) is near half the extent away, so the reference's moduloOp wraps exactly
+    // the shifted cells; with 4 cells the two differ only for candidates at least 2 cells away, beyond
+    // every threshold when those stay below 1.5 cells.  A shift
     // changes a difference by at most one rounding of the shifted coordinate plus the reference's
     // own rounding of q - c before its exact wrap: shift_delta bounds both.
     bool ok = cp.periodic_mask != 0;
     float delta = 0.0f;
+    const float tmax = fmaxf(a.mode == kScatter ? 0.0f : u.qmax, a.mode == kGather ? 0.0f : u.rmax);
     for (int d = 0; d < cp.dim; ++d)
         if ((cp.periodic_mask >> d) & 1) {
-            ok = ok && g.count[d] >= 6;
+            ok = ok && (g.count[d] >= 5 || (g.count[d] == 4 && tmax <= 1.5f * g.hcell_d[d]));
             // two roundings of magnitude <= half an ulp of (|coordinate| + ext) each: <= 2^-23 of it
             delta = fmaxf(delta, (fmaxf(fabsf(cp.dmin[d]), fabsf(cp.dmax[d])) + cp.ext[d]) * 1.1920928955078125e-7f);
         }
@@ -1125,6 +1150,21 @@ __device__ __forceinline__ void load_unit_ctx(UnitCtx& u, const WalkArgs& a, int
     // a float32 copy of a double coordinate x is off by <= |x| 2^-24, the float difference adds one
     // rounding: 2^-21 of the largest |coordinate| bounds a difference's error with room to spare
     u.f64_err = a.f64.qpos ? key_float(q.coord_key) * 4.76837158203125e-7f : 0.0f;
+    double cells = 1.0;
+    for (int d = 0; d < cp.dim; ++d) cells *= (double)max(g.count[d], 1);
+    u.plain_cells = !g.out_of_grid && cells < 2147483648.0;
+    float cell = 0.0f;
+    for (int d = 0; d < cp.dim; ++d) cell = fmaxf(cell, g.hcell_d[d]);
+    const uint32_t ex = min(max((__float_as_uint(cell) >> 23) & 0xffu, 1u), 253u);
+    u.scale = __uint_as_float((254u - ex) << 23);
+    u.scale_cell = cell * u.scale;
+    // |Q| is at most sqrt(3) * 0.55 cells, a candidate near the threshold at most that plus thr away
+    const float hq = a.mode == kScatter ? 0.0f : u.qmax * u.scale, hc = a.mode == kGather ? 0.0f : u.rmax * u.scale;
+    const float t = a.mode == kSymmetric ? 0.5f * (hq + hc) : fmaxf(hq, hc);
+    const float e = fmaf(0.96f, u.scale_cell, t), fe = u.f64_err * u.scale, dl = u.shift_delta * u.scale;
+    u.mma_band = kMmaBand * e * e + kBandEps * t * t + fmaf(2.0f * 1.7320508f * t, fe, 3.0f * fe * fe);
+    u.mma_seam = fmaf(2.0f * t, dl, dl * dl);
+    u.mma_ok = !u.exact_all && hq <= kMmaSupport && hc <= kMmaSupport && u.scale_cell >= 1.0f && u.scale_cell <= 2.0f;
 }
 
 __device__ __forceinline__ ExactCtx unit_exact_ctx(const UnitCtx& u, int mode) {
@@ -1139,36 +1179,49 @@ __device__ __forceinline__ ExactCtx unit_exact_ctx(const UnitCtx& u, int mode) {
 }
 
 // Looks up stencil cell `o` (getOffsets order, last coordinate fastest) around cell gc with the
-// reference's semantics; returns the sorted range or an empty one.
+// reference's semantics; returns the sorted range or an empty one, inside the sorted points.
+template <int DIM>
 __device__ __forceinline__ void stencil_lookup(const WalkArgs& a, const UnitCtx& u, const int32_t* gc, int o,
                                                int32_t& beg, int32_t& cnt) {
     int32_t c[3] = {0, 0, 0};
     int rem = o;
-    bool dup = false;
-    for (int d = u.dim - 1; d >= 0; --d) {
+    bool dup = false, inside = true;
+#pragma unroll
+    for (int d = DIM - 1; d >= 0; --d) {
         const int32_t off = rem % 3 - 1;
         rem /= 3;
         int32_t v = gc[d] + off;
+        const int32_t n = u.count[d];
         if ((u.periodic_mask >> d) & 1) {
-            const int32_t n = u.count[d];
-            v = pymod(v, n);
+            // a neighbour of a cell inside the grid wraps by one extent at most
+            const int32_t v1 = v < 0 ? v + n : (v >= n ? v - n : v);
+            v = (uint32_t)v1 < (uint32_t)n ? v1 : pymod(v, n);
             // with fewer than 3 cells the wrapped offsets repeat a cell; the clamped grid visits it once
             if (u.dedupe && ((n == 1 && off != 0) || (n == 2 && off == 1))) dup = true;
-        } else if (u.dedupe && (v < 0 || v >= u.count[d])) {
+        } else if (u.dedupe && (v < 0 || v >= n)) {
             dup = true;  // clamped grid: nothing lies outside it
         }
+        inside &= (uint32_t)v < (uint32_t)n;
         c[d] = v;
     }
     beg = 0;
     cnt = 0;
     if (dup) return;
-    const int32_t lin = linear_index(u.dim, c, u.count);
+    const int32_t lin = linear_index(DIM, c, u.count);
     const int32_t cell = map_find(a.map + u.map_base, u.map_cap, lin);
     if (cell < 0 || !TCR_GUARD(cell, a.nr_total)) return;
+    const int32_t b = __ldg(&a.cell_start[cell]), e = __ldg(&a.cell_start[cell + 1]);
     // queryHashMap matches the linear index inside bucket hash(c) only.
-    if ((uint32_t)__ldg(&a.cell_bucket[cell]) != ref_hash(u.dim, c, u.hash_len)) return;
-    beg = __ldg(&a.cell_start[cell]);
-    cnt = __ldg(&a.cell_start[cell + 1]) - beg;
+    if (!(inside && u.plain_cells) && (uint32_t)__ldg(&a.cell_bucket[cell]) != ref_hash(DIM, c, u.hash_len)) return;
+    if (b < 0 || e < b || e > a.nr_total) return;
+    beg = b;
+    cnt = e - b;
+}
+__device__ __forceinline__ void stencil_lookup_any(const WalkArgs& a, const UnitCtx& u, const int32_t* gc, int o,
+                                                   int32_t& beg, int32_t& cnt) {
+    if (u.dim == 1) stencil_lookup<1>(a, u, gc, o, beg, cnt);
+    else if (u.dim == 2) stencil_lookup<2>(a, u, gc, o, beg, cnt);
+    else stencil_lookup<3>(a, u, gc, o, beg, cnt);
 }
 
 template <int DIM>
@@ -1251,16 +1304,15 @@ __device__ __forceinline__ void lean_test(const WrapCtx& wc, const float4& q, co
 }
 
 constexpr int kWalkWarps = 4;
-// Resident blocks per SM the count walk is compiled for (registers <= 65536 / (128 * blocks)):
-// eight (64 registers) on non-periodic clouds and seven (72) on periodic ones.  More resident
-// warps beat the spills they cost: on the 1M workload 8/7/6/5/4 blocks measured
-// 0.348/0.355/0.363/0.372/0.385 ms non-periodic, 8/7/6/5/4 blocks 0.414/0.403/0.426/0.436/0.467 ms
-// periodic.
+// Resident blocks per SM the count walk is compiled for (registers <= 65536 / (128 * blocks)): seven
+// (72 registers) on non-periodic clouds, six (80) on periodic ones.  8/7/6 blocks measured
+// 239/216/219 us on the 1M workload, 168/162/163 us for 131k queries against it, 42/39/37 us on 65k periodic
+// points and 1274/1168/1098 us on the periodic 3D clouds of a batch of 256.
 #ifndef TCR_WALK_MIN_BLOCKS
-#define TCR_WALK_MIN_BLOCKS 8
+#define TCR_WALK_MIN_BLOCKS 7
 #endif
 #ifndef TCR_WALK_MIN_BLOCKS_PERIODIC
-#define TCR_WALK_MIN_BLOCKS_PERIODIC 7
+#define TCR_WALK_MIN_BLOCKS_PERIODIC 6
 #endif
 constexpr int kWalkMinBlocks = TCR_WALK_MIN_BLOCKS;
 constexpr int kWalkMinBlocksPeriodic = TCR_WALK_MIN_BLOCKS_PERIODIC;
@@ -1278,29 +1330,18 @@ __host__ __device__ __forceinline__ int64_t record_words(int32_t runs, int32_t n
     return kRecHeader + 2 * (int64_t)runs + 1 + (int64_t)nchunks * nb;
 }
 
+constexpr int kWalkWin = 1024;  // candidates whose runs are laid out at a time
 struct WalkSmem {
-    float4 q[kWalkWarps][32];        // the unit's queries: x, y, z and the query's share of the test
-    float4 qp[kWalkWarps][32];       // the same as 16 query pairs for the packed test (store_query_pair)
-    float qh[kWalkWarps][32];        // the queries' supports (for the exact re-test)
-    int32_t qid[kWalkWarps][32];     // the queries' cloud-local indices (float64 re-test)
-    int32_t run_beg[kWalkWarps][32];
-    int32_t run_pre[kWalkWarps][33];
-    float shift[kWalkWarps][3][32];  // per run: +-ext on the dimensions its cells lie across a seam
-    float4 ring[kWalkWarps][4][32];  // candidate chunks in flight (cp.async), one slot per lane
+    alignas(128) uint4 cand[kWalkWarps][2][2][32];  // two chunks' candidates as A fragments: first and second 8 factors (cand_slot)
+    uint4 query[kWalkWarps][32][2];     // the queries as B fragments
+    float csq[kWalkWarps][2][32];       // superSymmetric: the candidates' squared supports (scaled)
+    float qsq[kWalkWarps][32];          // and the queries'
+    // per chunk of the window (and the pair after it): bit k, a run starts at its candidate k; runs before it, minus one
+    uint2 starts[kWalkWarps][kWalkWin / 32 + 2];
+    int32_t delta[kWalkWarps][32];      // per run: its first sorted index minus its first candidate
+    float shift[kWalkWarps][3][32];     // per run: +-ext on the dimensions its cell lies across a seam
     UnitCtx u[kWalkWarps];
 };
-
-// cp.async of 16 bytes from global to shared memory, its commit and wait (the copies of one
-// thread land in program order of their groups; a thread reads back only what it copied itself).
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 
 // Candidate k of the unit (prefix pre[0..S]): returns its sorted index.
 __device__ __forceinline__ int32_t cand_index(const int32_t* pre, const int32_t* beg, int S, int32_t k) {
@@ -1389,118 +1430,131 @@ __device__ __forceinline__ uint32_t chunk_hits(const WrapCtx& wc, const float4* 
     return hit;
 }
 
-// Query pairs for the packed test: pair p holds queries 2p and 2p + 1 as two float4,
-// {x0, x1, y0, y1} and {z0, z1, s0, s1}, where s is the pair-share of packed_share.
-template <int MODE>
-__device__ __forceinline__ float packed_share(float hq) {
-    return MODE == kGather ? -(hq * hq) : (MODE == kSymmetric ? 0.5f * hq : hq);
+// ---- the tensor-core test
+//
+// d^2 - thr^2 of every (query, candidate) pair of a unit is one small matrix product: with positions
+// relative to the unit's cell centre (scaled by a power of two so that a cell's edge lies in [1, 2)),
+//   |Q - C|^2 - thr^2 = N_q + N_c - 2 Q.C [- hq hc / 2],
+// N_q = |Q|^2 - (gather hq^2, symmetric hq^2 / 4), N_c = |C|^2 - (scatter hc^2, symmetric hc^2 / 4), and
+// the last term in symmetric mode (thr = (hq + hc) / 2).  Every factor is split into two float16
+// (hi + lo: 22 bits); hi*hi, hi*lo and lo*hi of the three coordinates and the supports and both
+// halves of both norms are 16 products: one mma.m16n8k16 tests 16 queries against 8 candidates, with
+// float32 accumulation.  What bounds the walk is issue slots: the float32x2 form took ~9 instructions a
+// lane and test, the product leaves 1.5 (collect the sign, keep the smallest magnitude), and its
+// accumulator layout hands each lane 4 candidates of two queries, so the hit masks need three
+// shuffles per 16 queries and 64 candidates instead of a 32 x 32 bit transpose per chunk.  mma.sync and
+// not tcgen05: a unit has ~16 queries and a chunk 32 candidates, so a 128-row tile would span several
+// warps and wait on its commit for a product that takes 8 of a chunk's ~100 issue slots.
+//
+// The product only decides pairs outside a band.  Its error for a pair near the threshold: 16
+// products, each at most E = (|Q| + thr + ..)^2, aligned and summed in about 24 bits (<= 16 * 2^-24 E;
+// measured 2^-21.4 of the largest product), dropped lo*lo terms and the halves' rounding (<= 8e-7 E).
+// kMmaBand = 4e-6 covers the sum twice (measured over random cells: 1.7e-7 E).  The pairs inside the band
+// (three in a thousand queries have one) are listed and decided exactly after the walk.
+__device__ __forceinline__ uint32_t h2bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+// (a, b) as float16 pairs: hi = fl16(a, b), lo = fl16((a, b) - hi).
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    hi = h2bits(h);
+    lo = h2bits(__floats2half2_rn(a - f.x, b - f.y));
 }
-__device__ __forceinline__ void store_query_pair(float4* qp, int lane, float x, float y, float z, float s) {
-    float* f = reinterpret_cast<float*>(qp + 2 * (lane >> 1));
-    const int hi = lane & 1;
-    f[hi] = x;
-    f[2 + hi] = y;
-    f[4 + hi] = z;
-    f[6 + hi] = s;
+// One number as the float16 pair (hi, lo).
+__device__ __forceinline__ uint32_t split_one(float n) {
+    return h2bits(__floats2half2_rn(n, n - __half2float(__float2half_rn(n))));
+}
+constexpr uint32_t kHalfOnes = 0x3c003c00u;
+
+// The 16 factors of a candidate, as 8 pairs of float16 (two 16-byte rows): (xy hi, z hc hi, xy lo,
+// z hc lo) and (xy hi, z hc hi, N_c, ones).  A query's, which meet them: -2 xy and (-2 z, -hq / 2) hi twice,
+// and (their lo parts, ones, N_q).
+template <int MODE>
+__device__ __forceinline__ void store_query_frag(uint4* f, float x, float y, float z, float h, bool live) {
+    uint32_t xyh = 0, xyl = 0, zhh = 0, zhl = 0;
+    float n = kMmaFar;
+    if (live) {
+        n = fmaf(x, x, fmaf(y, y, z * z));
+        if (MODE == kGather) n = fmaf(-h, h, n);
+        if (MODE == kSymmetric) n = fmaf(-0.25f * h, h, n);
+        split_pair(-2.0f * x, -2.0f * y, xyh, xyl);
+        split_pair(-2.0f * z, MODE == kSymmetric ? -0.5f * h : 0.0f, zhh, zhl);
+    }
+    f[0] = make_uint4(xyh, zhh, xyh, zhh);
+    f[1] = make_uint4(xyl, zhl, kHalfOnes, split_one(n));
+}
+// Returns false when the candidate is too far off for float16 (or NaN): its products decide nothing.
+// (The last pair of the second row, the ones, stays from one chunk to the next.)
+template <int MODE>
+__device__ __forceinline__ bool store_cand_frag(uint4* first, uint4* second, float x, float y, float z, float h) {
+    uint4 f;
+    const float d = fmaf(x, x, fmaf(y, y, z * z));
+    float n = d;
+    if (MODE == kScatter) n = fmaf(-h, h, n);
+    if (MODE == kSymmetric) n = fmaf(-0.25f * h, h, n);
+    split_pair(x, y, f.x, f.z);
+    split_pair(z, MODE == kSymmetric ? h : 0.0f, f.y, f.w);
+    *first = f;
+    *reinterpret_cast<uint2*>(second) = make_uint2(f.x, f.y);
+    reinterpret_cast<uint32_t*>(second)[2] = split_one(n);
+    return d <= kMmaReach * kMmaReach;
+}
+// Candidates are the product's 16 rows, queries its 8 columns (units hold any number of queries, so the
+// finer step wastes less).  Row r + 8 i of tile t is candidate 4r + 2t + i of the chunk, so that lane
+// (g = lane >> 2, t = lane & 3) holds candidates 4g .. 4g + 3 of queries 2t and 2t + 1 in the two tiles'
+// accumulators.  Candidate k's place in shared memory is k with its low bits mixed so that neither the
+// stores nor ldmatrix's eight rows (4 apart) meet in a bank.
+__device__ __forceinline__ int cand_slot(int k) { return k ^ ((k >> 3) & 3); }
+static_assert(kWalkWin == 32 * kWarp, "one chunk's starts per lane");
+static_assert(kMmaPad > 3.0f * kMmaSupport, "the lanes past the candidates must not hit");
+
+// Four 8 x 8 matrices of float16: one register each, lane (g, t) holding pair t of row g.
+__device__ __forceinline__ void load_matrix(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ void mma_16x8(float (&d)[4], const uint32_t (&c)[4], uint32_t q0, uint32_t q1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%10, %10, %10, %10};\n"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(q0), "r"(q1), "f"(0.0f));
 }
 
-// chunk_hits for non-wrapping differences (non-periodic clouds and pre-shifted seam candidates) in
-// gather, scatter and symmetric mode, two queries per instruction: the differences and the squared
-// distance run as packed float32x2 operations (each element rounded exactly as the scalar operation),
-// so the residuals and hit bits equal chunk_hits's bit for bit.  umin collects the smallest |r|
-// (NaN rows are ignored by fminf); the caller compares it with the candidate's band once per chunk.
-template <int DIM, int MODE>
-__device__ __forceinline__ uint32_t chunk_hits_x2(const float4* __restrict__ qp, int K4, const float4& cv, float cw,
-                                                  float& umin) {
-    const float2 ncx = make_float2(-cv.x, -cv.x), ncy = make_float2(-cv.y, -cv.y), ncz = make_float2(-cv.z, -cv.z);
-    const float2 ncw = make_float2(-cv.w, -cv.w), pcw = make_float2(cv.w, cv.w);
-    uint32_t hit = 0;
-    for (int p = (K4 >> 1) - 2; p >= 0; p -= 2) {  // two query pairs per iteration (K4 a multiple of 4)
-#pragma unroll
-        for (int i = 1; i >= 0; --i) {
-            const float4 a = qp[2 * (p + i)];
-            const float4 b = qp[2 * (p + i) + 1];
-            const float2 dx = __fadd2_rn(make_float2(a.x, a.y), ncx);
-            float2 d2 = __fmul2_rn(dx, dx);
-            if (DIM > 1) {
-                const float2 dy = __fadd2_rn(make_float2(a.z, a.w), ncy);
-                d2 = __ffma2_rn(dy, dy, d2);
-            }
-            if (DIM > 2) {
-                const float2 dz = __fadd2_rn(make_float2(b.x, b.y), ncz);
-                d2 = __ffma2_rn(dz, dz, d2);
-            }
-            float r0, r1;
-            if (MODE == kGather) {  // d2 - hq^2, the share holding -hq^2
-                const float2 r = __fadd2_rn(d2, make_float2(b.z, b.w));
-                r0 = r.x;
-                r1 = r.y;
-            } else if (MODE == kScatter) {  // d2 - hc^2
-                const float2 r = __ffma2_rn(ncw, pcw, d2);
-                r0 = r.x;
-                r1 = r.y;
-            } else {  // symmetric: thr = hq / 2 + hc / 2, d2 - thr^2
-                const float t0 = b.z + cw, t1 = b.w + cw;
-                r0 = fmaf(-t0, t0, d2.x);
-                r1 = fmaf(-t1, t1, d2.y);
-            }
-            hit = __funnelshift_l(__float_as_uint(r1), hit, 1);
-            hit = __funnelshift_l(__float_as_uint(r0), hit, 1);
-            umin = fminf(umin, fminf(fabsf(r0), fabsf(r1)));
-        }
+// The 32 candidates of tiles c0, c1 against the 8 queries (q0, q1): shifts 8 hits into `hit`, bits 0..3 query
+// 2t's among candidates 4g .. 4g + 3, bits 4..7 query 2t + 1's.  umin collects the smallest magnitude.
+// superSymmetric: the product is d^2, compared with max(hq, hc)^2 (cs, qs: the squared supports).
+template <int MODE>
+__device__ __forceinline__ uint32_t mma_hits(uint32_t hit, const uint32_t (&c0)[4], const uint32_t (&c1)[4],
+                                             const float4& cs, uint32_t q0, uint32_t q1, const float2& qs,
+                                             float& umin) {
+    float d0[4], d1[4];
+    mma_16x8(d0, c0, q0, q1);
+    mma_16x8(d1, c1, q0, q1);
+    if (MODE == kSuperSymmetric) {
+        d0[0] -= fmaxf(qs.x, cs.x), d0[1] -= fmaxf(qs.y, cs.x), d0[2] -= fmaxf(qs.x, cs.y), d0[3] -= fmaxf(qs.y, cs.y);
+        d1[0] -= fmaxf(qs.x, cs.z), d1[1] -= fmaxf(qs.y, cs.z), d1[2] -= fmaxf(qs.x, cs.w), d1[3] -= fmaxf(qs.y, cs.w);
     }
+    hit = __funnelshift_l(__float_as_uint(d1[3]), hit, 1);
+    hit = __funnelshift_l(__float_as_uint(d1[1]), hit, 1);
+    hit = __funnelshift_l(__float_as_uint(d0[3]), hit, 1);
+    hit = __funnelshift_l(__float_as_uint(d0[1]), hit, 1);
+    hit = __funnelshift_l(__float_as_uint(d1[2]), hit, 1);
+    hit = __funnelshift_l(__float_as_uint(d1[0]), hit, 1);
+    hit = __funnelshift_l(__float_as_uint(d0[2]), hit, 1);
+    hit = __funnelshift_l(__float_as_uint(d0[0]), hit, 1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) umin = fminf(umin, fminf(fabsf(d0[i]), fabsf(d1[i])));
     return hit;
 }
 
-// chunk_hits_x2 for the lane's candidates of two chunks at once: each query pair is read once for
-// both, and the two candidates' chains of operations are independent, so they overlap.
-template <int DIM, int MODE>
-__device__ __forceinline__ void chunk_hits_x2_two(const float4* __restrict__ qp, int K4, const float4& cv0,
-                                                  float cw0, const float4& cv1, float cw1, float& umin0,
-                                                  float& umin1, uint32_t& hit0, uint32_t& hit1) {
-    const float2 ax = make_float2(-cv0.x, -cv0.x), ay = make_float2(-cv0.y, -cv0.y), az = make_float2(-cv0.z, -cv0.z);
-    const float2 bx = make_float2(-cv1.x, -cv1.x), by = make_float2(-cv1.y, -cv1.y), bz = make_float2(-cv1.z, -cv1.z);
-    const float2 an = make_float2(-cv0.w, -cv0.w), ap = make_float2(cv0.w, cv0.w);
-    const float2 bn = make_float2(-cv1.w, -cv1.w), bp = make_float2(cv1.w, cv1.w);
-    uint32_t h0 = 0, h1 = 0;
-    for (int p = (K4 >> 1) - 1; p >= 0; --p) {
-        const float4 a = qp[2 * p];
-        const float4 b = qp[2 * p + 1];
-        const float2 qx = make_float2(a.x, a.y), qy = make_float2(a.z, a.w), qz = make_float2(b.x, b.y);
-        const float2 dx0 = __fadd2_rn(qx, ax), dx1 = __fadd2_rn(qx, bx);
-        float2 e0 = __fmul2_rn(dx0, dx0), e1 = __fmul2_rn(dx1, dx1);
-        if (DIM > 1) {
-            const float2 dy0 = __fadd2_rn(qy, ay), dy1 = __fadd2_rn(qy, by);
-            e0 = __ffma2_rn(dy0, dy0, e0);
-            e1 = __ffma2_rn(dy1, dy1, e1);
-        }
-        if (DIM > 2) {
-            const float2 dz0 = __fadd2_rn(qz, az), dz1 = __fadd2_rn(qz, bz);
-            e0 = __ffma2_rn(dz0, dz0, e0);
-            e1 = __ffma2_rn(dz1, dz1, e1);
-        }
-        float2 r0, r1;  // residuals of the query pair against each candidate
-        if (MODE == kGather) {
-            const float2 s = make_float2(b.z, b.w);
-            r0 = __fadd2_rn(e0, s);
-            r1 = __fadd2_rn(e1, s);
-        } else if (MODE == kScatter) {
-            r0 = __ffma2_rn(an, ap, e0);
-            r1 = __ffma2_rn(bn, bp, e1);
-        } else {
-            const float t00 = b.z + cw0, t01 = b.w + cw0, t10 = b.z + cw1, t11 = b.w + cw1;
-            r0 = make_float2(fmaf(-t00, t00, e0.x), fmaf(-t01, t01, e0.y));
-            r1 = make_float2(fmaf(-t10, t10, e1.x), fmaf(-t11, t11, e1.y));
-        }
-        h0 = __funnelshift_l(__float_as_uint(r0.y), h0, 1);
-        h0 = __funnelshift_l(__float_as_uint(r0.x), h0, 1);
-        h1 = __funnelshift_l(__float_as_uint(r1.y), h1, 1);
-        h1 = __funnelshift_l(__float_as_uint(r1.x), h1, 1);
-        umin0 = fminf(umin0, fminf(fabsf(r0.x), fabsf(r0.y)));
-        umin1 = fminf(umin1, fminf(fabsf(r1.x), fabsf(r1.y)));
-    }
-    hit0 = h0;
-    hit1 = h1;
+// 8 x 8 transpose of nibbles across the lanes of equal t: nibble i of lane g goes to nibble g of lane i.
+__device__ __forceinline__ uint32_t nibble_transpose(uint32_t x, int lane) {
+    x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 16), (lane & 16) ? 0x3276u : 0x5410u);
+    x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 8), (lane & 8) ? 0x3715u : 0x6240u);
+    const uint32_t keep = (lane & 4) ? 0xf0f0f0f0u : 0x0f0f0f0fu, rot = (lane & 4) ? 4u : 28u;
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, 4);
+    return (x & keep) | (__funnelshift_r(y, y, rot) & ~keep);
 }
 
 // The same with every pair inside the band decided by the reference's exact test, on the original
@@ -1525,90 +1579,202 @@ __device__ __noinline__ uint32_t chunk_hits_exact(ExactCtx xc, const float4* qsm
     return hit;
 }
 
-// Count walk of one unit: test every (query, candidate) once, count, and stage the unit's record.
-//
-// The unit's candidates stream in chunks of 32, one per lane (a coalesced load of consecutive
-// sorted points); the unit's queries sit in shared memory and are broadcast to every lane, so each
-// lane tests its candidate against every query with no lane left idle but the last chunk's.  A
-// lane's hit bits over the queries are transposed across the warp into the (query, chunk) masks.
-template <int DIM, bool PERIODIC, int MODE>
-__device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int32_t unit, int32_t grp, int lane,
-                                           int w) {
+// A unit as both walks start it: its queries (one per lane), its stencil cells (one per lane) and where
+// the cells' candidates lie in the unit's sequence.
+struct Unit {
+    int32_t nb, M;        // queries, candidates
+    int32_t gc[3];
+    float4 q;             // the lane's query (NaN past the unit's queries and for strays)
+    int32_t qorig;
+    bool active;          // the lane holds a query of this unit's cell
+    int32_t beg, cnt, pre;  // the lane's stencil cell: first sorted point, points, first candidate
+    float sh[3];          // its seam shift
+    bool shift_mode, seam;
+};
+
+// STRAYS: append the queries whose own cell is not the unit's to the stray list.
+template <int DIM, bool PERIODIC, bool STRAYS>
+__device__ __forceinline__ Unit open_unit(const WalkArgs& a, const UnitCtx& u, int32_t unit, int32_t grp, int lane) {
     constexpr int S = DIM == 1 ? 3 : (DIM == 2 ? 9 : 27);
-    const UnitCtx& u = sm.u[w];
-    const float inf = __int_as_float(0x7f800000);
-    const float4 nan4 = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
+    Unit n;
     const int32_t t0 = a.unit_t0[unit];
-    const int32_t nb = min(*a.unit_cap, a.group_start[grp + 1] - t0);
-    const int32_t gc[3] = {a.group_coords[3 * grp], a.group_coords[3 * grp + 1], a.group_coords[3 * grp + 2]};
+    n.nb = min(*a.unit_cap, a.group_start[grp + 1] - t0);
+    for (int d = 0; d < 3; ++d) n.gc[d] = a.group_coords[3 * grp + d];
     // the unit's queries, loaded before the stencil look-ups so that both latencies overlap
-    const bool qlane = lane < nb && TCR_IN(t0 + lane, a.nq_total);
-    float4 qv = nan4;
-    int32_t qorig = 0;
+    const float4 nan4 = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
+    const bool qlane = lane < n.nb && TCR_IN(t0 + lane, a.nq_total);
+    n.q = nan4;
+    n.qorig = 0;
     if (qlane) {
-        qv = a.qsorted[t0 + lane];
-        qorig = a.qsidx[t0 + lane];
+        n.q = a.qsorted[t0 + lane];
+        n.qorig = a.qsidx[t0 + lane];
     }
-    int32_t beg = 0, cnt = 0;
-    if (lane < S) stencil_lookup(a, u, gc, lane, beg, cnt);
-    const bool shift_mode = PERIODIC && u.shift_ok;
-    float sh[3] = {0.f, 0.f, 0.f};  // the stencil cell's seam shift, in stencil_lookup's offset order
-    if (shift_mode) {
+    n.beg = n.cnt = 0;
+    if (lane < S) stencil_lookup<DIM>(a, u, n.gc, lane, n.beg, n.cnt);
+    n.shift_mode = PERIODIC && u.shift_ok;
+    n.sh[0] = n.sh[1] = n.sh[2] = 0.f;
+    if (n.shift_mode) {  // in stencil_lookup's offset order
         int rem = lane;
 #pragma unroll
         for (int d = DIM - 1; d >= 0; --d) {
-            const int32_t v = gc[d] + rem % 3 - 1;
+            const int32_t v = n.gc[d] + rem % 3 - 1;
             rem /= 3;
             if (lane < S && ((u.periodic_mask >> d) & 1))
-                sh[d] = v < 0 ? -u.ext[d] : (v >= u.count[d] ? u.ext[d] : 0.f);
+                n.sh[d] = v < 0 ? -u.ext[d] : (v >= u.count[d] ? u.ext[d] : 0.f);
         }
     }
-    const bool seam = shift_mode && __any_sync(0xffffffffu, sh[0] != 0.f || sh[1] != 0.f || sh[2] != 0.f);
-    // runs: a stencil cell whose range continues the previous cell's (same shift) extends its run
-    const int32_t inc = warp_inclusive_scan(cnt);
-    const int32_t M = __shfl_sync(0xffffffffu, inc, 31);
-    const int32_t pbeg = __shfl_up_sync(0xffffffffu, beg, 1);
-    const int32_t pcnt = __shfl_up_sync(0xffffffffu, cnt, 1);
-    bool cont = lane > 0 && pcnt > 0 && pbeg + pcnt == beg;
-    if (shift_mode) {  // every lane takes part in the shuffles (no short-circuit around them)
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-            const float psh = __shfl_up_sync(0xffffffffu, sh[d], 1);
-            cont = cont && psh == sh[d];
+    n.seam = n.shift_mode && __any_sync(0xffffffffu, n.sh[0] != 0.f || n.sh[1] != 0.f || n.sh[2] != 0.f);
+    const int32_t inc = warp_inclusive_scan(n.cnt);
+    n.M = __shfl_sync(0xffffffffu, inc, 31);
+    n.pre = inc - n.cnt;
+    // a query whose own cell differs from the group's leaves for the serial path
+    n.active = false;
+    if (qlane) {
+        n.active = TCR_IN(n.qorig, a.nq_total);
+        if (n.active && (!a.no_stray_check || u.out_of_grid)) {
+            int32_t qc[3];
+            cell_of(DIM, u.dedupe, u.dmin, u.hcell, u.count, n.q, qc);
+            n.active = same_cell<DIM>(qc, n.gc);
+        }
+        if (!n.active) {  // own cell differs from the group's (aliasing or wrap rounding)
+            if (STRAYS) {
+                const int32_t k = atomicAdd(a.num_stray, 1);
+                if (TCR_IN(k, a.nq_total)) a.stray[k] = t0 + lane;
+            }
+            n.q = nan4;
         }
     }
-    const bool starts = cnt > 0 && !cont;
+    return n;
+}
+
+// What fix_unit keeps in shared memory, in place of the candidates' fragments.
+struct FixSmem {
+    float4 q[32];        // the unit's queries: x, y, z and the query's share of the test
+    float qh[32];        // the queries' supports (for the exact test)
+    int32_t qid[32];     // the queries' cloud-local indices (float64 inputs)
+    int32_t pre[33];     // candidate prefix of the stencil cells
+    int32_t beg[32];
+    float shift[3][32];
+};
+static_assert(sizeof(FixSmem) <= sizeof(uint4) * 2 * 2 * 32, "fits the fragments of one warp");
+
+// A unit the product did not take: a periodic cloud with so few cells that differences wrap, supports
+// outside the fast test's range, points far outside their cell.  One candidate per lane against every
+// query in float32; a chunk with a pair inside the float32 band once more with those pairs decided by
+// the reference's exact test; the hit bits transposed into the masks.  Out of line, at the unit's end, so
+// that its registers do not cost the main loop spills.
+template <int DIM, bool PERIODIC, int MODE>
+__device__ __noinline__ void fix_unit(const WalkArgs& a, WalkSmem& wsm, int32_t unit, int32_t grp, int lane, int w) {
+    const UnitCtx& u = wsm.u[w];
+    FixSmem& sm = *reinterpret_cast<FixSmem*>(&wsm.cand[w][0][0][0]);
+    const float4 nan4 = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
+    const Unit n = open_unit<DIM, PERIODIC, false>(a, u, unit, grp, lane);
+    constexpr int S = DIM == 1 ? 3 : (DIM == 2 ? 9 : 27);
+    sm.pre[lane] = n.pre;
+    if (lane == 0) sm.pre[S] = n.M;
+    sm.beg[lane] = n.beg;
+    for (int d = 0; d < 3; ++d) sm.shift[d][lane] = n.sh[d];
+    sm.q[lane] = make_float4(n.q.x, n.q.y, n.q.z, query_share<MODE>(n.q.w));  // rows >= nb: NaN, never hit
+    sm.qh[lane] = n.q.w;
+    sm.qid[lane] = n.qorig - u.qshift;
+    __syncwarp();
+    const int32_t base = a.rec[unit];
+    uint32_t* msk = nullptr;
+    if (base >= 0 && TCR_GUARD(base + kRecHeader, a.stage_cap)) {
+        const int32_t* rec = a.stage + base;
+        msk = reinterpret_cast<uint32_t*>(a.stage + base + kRecHeader + 2 * rec[1] + 1);
+    }
+    const WrapCtx wc = wrap_ctx(u.periodic_mask, u.ext);
+    const int K4 = (n.nb + 3) & ~3;
+    const int32_t nchunks = (n.M + 31) >> 5;
+    const bool has = msk != nullptr && lane < n.nb;
+    int32_t count = 0;
+    for (int32_t c = 0; c < nchunks; ++c) {
+        const int32_t k = (c << 5) + lane;
+        float4 cv = nan4, cs = nan4;
+        int32_t j = 0;
+        if (k < n.M) {
+            int lo = 0, hi = S;  // pre[lo] <= k < pre[hi]
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (sm.pre[mid] <= k) lo = mid; else hi = mid;
+            }
+            j = sm.beg[lo] + (k - sm.pre[lo]);
+            if (TCR_GUARD(j, a.nr_total)) cv = __ldg(&a.rsorted[j]);
+            cs = cv;
+            if (PERIODIC && n.seam) {
+                cs.x += sm.shift[0][lo];
+                if (DIM > 1) cs.y += sm.shift[1][lo];
+                if (DIM > 2) cs.z += sm.shift[2][lo];
+            }
+        }
+        const float cw = cand_share<MODE>(cv.w);
+        const float t = cand_tmax<MODE>(cw, u.qmax);
+        float band = u.exact_all ? __int_as_float(0x7f800000) : kBandEps * t * t;
+        // float64 inputs: the band also covers the rounding of the coordinates to float32
+        if (u.f64_err > 0.0f) band += fmaf(2.0f * 1.7320508f * t, u.f64_err, 3.0f * u.f64_err * u.f64_err);
+        // shifted candidates: the band also covers the shift's rounding (|d2 error| <= 2 T delta + delta^2)
+        const float bs = n.seam ? band + fmaf(2.0f * t, u.shift_delta, u.shift_delta * u.shift_delta) : band;
+        bool unc = false;
+        uint32_t hit;
+        if (!PERIODIC || n.shift_mode)
+            hit = chunk_hits<DIM, false, MODE>(wc, sm.q, K4, cs, cw, bs, unc);
+        else
+            hit = chunk_hits<DIM, PERIODIC, MODE>(wc, sm.q, K4, cv, cw, bs, unc);
+        if (__any_sync(0xffffffffu, unc)) {
+            hit = chunk_hits_exact<DIM, MODE>(unit_exact_ctx(u, MODE), sm.q, sm.qh, sm.qid, K4, cv, j, band,
+                                              a.f64);
+        }
+        const uint32_t m = warp_transpose32(hit, lane);
+        if (lane < n.nb) {
+            count += __popc(m);
+            if (has) msk[c * n.nb + lane] = m;
+        }
+    }
+    if (n.active) a.counts[n.qorig] = count;
+    __syncwarp();
+    wsm.cand[w][0][1][lane].w = wsm.cand[w][1][1][lane].w = kHalfOnes;
+}
+
+// Count walk of one unit: test every (query, candidate) once, count, and stage the unit's record.
+//
+// The unit's candidates stream two chunks of 32 at a time, one per lane and chunk (a lane finds its
+// candidate's run by its rank among the runs' starts), loaded a pair ahead of their use; they are written to
+// shared memory as A fragments and meet the unit's queries (B fragments, in registers) in
+// tensor-core products.
+template <int DIM, bool PERIODIC, int MODE>
+__device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int32_t unit, int32_t grp, int lane,
+                                           int w) {
+    const UnitCtx& u = sm.u[w];
+    const Unit n = open_unit<DIM, PERIODIC, true>(a, u, unit, grp, lane);
+    const int32_t nb = n.nb, M = n.M;
+    // runs: the non-empty stencil cells
+    const bool starts = n.cnt > 0;
     const uint32_t smask = __ballot_sync(0xffffffffu, starts);
     const int32_t R = __popc(smask);
     const int rid = __popc(smask & ((1u << lane) - 1u));
     if (starts) {
-        sm.run_beg[w][rid] = beg;
-        sm.run_pre[w][rid] = inc - cnt;
-        sm.shift[w][0][rid] = sh[0];
-        sm.shift[w][1][rid] = sh[1];
-        sm.shift[w][2][rid] = sh[2];
-    }
-    if (lane == 0) sm.run_pre[w][R] = M;
-    // the unit's queries: a query whose own cell differs from the group's leaves for the serial path
-    bool active = false;
-    if (qlane) {
-        const int32_t t = t0 + lane;
-        active = TCR_IN(qorig, a.nq_total);
-        if (active && (!a.no_stray_check || u.out_of_grid)) {
-            int32_t qc[3];
-            cell_of(DIM, u.dedupe, u.dmin, u.hcell, u.count, qv, qc);
-            active = same_cell<DIM>(qc, gc);
-        }
-        if (!active) {  // own cell differs from the group's (aliasing or wrap rounding): serial path
-            const int32_t k = atomicAdd(a.num_stray, 1);
-            if (TCR_IN(k, a.nq_total)) a.stray[k] = t;
-            qv = nan4;
+        sm.delta[w][rid] = n.beg - n.pre;
+        if (PERIODIC) {
+            sm.shift[w][0][rid] = n.sh[0];
+            sm.shift[w][1][rid] = n.sh[1];
+            sm.shift[w][2][rid] = n.sh[2];
         }
     }
-    sm.qh[w][lane] = qv.w;
-    sm.qid[w][lane] = qorig - u.qshift;
-    sm.q[w][lane] = make_float4(qv.x, qv.y, qv.z, query_share<MODE>(qv.w));  // rows >= nb: NaN, never hit
-    store_query_pair(sm.qp[w], lane, qv.x, qv.y, qv.z, packed_share<MODE>(qv.w));
+    // scaled positions relative to the cell's centre: fma(x, s, -centre * s) is exact up to one rounding
+    const float s = u.scale;
+    float os[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) os[d] = d < DIM ? -s * fmaf((float)n.gc[d] + 0.5f, u.hcell[d], u.dmin[d]) : 0.f;
+    const float X = fmaf(n.q.x, s, os[0]), Y = DIM > 1 ? fmaf(n.q.y, s, os[1]) : 0.f,
+                Z = DIM > 2 ? fmaf(n.q.z, s, os[2]) : 0.f, H = n.q.w * s;
+    store_query_frag<MODE>(sm.query[w][lane], X, Y, Z, H, n.active);
+    if (MODE == kSuperSymmetric) sm.qsq[w][lane] = H * H;
+    // the product takes the unit when its points are where their cell says (a query is at most half a
+    // cell off the centre) and every support is in its range; otherwise fix_unit tests it
+    const float far = u.scale_cell * 0.55f;
+    const bool near = !n.active || (fabsf(X) <= far && fabsf(Y) <= far && fabsf(Z) <= far);
+    const bool product = u.mma_ok && (!PERIODIC || n.shift_mode) && __all_sync(0xffffffffu, near);
     // the unit's record, reserved up front
     const int32_t nchunks = (M + 31) >> 5;
     bool stage = false;
@@ -1630,120 +1796,12 @@ __device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int3
                 a.rec[unit] = (int32_t)base;
             }
             if (starts) {
-                rec[kRecHeader + rid] = beg;
-                rec[kRecHeader + R + rid] = inc - cnt;
+                rec[kRecHeader + rid] = n.beg;
+                rec[kRecHeader + R + rid] = n.pre;
             }
             msk = reinterpret_cast<uint32_t*>(rec + kRecHeader + 2 * R + 1);
         }
     }
-    __syncwarp();
-    // lane k of chunk c holds candidate 32c + k; its run only moves forward from chunk to chunk
-    const int32_t* rpre = sm.run_pre[w];
-    const int32_t* rbeg = sm.run_beg[w];
-    const float4* __restrict__ rs = a.rsorted;
-    int32_t cr = 0;
-    const WrapCtx wc = wrap_ctx(u.periodic_mask, u.ext);
-    const float qmax = u.qmax;
-    const bool exact_all = u.exact_all != 0;
-    const float dl = u.shift_delta;
-    const float fe = u.f64_err;
-    const int K4 = (nb + 3) & ~3;
-    const float4* qsm = sm.q[w];
-    uint32_t count = 0;
-    // The fast pass takes the chunks two at a time (each lane tests its candidate of both against
-    // every query, reading each query pair once) and streams them into a four-slot ring in shared
-    // memory by cp.async, a pair of chunks ahead of its use, so the loads' latency hides behind the
-    // tests without holding registers.  Lanes past the unit's candidates get NaN (never a hit).
-    float4* ring = &sm.ring[w][0][0];
-    auto issue = [&](int32_t c) {
-        const int32_t k = (c << 5) + lane;
-        float4* dst = ring + (c & 3) * 32 + lane;
-        bool copied = false;
-        if (k < M) {
-            while (rpre[cr + 1] <= k) ++cr;
-            const int32_t j = rbeg[cr] + (k - rpre[cr]);
-            if (TCR_GUARD(j, a.nr_total)) {
-                cp_async16(dst, &rs[j]);
-                copied = true;
-            }
-        }
-        if (!copied) *dst = nan4;
-        cp_async_commit();
-        return cr;
-    };
-    // one landed chunk: the candidate (shifted across a seam for the fast test) and its bands
-    auto take = [&](int32_t c, int32_t crn, float4& cv, float& cw, float& band, float& band_exact) {
-        cv = ring[(c & 3) * 32 + lane];
-        if (PERIODIC && shift_mode) {
-            cv.x += sm.shift[w][0][crn];
-            if (DIM > 1) cv.y += sm.shift[w][1][crn];
-            if (DIM > 2) cv.z += sm.shift[w][2][crn];
-        }
-        cw = cand_share<MODE>(cv.w);
-        const float t = cand_tmax<MODE>(cw, qmax);
-        band = exact_all ? inf : kBandEps * t * t;
-        // float64 inputs: the band also covers the rounding of the coordinates to float32
-        if (fe > 0.0f) band += fmaf(2.0f * 1.7320508f * t, fe, 3.0f * fe * fe);
-        band_exact = band;
-        // shifted candidates: the band also covers the shift's rounding (|d2 error| <= 2 T delta + delta^2)
-        if (seam) band += fmaf(2.0f * t, dl, dl * dl);
-    };
-    // some pair of a chunk lies within the band: the chunk again, every pair in the band decided by
-    // the reference's exact test on the original (unshifted) candidates
-    auto exact = [&](int32_t c, int32_t crn, float band_exact) {
-        if (lane == 0) atomicAdd(a.num_exact, 1);
-        const int32_t k = (c << 5) + lane;
-        float4 v0 = nan4;
-        int32_t j = 0;
-        if (k < M) {
-            j = rbeg[crn] + (k - rpre[crn]);
-            if (TCR_GUARD(j, a.nr_total)) v0 = __ldg(&rs[j]);
-        }
-        return chunk_hits_exact<DIM, MODE>(unit_exact_ctx(u, MODE), qsm, sm.qh[w], sm.qid[w], K4, v0, j, band_exact,
-                                           a.f64);
-    };
-    auto store = [&](int32_t c, uint32_t m) {
-        if (lane < nb) {
-            count += __popc(m);
-            if (stage && TCR_IN((int64_t)(msk - reinterpret_cast<uint32_t*>(a.stage)) + c * nb + lane, a.stage_cap))
-                msk[c * nb + lane] = m;
-        }
-    };
-    int32_t cr0 = issue(0);  // runs of the candidates of chunks c and c + 1 (seam shifts)
-    int32_t cr1 = issue(1);
-    for (int32_t c = 0; c < nchunks; c += 2) {
-        const int32_t cr2 = issue(c + 2), cr3 = issue(c + 3);
-        cp_async_wait<2>();  // chunks c and c + 1 have landed
-        const bool two = c + 1 < nchunks;  // (past the last chunk the ring holds NaN: no hits)
-        float4 cv0, cv1;
-        float cw0, cw1, band0, band1, bx0, bx1;
-        take(c, cr0, cv0, cw0, band0, bx0);
-        take(c + 1, cr1, cv1, cw1, band1, bx1);
-        uint32_t hit0, hit1 = 0;
-        bool in0 = false, in1 = false;  // some pair of this lane's candidate lies within the band
-        if (MODE != kSuperSymmetric && (!PERIODIC || shift_mode)) {
-            float umin0 = inf, umin1 = inf;
-            chunk_hits_x2_two<DIM, MODE>(sm.qp[w], K4, cv0, cw0, cv1, cw1, umin0, umin1, hit0, hit1);
-            in0 = umin0 <= band0;
-            in1 = umin1 <= band1;
-        } else if (shift_mode) {
-            hit0 = chunk_hits<DIM, false, MODE>(wc, qsm, K4, cv0, cw0, band0, in0);
-            if (two) hit1 = chunk_hits<DIM, false, MODE>(wc, qsm, K4, cv1, cw1, band1, in1);
-        } else {
-            hit0 = chunk_hits<DIM, PERIODIC, MODE>(wc, qsm, K4, cv0, cw0, band0, in0);
-            if (two) hit1 = chunk_hits<DIM, PERIODIC, MODE>(wc, qsm, K4, cv1, cw1, band1, in1);
-        }
-        if (__any_sync(0xffffffffu, in0)) hit0 = exact(c, cr0, bx0);
-        if (two && __any_sync(0xffffffffu, in1)) hit1 = exact(c + 1, cr1, bx1);
-        // the two transposes are independent, so their shuffle chains overlap
-        const uint32_t m0 = warp_transpose32(hit0, lane);
-        const uint32_t m1 = warp_transpose32(hit1, lane);
-        store(c, m0);
-        if (two) store(c + 1, m1);
-        cr0 = cr2;
-        cr1 = cr3;
-    }
-    if (active) a.counts[qorig] = (int32_t)count;
     if (lane == 0 && !stage && TCR_IN(unit, a.nq_total)) {
         a.rec[unit] = -1;
         if (nchunks > 0) {  // not staged: the emit walk tests the unit again
@@ -1752,6 +1810,177 @@ __device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int3
         }
     }
     __syncwarp();
+    uint32_t count = 0;
+    bool redo = false;  // the unit goes to fix_unit after all
+    if (product) {
+        float band = u.mma_band;
+        if (PERIODIC && n.seam) band += u.mma_seam;
+        const int g = lane >> 2, tq = lane & 3;
+        const int slot = cand_slot(lane);
+        // ldmatrix row of this lane: matrix i = lane >> 3 is factors 8 (i >> 1) .. of rows 8 (i & 1) .. of a tile
+        // (the second tile's candidates are two on: the place with bit 1 flipped)
+        const uint32_t crow = (uint32_t)__cvta_generic_to_shared(
+            &sm.cand[w][0][lane >> 4][cand_slot(4 * (lane & 7) + ((lane >> 3) & 1))]);
+        // the masks this lane ends up with: query (and 16 more), chunk of the pair
+        const int row0 = 8 * ((lane >> 3) & 1) + 2 * tq + (g & 1), half = lane >> 4;
+        const bool keep0 = stage && row0 < nb, keep1 = stage && row0 + 16 < nb;
+        uint32_t* out = msk + half * nb + row0;
+        uint32_t count1 = 0;
+        const uint32_t le = (2u << lane) - 1u;  // bits 0 .. lane
+        for (int32_t w0 = 0; w0 < M; w0 += kWalkWin) {
+            // where the window's runs start, and the rank of each chunk's first run
+            const int32_t wn = min(M - w0, kWalkWin);
+            sm.starts[w][lane] = make_uint2(0u, 0u);
+            __syncwarp();
+            const int32_t at = n.pre - w0;
+            if (starts && at >= 0 && at < kWalkWin) atomicOr(&sm.starts[w][at >> 5].x, 1u << (at & 31));
+            __syncwarp();
+            const int32_t before = __popc(__ballot_sync(0xffffffffu, starts && at < 0));
+            const int32_t here = __popc(sm.starts[w][lane].x);
+            const int32_t upto = before + warp_inclusive_scan(here) - 1;
+            sm.starts[w][lane].y = (uint32_t)(upto - here);
+            if (lane == 31) sm.starts[w][32] = sm.starts[w][33] = make_uint2(0u, (uint32_t)upto);
+            __syncwarp();
+            // candidate k of the window (lanes past the last one repeat it)
+            auto run_of = [&](int32_t k) -> int32_t {
+                const uint2 st = sm.starts[w][k >> 5];
+                return (int32_t)st.y + __popc(st.x & le);
+            };
+            auto fetch = [&](int32_t k, int32_t& run) -> float4 {
+                run = run_of(k);
+                const int32_t j = sm.delta[w][run] + (w0 + min(k, wn - 1));
+                return __ldg(&a.rsorted[j]);
+            };
+            uint32_t marked = 0;  // the window's pairs of chunks with a pair inside the band
+            // one copy of the loop per number of query tiles: a tile costs no branch
+            auto pairs = [&](auto tiles) {
+                constexpr int NT = decltype(tiles)::value;
+                uint32_t qa[4], qb[4];  // (first, second row) of query tiles 0, 1 and 2, 3
+                float2 qs[4];
+                const uint32_t qrow = (uint32_t)__cvta_generic_to_shared(
+                    &sm.query[w][8 * (lane >> 4) + (lane & 7)][(lane >> 3) & 1]);
+                load_matrix(qa, qrow);
+                if (NT >= 3) load_matrix(qb, qrow + 16 * 2 * 16);
+                if (MODE == kSuperSymmetric)
+#pragma unroll
+                    for (int i = 0; i < NT; ++i) qs[i] = *reinterpret_cast<const float2*>(&sm.qsq[w][8 * i + 2 * tq]);
+                int32_t run[2];
+                float4 v[2];
+                v[0] = fetch(lane, run[0]);
+                v[1] = fetch(32 + lane, run[1]);
+                for (int32_t k0 = 0; k0 < wn; k0 += 64) {
+                    float umin = __int_as_float(0x7f800000);
+                    bool far = false;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float x = v[e].x, y = v[e].y, z = v[e].z;
+                        if (PERIODIC && n.seam) {
+                            x += sm.shift[w][0][run[e]];
+                            if (DIM > 1) y += sm.shift[w][1][run[e]];
+                            if (DIM > 2) z += sm.shift[w][2][run[e]];
+                        }
+                        x = k0 + 32 * e + lane < wn ? fmaf(x, s, os[0]) : kMmaPad;
+                        y = DIM > 1 ? fmaf(y, s, os[1]) : 0.f;
+                        z = DIM > 2 ? fmaf(z, s, os[2]) : 0.f;
+                        const float h = v[e].w * s;
+                        far |= !store_cand_frag<MODE>(&sm.cand[w][e][0][slot], &sm.cand[w][e][1][slot], x, y, z, h);
+                        if (MODE == kSuperSymmetric) sm.csq[w][e][lane] = h * h;
+                    }
+                    __syncwarp();
+                    v[0] = fetch(k0 + 64 + lane, run[0]);
+                    v[1] = fetch(k0 + 96 + lane, run[1]);
+                    // nibbles: (query 2t, 2t + 1) x (queries 0 .. 7, 8 .. 15) x (chunk 0, 1); p1 the same for queries 16 ..
+                    uint32_t p0 = 0, p1 = 0;
+#pragma unroll
+                    for (int e = 1; e >= 0; --e) {
+                        if (e == 1 && k0 + 32 >= wn) continue;
+                        uint32_t c0[4], c1[4];
+                        load_matrix(c0, crow + e * (2 * 32 * 16));
+                        load_matrix(c1, (crow ^ 32u) + e * (2 * 32 * 16));
+                        float4 cs;
+                        if (MODE == kSuperSymmetric) cs = *reinterpret_cast<const float4*>(&sm.csq[w][e][4 * g]);
+                        if (NT >= 2) p0 = mma_hits<MODE>(p0, c0, c1, cs, qa[2], qa[3], qs[1], umin);
+                        else p0 <<= 8;
+                        p0 = mma_hits<MODE>(p0, c0, c1, cs, qa[0], qa[1], qs[0], umin);
+                        if (NT >= 4) p1 = mma_hits<MODE>(p1, c0, c1, cs, qb[2], qb[3], qs[3], umin);
+                        else if (NT >= 3) p1 <<= 8;
+                        if (NT >= 3) p1 = mma_hits<MODE>(p1, c0, c1, cs, qb[0], qb[1], qs[2], umin);
+                    }
+                    redo |= far;
+                    if (__any_sync(0xffffffffu, umin <= band)) marked |= 1u << (k0 >> 6);
+                    const bool in = k0 + 32 * half < wn;
+                    const uint32_t m0 = nibble_transpose(p0, lane);
+                    count += __popc(m0);
+                    if (keep0 && in) out[0] = m0;
+                    if (NT >= 3) {
+                        const uint32_t m1 = nibble_transpose(p1, lane);
+                        count1 += __popc(m1);
+                        if (keep1 && in) out[16] = m1;
+                    }
+                    out += 2 * nb;
+                    __syncwarp();  // the fragments are read before the next pair's are written
+                }
+            };
+            if (nb <= 8) pairs(std::integral_constant<int, 1>());
+            else if (nb <= 16) pairs(std::integral_constant<int, 2>());
+            else if (nb <= 24) pairs(std::integral_constant<int, 3>());
+            else pairs(std::integral_constant<int, 4>());
+            // rare: list the pairs inside the band among the marked chunks -- their products again, tile by
+            // tile, each lane keeping its own
+            if (!stage && marked) redo = true;
+#pragma unroll 1
+            for (int32_t c = 0; stage && 32 * c < wn && (marked >> (c >> 1)); ++c) {
+                if (!((marked >> (c >> 1)) & 1u)) continue;
+                int32_t run;
+                const float4 v = fetch(32 * c + lane, run);
+                float x = v.x, y = v.y, z = v.z;
+                if (PERIODIC && n.seam) {
+                    x += sm.shift[w][0][run];
+                    if (DIM > 1) y += sm.shift[w][1][run];
+                    if (DIM > 2) z += sm.shift[w][2][run];
+                }
+                store_cand_frag<MODE>(&sm.cand[w][0][0][slot], &sm.cand[w][0][1][slot], fmaf(x, s, os[0]),
+                                      DIM > 1 ? fmaf(y, s, os[1]) : 0.f, DIM > 2 ? fmaf(z, s, os[2]) : 0.f, v.w * s);
+                if (MODE == kSuperSymmetric) sm.csq[w][0][lane] = (v.w * s) * (v.w * s);
+                __syncwarp();
+#pragma unroll 1
+                for (int i = 0; 8 * (i >> 1) < nb; ++i) {  // tile i & 1 of the candidates, i >> 1 of the queries
+                    uint32_t cf[4];
+                    load_matrix(cf, crow ^ (32u * (i & 1)));
+                    const uint32_t* qf = reinterpret_cast<const uint32_t*>(&sm.query[w][8 * (i >> 1) + g][0]);
+                    float d[4];
+                    mma_16x8(d, cf, qf[tq], qf[4 + tq]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int q = 8 * (i >> 1) + 2 * tq + (j & 1), k = 32 * c + 4 * g + 2 * (i & 1) + (j >> 1);
+                        float r = d[j];
+                        if (MODE == kSuperSymmetric) r -= fmaxf(sm.qsq[w][q], sm.csq[w][0][k & 31]);
+                        if (!(fabsf(r) <= band) || q >= nb || k >= wn) continue;
+                        const int32_t f = atomicAdd(a.num_exact, 1);
+                        const uint2 st = sm.starts[w][k >> 5];
+                        run = (int32_t)st.y + __popc(st.x & ((2u << (k & 31)) - 1u));
+                        if (f < a.nq_total)
+                            a.band_pairs[f] = make_int4(
+                                a.unit_t0[unit] + q, sm.delta[w][run] + w0 + k,
+                                a.rec[unit] + kRecHeader + 2 * R + 1 + ((w0 + k) >> 5) * nb + q, k & 31);
+                        else
+                            redo = true;  // the list is full
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        redo = __any_sync(0xffffffffu, redo);
+        // the two chunks of a pair were counted by different lanes; query q's count to lane q
+        count += __shfl_xor_sync(0xffffffffu, count, 16);
+        count1 += __shfl_xor_sync(0xffffffffu, count1, 16);
+        const int from = (lane & 8) | ((lane & 1) << 2) | ((lane >> 1) & 3);
+        const uint32_t ca = __shfl_sync(0xffffffffu, count, from), cb = __shfl_sync(0xffffffffu, count1, from);
+        count = lane < 16 ? ca : cb;
+    }
+    if (n.active) a.counts[n.qorig] = (int32_t)count;
+    __syncwarp();
+    if (nchunks > 0 && (!product || redo)) fix_unit<DIM, PERIODIC, MODE>(a, sm, unit, grp, lane, w);
 }
 
 // Class (dim * 2 + any periodic dim) of a cloud, the key of the walk kernels' template.
@@ -1779,9 +2008,10 @@ __device__ __forceinline__ uint32_t next_units(const WalkArgs& a, int32_t* count
 
 template <int DIM, bool PERIODIC, int MODE>
 __global__ void __launch_bounds__(kWalkWarps * 32, PERIODIC ? kWalkMinBlocksPeriodic : kWalkMinBlocks)
-    walk_count_kernel(WalkArgs a) {
+    walk_count_kernel(const __grid_constant__ WalkArgs a) {
     __shared__ WalkSmem sm;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int e = 0; e < 2; ++e) sm.cand[w][e][1][lane].w = kHalfOnes;
     const int32_t nunits = *a.num_units;
     int32_t* counter = &a.work[a.class_filter >= 0 ? 2 + a.class_filter : 0];
     int cur = -1;
@@ -1843,7 +2073,7 @@ __device__ __forceinline__ void emit_unit(const WalkArgs& a, EmitSmem& sm, int32
     const int32_t nb = min(*a.unit_cap, a.group_start[grp + 1] - t0);
     const int32_t gc[3] = {a.group_coords[3 * grp], a.group_coords[3 * grp + 1], a.group_coords[3 * grp + 2]};
     int32_t beg = 0, cnt = 0;
-    if (lane < S) stencil_lookup(a, u, gc, lane, beg, cnt);
+    if (lane < S) stencil_lookup<DIM>(a, u, gc, lane, beg, cnt);
     const int32_t inc = warp_inclusive_scan(cnt);
     sm.pre[w][lane + 1] = inc;
     if (lane == 0) sm.pre[w][0] = 0;
@@ -2201,9 +2431,39 @@ __global__ void __launch_bounds__(kExpandWarps * 32, 4) expand_records_kernel(Ex
 }
 
 // Serial walk for queries whose own cell differs from their group's (one thread per query).
+// After the count walk also: each pair inside the product's band decided by the reference's exact test, its
+// hit bit and its query's count corrected where the product's sign said otherwise (one thread per pair).
+__device__ __forceinline__ void decide_band_pair(const WalkArgs& a, const int4& p) {
+    if (!TCR_GUARD(p.x, a.nq_total) || !TCR_GUARD(p.y, a.nr_total) || !TCR_GUARD(p.z, a.stage_cap)) return;
+    const int32_t qorig = a.qsidx[p.x];
+    const CloudParams& cp = a.table[cloud_of(a.query_prefix, a.num_clouds, qorig)];
+    bool in;
+    if (a.f64.qpos) {
+        in = f64_pair_decide(a.f64, cp.dim, cp.periodic_mask, a.mode, qorig - (a.local_index ? cp.query_base : 0), p.y);
+    } else {
+        ExactCtx xc;
+        xc.dim = cp.dim;
+        xc.mode = a.mode;
+        xc.periodic_mask = cp.periodic_mask;
+        for (int d = 0; d < 3; ++d) xc.ext[d] = cp.ext[d];
+        const float4 q = a.qsorted[p.x], c = a.rsorted[p.y];
+        in = exact_pair_test(xc, q, q.w, c, c.w);
+    }
+    const uint32_t bit = 1u << (p.w & 31);
+    const bool was = (a.stage[p.z] & bit) != 0;
+    if (in == was) return;
+    atomicXor(reinterpret_cast<uint32_t*>(&a.stage[p.z]), bit);
+    atomicAdd(&a.counts[qorig], in ? 1 : -1);
+}
+
 template <bool EMIT>
 __global__ void stray_kernel(WalkArgs a) {
     const int32_t ns = *a.num_stray;
+    if (!EMIT) {
+        const int64_t nband = min((int64_t)*a.num_exact, a.nq_total);
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nband; i += (int64_t)gridDim.x * blockDim.x)
+            decide_band_pair(a, a.band_pairs[i]);
+    }
     for (int32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
         const int32_t t = a.stray[s];
         const float4 q = a.qsorted[t];
@@ -2219,7 +2479,7 @@ __global__ void stray_kernel(WalkArgs a) {
         int32_t n = 0;
         for (int o = 0; o < S; ++o) {
             int32_t beg, cnt;
-            stencil_lookup(a, u, qc, o, beg, cnt);
+            stencil_lookup_any(a, u, qc, o, beg, cnt);
             for (int32_t j = beg; j < beg + cnt; ++j) {
                 const float4 cv = a.rsorted[j];
                 const bool in = a.f64.qpos ? f64_pair_decide(a.f64, u.dim, u.periodic_mask, a.mode, qorig - u.qshift, j)
@@ -2591,6 +2851,7 @@ static WalkArgs make_walk(const HostBatch& b, const Structure& S, const Scratch&
     a.flagged = W.flagged;
     a.num_flagged = W.num_flagged;
     a.num_exact = W.num_exact;
+    a.band_pairs = reinterpret_cast<int4*>(W.pack);  // the packed points are sorted away by now
     a.cursor = W.cursor;
     a.query_ids = b.query_ids;
     a.ref_ids = b.ref_ids;
