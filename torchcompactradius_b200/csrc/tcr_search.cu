@@ -62,6 +62,7 @@ constexpr int64_t kBatchMapMin = 64;     // per cloud of a batch
 // one cloud class (cls = dim * 2 + periodic, 2..7) in a batch that mixes classes, [16 + the same]
 // for the count walk of the units recorded window by window.
 constexpr int kWorkCounters = 32;
+constexpr int kExpandCounter = 30;  // the record expansion
 
 // Default tuning of a search (tcr_search_desc / tcr_batch_desc unit_queries and walk_blocks_per_sm):
 // queries per work unit and resident walk blocks per SM.  Neither changes a result: a query's
@@ -132,7 +133,7 @@ struct Scratch {
     int32_t* exact_clouds;  // [1] clouds whose every pair takes the exact test
     int32_t* num_exact;     // [1] pairs inside the count walk's band, decided exactly
     int32_t* unit_cap;      // [1] queries per work unit of this search (set by the count phase)
-    unsigned long long* cursor;  // [1] staging fill
+    unsigned long long* cursor;  // [2] staging fill, staging capacity
     float4* pack;           // [max(nq,nr)] packed input points before sorting
     void* keys[2];          // [max(nq,nr)] 64-bit slots (32-bit keys use the first half)
     int32_t* vals[2];
@@ -180,7 +181,7 @@ static Scratch carve_scratch(void* buf, int64_t nq, int64_t nr, int64_t C, bool 
     s.exact_clouds = c.take<int32_t>(1);
     s.num_exact = c.take<int32_t>(1);
     s.unit_cap = c.take<int32_t>(1);
-    s.cursor = c.take<unsigned long long>(1);
+    s.cursor = c.take<unsigned long long>(2);
     s.pack = c.take<float4>(nmax);
     s.keys[0] = c.take<unsigned long long>(nmax);
     s.keys[1] = c.take<unsigned long long>(nmax);
@@ -469,7 +470,7 @@ __global__ void query_params_kernel(const CloudParams* __restrict__ table, const
 }
 
 // Zeroes the per-search counters, the per-cloud query statistics and the per-query counts.
-__global__ void count_init_kernel(Scratch W, int C, int unit_cap, int64_t nq) {
+__global__ void count_init_kernel(Scratch W, int C, int unit_cap, int64_t nq, int64_t stage_cap) {
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
         W.qparams[c].stats.max_key = 0;
         W.qparams[c].stats.bad = 0;
@@ -485,7 +486,8 @@ __global__ void count_init_kernel(Scratch W, int C, int unit_cap, int64_t nq) {
         *W.exact_clouds = 0;
         *W.num_exact = 0;
         *W.unit_cap = unit_cap;
-        *W.cursor = 0ull;
+        W.cursor[0] = 0ull;
+        W.cursor[1] = (unsigned long long)stage_cap;
     }
 }
 
@@ -2172,30 +2174,64 @@ __device__ __forceinline__ uint32_t top_set_bit(uint32_t m) {
     return b;
 }
 
-// Emit pass for staged units: expand each unit's record into its queries' CSR/COO slots, one warp
-// per unit, window by window of kExpandWin chunks.  The window's candidate columns are gathered
-// into shared memory once (consecutive sorted indices: coalesced reads of the sort index; each
-// lane finds its candidate's run by a rank in the window's run-start bitmap).  Lanes over
-// (query, chunk) pairs -- lane = query + nbp * g takes chunk g of each group of 32 / nbp chunks,
-// nbp the unit's query count rounded up to a power of two -- expand their hit bits into a shared
-// output table (query, chunk and bit of every output, in output order), and lanes over output
-// positions write consecutive slots.  A window of more than kExpandTab outputs is written query by
-// query instead.
+// Emit pass for staged units: expand each unit's record into its queries' CSR/COO slots, one warp per unit,
+// window by window of up to kExpandWin chunks.  The window's hit masks come into shared memory in
+// (query, chunk) order, an equal share of consecutive words per lane; every lane turns the set bits of its share
+// into 16-bit tags (word and bit) in the shared output table, which so is in output order.  The
+// window's candidate columns are gathered (consecutive sorted indices; each lane finds its candidate's run
+// by a rank in the window's run-start bitmap) and lanes over output positions write consecutive slots.
+//
+// The expansion is bound by issue slots (11% of the mask bits are set), then by the output's HBM
+// writes.  A lane walks its share in one loop over its set bits, all lanes together as many steps as the
+// fullest share has (42 of 25 on the 1M workload); a loop per word, as long as the fullest word of 32
+// each time, took 99.  Units are claimed one by one: a fixed share per warp left the SMs idle for 20% of the
+// 1M workload and 70% of a 65k one.
 constexpr int kExpandWarps = 8;
 constexpr int kExpandWin = 16;    // chunks per window: 512 candidates
 constexpr int kExpandTab = 1920;  // outputs one table holds (four blocks of eight warps fit an SM)
-constexpr int kExpandBatch = 8;   // global loads a lane issues before it waits for the first
 struct ExpandSmem {
-    int32_t col[kExpandWarps][kExpandWin * 32];    // output column of each candidate of the window
-    uint16_t tab[kExpandWarps][kExpandTab];        // (query << 9) | (chunk << 5) | bit, in output order
-    uint32_t rstart[kExpandWarps][kExpandWin];     // bit k of word c: a run starts at candidate 32 c + k
-    int32_t rrank[kExpandWarps][kExpandWin];       // runs starting before word c, minus one
-    int32_t run_beg[kExpandWarps][32];
-    int32_t run_pre[kExpandWarps][33];
+    union {
+        uint32_t word[kExpandWarps][kExpandWin * 32];  // hit masks: word i of lane L's share at 32 i + L
+        int32_t col[kExpandWarps][kExpandWin * 32];    // then the output column of each candidate of the window
+    };
+    uint16_t tab[kExpandWarps][kExpandTab];        // (word << 5) | bit of each output, word = query * chunks + chunk
+    uint2 starts[kExpandWarps][kExpandWin];        // per chunk: bit k, a run starts at its candidate k; runs before it, minus one
+    int32_t delta[kExpandWarps][32];               // per run: its first sorted index minus its first candidate
     long long* qcol[kExpandWarps][32];             // column output of table entry 0 of each query (this window)
-    int64_t qoff[kExpandWarps][32];                // output position of each query's next hit
     int32_t qrow[kExpandWarps][32];
 };
+// ceil(2^16 / k): x / k == x * kInverse[k] >> 16 for x < 2^16 / k.
+__constant__ uint32_t kInverse[33] = {0,    65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192, 7282, 6554,
+                                      5958, 5462,  5042,  4682,  4370,  4096,  3856,  3641, 3450, 3277, 3121,
+                                      2979, 2850,  2731,  2622,  2521,  2428,  2341,  2260, 2185, 2115, 2048};
+
+// One step of a lane through its share (words 128 bytes apart, last first): takes the next word when the
+// current one, m, is spent, and writes the tag of its highest set bit below pos.  Predicated by hand:
+// as branches the two halves diverge in every step (217 against 199 us for the 1M workload's expansion).
+__device__ __forceinline__ void expand_step(uint32_t base, uint32_t& at, uint32_t& m, uint32_t& tag, uint32_t& pos) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        ".reg .u32 b, t;\n"
+        ".reg .u16 h;\n"
+        "setp.gt.u32 p, %0, %4;\n"
+        "setp.eq.and.u32 p, %1, 0, p;\n"
+        "@p sub.u32 %0, %0, 128;\n"
+        "@p sub.u32 %2, %2, 32;\n"
+        "@p ld.shared.u32 %1, [%0];\n"
+        "setp.ne.u32 q, %1, 0;\n"
+        "bfind.u32 b, %1;\n"
+        "add.u32 t, %2, b;\n"
+        "cvt.u16.u32 h, t;\n"
+        "@q sub.u32 %3, %3, 2;\n"
+        "@q st.shared.u16 [%3], h;\n"
+        "shl.b32 t, 1, b;\n"  // (no bit: shifted out)
+        "xor.b32 %1, %1, t;\n"
+        "}\n"
+        : "+r"(at), "+r"(m), "+r"(tag), "+r"(pos)
+        : "r"(base)
+        : "memory");
+}
 
 struct ExpandArgs {
     const int32_t* __restrict__ stage;
@@ -2205,228 +2241,242 @@ struct ExpandArgs {
     const int32_t* __restrict__ unit_group;
     const int32_t* __restrict__ group_cloud;
     const int32_t* __restrict__ qsidx;
-    const int32_t* __restrict__ rsidx;
+    const int32_t* __restrict__ col_of;  // [nr] column of each sorted reference (composed: with ref_ids applied)
+    int32_t composed;
     const int64_t* __restrict__ offsets;
     const int32_t* __restrict__ query_ids;
-    const int32_t* __restrict__ ref_ids;
     const CloudParams* __restrict__ table;
     int32_t num_clouds;
     int32_t local_index;
     int64_t* __restrict__ row_out;
     int64_t* __restrict__ col_out;
     int64_t out_cap;
-    int64_t stage_cap, nq, nr;  // bounds of the checked build
+    int32_t* work;              // the next unit to claim
+    const unsigned long long* __restrict__ stage_cap;  // words of the staging list
+    int64_t nq, nr;
 };
 
-__global__ void __launch_bounds__(kExpandWarps * 32, 4) expand_records_kernel(ExpandArgs a) {
+__global__ void __launch_bounds__(kExpandWarps * 32, 4) expand_records_kernel(const __grid_constant__ ExpandArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ExpandSmem& sm = *reinterpret_cast<ExpandSmem*>(smem_raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int32_t nu = *a.num_units;
-    const int64_t warps = (int64_t)gridDim.x * kExpandWarps;
-    int32_t* __restrict__ rbeg = sm.run_beg[w];
-    int32_t* __restrict__ rpre = sm.run_pre[w];
+    uint32_t* __restrict__ word = sm.word[w];
     int32_t* __restrict__ cols = sm.col[w];
     uint16_t* __restrict__ tab = sm.tab[w];
-    int64_t u = (int64_t)blockIdx.x * kExpandWarps + w;
-    // A unit's record offset and first query are read two iterations before it runs, its record
-    // header (lanes 0..2) and query rows (lane < 32 covers every unit size) one iteration before,
-    // so a unit starts with its header at hand instead of two dependent round trips.
-    auto header = [&](int32_t r0) -> int32_t {
-        return (r0 >= 0 && lane < 3 && TCR_GUARD(r0 + 3, a.stage_cap)) ? a.stage[r0 + lane] : 0;
+    const uint32_t le = (2u << lane) - 1u;  // bits 0 .. lane
+    const int64_t cap = (int64_t)*a.stage_cap;
+    // A unit is claimed three iterations before it runs, its record offset and first query are read two
+    // before, its record's first 64 words (the header and the runs) and query rows (lane < 32 covers every
+    // unit size) one before, so a unit starts with them at hand instead of dependent round trips.
+    auto claim = [&]() -> int32_t { return lane == 0 ? atomicAdd(a.work, 1) : 0; };
+    auto words_of = [&](int32_t r0, int32_t k) -> int32_t {
+        return (r0 >= 0 && (int64_t)r0 + k < cap) ? a.stage[r0 + k] : 0;
     };
-    auto qrows = [&](int64_t v, int32_t t0) -> int32_t {
+    auto qrows = [&](int32_t v, int32_t t0) -> int32_t {
         return (v < nu && TCR_GUARD(t0 + lane, a.nq)) ? a.qsidx[t0 + lane] : -1;
     };
-    int32_t r0a = u < nu ? a.rec[u] : -1, t0a = u < nu ? a.unit_t0[u] : 0;
-    int32_t r0b = u + warps < nu ? a.rec[u + warps] : -1, t0b = u + warps < nu ? a.unit_t0[u + warps] : 0;
-    int32_t ha = header(r0a), qa = qrows(u, t0a);
-    for (; u < nu; u += warps) {
-        const int32_t r0 = r0a, hw = ha, qrow_l = qa;
-        ha = header(r0b);
-        qa = qrows(u + warps, t0b);
+    int32_t ua = __shfl_sync(0xffffffffu, claim(), 0);
+    int32_t ub = __shfl_sync(0xffffffffu, claim(), 0);
+    int32_t next = claim();
+    int32_t r0a = ua < nu ? a.rec[ua] : -1, t0a = ua < nu ? a.unit_t0[ua] : 0;
+    int32_t r0b = ub < nu ? a.rec[ub] : -1, t0b = ub < nu ? a.unit_t0[ub] : 0;
+    int32_t ha = words_of(r0a, lane), hb = words_of(r0a, 32 + lane), qa = qrows(ua, t0a);
+    while (ua < nu) {
+        const int32_t u = ua, r0 = r0a, h0 = ha, h1 = hb, qrow_l = qa;
+        ha = words_of(r0b, lane);
+        hb = words_of(r0b, 32 + lane);
+        qa = qrows(ub, t0b);
+        ua = ub;
         r0a = r0b;
-        t0a = t0b;
+        ub = __shfl_sync(0xffffffffu, next, 0);
         r0b = -1;
-        if (u + 2 * warps < nu) {
-            r0b = a.rec[u + 2 * warps];
-            t0b = a.unit_t0[u + 2 * warps];
+        if (ub < nu) {
+            r0b = a.rec[ub];
+            t0b = a.unit_t0[ub];
         }
+        next = claim();
         if (r0 < 0) continue;  // no candidates, or re-tested by the emit walk
-        if (!TCR_GUARD(r0 + 3, a.stage_cap)) continue;
-        const int32_t* rec = a.stage + r0;
-        const int32_t nchunks = __shfl_sync(0xffffffffu, hw, 0), R = __shfl_sync(0xffffffffu, hw, 1),
-                      nb = __shfl_sync(0xffffffffu, hw, 2);
-        if (!TCR_GUARD(R, 28) || !TCR_GUARD(nb - 1, 32) || !TCR_GUARD(r0 + record_words(R, nchunks, nb) - 1, a.stage_cap))
+        const int32_t nchunks = __shfl_sync(0xffffffffu, h0, 0), R = __shfl_sync(0xffffffffu, h0, 1),
+                      nb = __shfl_sync(0xffffffffu, h0, 2);
+        if (!TCR_GUARD(R, 28) || !TCR_GUARD(nb - 1, 32) || !TCR_GUARD(r0 + record_words(R, nchunks, nb) - 1, cap))
             continue;
+        const int32_t* rec = a.stage + r0;
         const uint32_t* masks = reinterpret_cast<const uint32_t*>(rec + kRecHeader + 2 * R + 1);
         int32_t rshift = 0, qshift = 0;
         if (a.local_index) {
             const CloudParams& cp = a.table[a.num_clouds == 1 ? 0 : a.group_cloud[a.unit_group[u]]];
-            rshift = cp.ref_base;
+            rshift = a.composed ? 0 : cp.ref_base;
             qshift = cp.query_base;
         }
-        if (lane < R) rbeg[lane] = rec[kRecHeader + lane];
-        if (lane <= R) rpre[lane] = rec[kRecHeader + R + lane];
-        if (lane < nb && TCR_GUARD(qrow_l, a.nq)) {
-            sm.qrow[w][lane] = a.query_ids ? a.query_ids[qrow_l] : qrow_l - qshift;
-            sm.qoff[w][lane] = a.offsets[qrow_l];
+        auto word_at = [&](int32_t k) -> int32_t {  // word k of the record, k < 64
+            const int32_t x = __shfl_sync(0xffffffffu, h0, k & 31), y = __shfl_sync(0xffffffffu, h1, k & 31);
+            return k < 32 ? x : y;
+        };
+        const int32_t beg = word_at(kRecHeader + lane);
+        const int32_t pre = word_at(min(kRecHeader + R + lane, 63));  // candidate prefix of the runs, then M
+        if (lane < R) sm.delta[w][lane] = beg - pre;
+        const int32_t M = __shfl_sync(0xffffffffu, pre, R);
+        const bool mine = lane < nb && TCR_GUARD(qrow_l, a.nq);
+        int64_t qoff = 0;  // lane q: output position of query q's next hit
+        if (mine) {
+            qoff = a.offsets[qrow_l];
+            if (a.row_out) sm.qrow[w][lane] = a.query_ids ? a.query_ids[qrow_l] : qrow_l - qshift;
         }
-        __syncwarp();
-        const int32_t M = rpre[R];
-        // lane = q + nbp * g: query q, chunk g of each group of G chunks
-        const int lg = nb > 1 ? 32 - __clz(nb - 1) : 0;
-        const int nbp = 1 << lg, G = 32 >> lg;
-        const int q = lane & (nbp - 1), g = lane >> lg;
-        const bool qlane = q < nb;
-        for (int32_t c0 = 0; c0 < nchunks; c0 += kExpandWin) {
-            const int32_t nc = min(kExpandWin, nchunks - c0);
-            const int32_t wbase = c0 << 5;
-            // the window's masks, in registers: lane (q, g) holds the masks of chunks g, g + G, ...
-            // (G = 1 when the unit has more than 16 queries), all loaded at the window's start;
-            // consecutive lanes read consecutive words
-            const uint32_t* src = masks + (int64_t)c0 * nb;
-            uint32_t mv[kExpandWin];
-#pragma unroll
-            for (int t = 0; t < kExpandWin; ++t) {
-                const int32_t c = g + G * t;
-                mv[t] = (qlane && c < nc) ? __ldcs(&src[c * nb + q]) : 0u;
-            }
-            // run of candidate wbase + k: the runs starting at or before it, minus one
-            if (lane < kExpandWin) sm.rstart[w][lane] = 0u;
-            __syncwarp();
-            const bool rl = lane < R;
-            const int32_t rs = rl ? rpre[lane] - wbase : -1;
-            const int32_t nbefore = __popc(__ballot_sync(0xffffffffu, rl && rs < 0));
-            if (rl && rs >= 0 && rs < (nc << 5)) atomicOr(&sm.rstart[w][rs >> 5], 1u << (rs & 31));
-            __syncwarp();
-            const int32_t wp = lane < kExpandWin ? __popc(sm.rstart[w][lane]) : 0;
-            const int32_t wpi = warp_inclusive_scan(wp);
-            if (lane < kExpandWin) sm.rrank[w][lane] = nbefore + wpi - wp - 1;
-            __syncwarp();
-            // the window's candidate columns, the loads of each batch issued together so that their
-            // latencies overlap (one load waited for at a time left the warps idle)
-            const uint32_t le = (2u << lane) - 1u;  // bits 0 .. lane
-            for (int32_t cc0 = 0; cc0 < nc; cc0 += kExpandBatch) {
-                int32_t jl[kExpandBatch];
-                bool ok[kExpandBatch];
-#pragma unroll
-                for (int i = 0; i < kExpandBatch; ++i) {
-                    const int32_t cc = cc0 + i;
-                    const int32_t k = wbase + (cc << 5) + lane;
-                    jl[i] = 0;
-                    ok[i] = false;
-                    if (cc < nc && k < M) {
-                        const int32_t cr = sm.rrank[w][cc] + __popc(sm.rstart[w][cc] & le);
-                        if (TCR_GUARD(cr, R)) {
-                            const int32_t j = rbeg[cr] + (k - rpre[cr]);
-                            ok[i] = true;
-                            if (TCR_GUARD(j, a.nr)) jl[i] = __ldg(&a.rsidx[j]);
-                        }
-                    }
-                }
-                int32_t col[kExpandBatch];
-#pragma unroll
-                for (int i = 0; i < kExpandBatch; ++i)
-                    col[i] = !ok[i] ? 0 : (a.ref_ids ? __ldg(&a.ref_ids[jl[i]]) : jl[i] - rshift);
-#pragma unroll
-                for (int i = 0; i < kExpandBatch; ++i)
-                    if (cc0 + i < nc) cols[((cc0 + i) << 5) + lane] = col[i];
-            }
-            __syncwarp();
-            // the window's outputs of each query, and their exclusive prefix over the queries
-            int32_t tot = 0;
-#pragma unroll
-            for (int t = 0; t < kExpandWin; ++t) tot += __popc(mv[t]);
-            for (int sft = nbp; sft < 32; sft <<= 1) tot += __shfl_xor_sync(0xffffffffu, tot, sft);
-            const int32_t tv = (g == 0 && qlane) ? tot : 0;
-            const int32_t tinc = warp_inclusive_scan(tv);
-            const int32_t n = __shfl_sync(0xffffffffu, tinc, 31);
-            const int32_t qpre = __shfl_sync(0xffffffffu, tinc - tv, q);
-            if (n <= kExpandTab) {
-                // each lane expands its (query, chunk) mask into the table, highest bit at the end
-                int32_t run = qpre;  // table slot of the query's next output
-#pragma unroll
-                for (int t = 0; t < kExpandWin; ++t) {
-                    if (G * t >= nc) break;
-                    const int32_t c = G * t + g;
-                    uint32_t m = mv[t];
-                    int32_t inc = __popc(m);
-                    for (int sft = nbp; sft < 32; sft <<= 1) {  // inclusive scan over g, per query
-                        const int32_t t = __shfl_up_sync(0xffffffffu, inc, sft);
-                        if (lane >= sft) inc += t;
-                    }
-                    const int32_t tq = __shfl_sync(0xffffffffu, inc, q + 32 - nbp);
-                    int32_t pos = run + inc;
-                    const uint32_t tag = ((uint32_t)q << 9) | ((uint32_t)c << 5);
-                    while (m) {
-                        const uint32_t bit = top_set_bit(m);
-                        m ^= 1u << bit;
-                        tab[--pos] = (uint16_t)(tag | bit);
-                    }
-                    run += tq;
-                }
-                // per query: the output slot of its table entry 0, and whether all of the window's
-                // outputs fit the output buffer (then the column-only loop writes without checks)
-                bool fits = true;
-                if (g == 0 && qlane) {
-                    sm.qcol[w][q] = reinterpret_cast<long long*>(a.col_out) + (sm.qoff[w][q] - qpre);
-                    fits = sm.qoff[w][q] + tot <= a.out_cap;
-                }
-                fits = __all_sync(0xffffffffu, fits);
+        const uint32_t inb = kInverse[nb];
+        int32_t nc = 0;
+        for (int32_t c0 = 0; c0 < nchunks; c0 += nc) {
+            nc = min(kExpandWin, nchunks - c0);
+            int32_t words, share, nw, bits, steps, end, n;
+            for (;;) {
+                // the window's masks: read in the record's order (chunk, query), stored in output order
+                words = nb * nc;
+                share = (words + 31) >> 5;
+                const uint32_t ishare = kInverse[share];
+                const uint32_t* src = masks + (int64_t)c0 * nb;
                 __syncwarp();
-                const bool rows = a.row_out != nullptr;
-                if (fits && !rows) {
-#pragma unroll 4
-                    for (int32_t o = lane; o < n; o += 32) {
-                        const uint32_t v = tab[o];
-                        __stcs(sm.qcol[w][v >> 9] + o, (long long)cols[v & 0x1ffu]);
+                auto place = [&](int32_t i0, auto count) {
+                    constexpr int N = decltype(count)::value;
+                    uint32_t m[N];
+#pragma unroll
+                    for (int i = 0; i < N; ++i) {
+                        const int32_t x = ((i0 + i) << 5) + lane;
+                        m[i] = x < words ? __ldcs(&src[x]) : 0u;
                     }
-                } else if (fits) {  // COO: the row of an output sits at the same slot of row_out
-                    const int64_t rd = ((intptr_t)a.row_out - (intptr_t)a.col_out) / 8;  // both int64-aligned
-#pragma unroll 4
-                    for (int32_t o = lane; o < n; o += 32) {
-                        const uint32_t v = tab[o];
-                        const uint32_t vq = v >> 9;
-                        long long* p = sm.qcol[w][vq] + o;
-                        __stcs(p, (long long)cols[v & 0x1ffu]);
-                        __stcs(p + rd, (long long)sm.qrow[w][vq]);
+#pragma unroll
+                    for (int i = 0; i < N; ++i) {
+                        const uint32_t x = ((i0 + i) << 5) + lane;
+                        const uint32_t c = (x * inb) >> 16, q = x - c * nb, v = q * nc + c;
+                        const uint32_t owner = (v * ishare) >> 16;
+                        if (x < (uint32_t)words) word[((v - owner * share) << 5) + owner] = m[i];
                     }
+                };
+                if (share > 4)
+                    for (int32_t i0 = 0; i0 < share; i0 += 8) place(i0, std::integral_constant<int, 8>());
+                else
+                    place(0, std::integral_constant<int, 4>());
+                __syncwarp();
+                nw = min(max(words - lane * share, 0), share);  // words of this lane's share
+                bits = 0;
+                steps = 0;
+                for (int32_t i = 0; i < nw; ++i) {
+                    const int32_t p = __popc(word[(i << 5) + lane]);
+                    bits += p;
+                    steps += max(p, 1);
+                }
+                end = warp_inclusive_scan(bits);
+                n = __shfl_sync(0xffffffffu, end, 31);
+                if (n <= kExpandTab) break;
+                nc = (nc + 1) >> 1;  // more outputs than the table holds (one chunk's always fit)
+            }
+            // lane q: the table entries before query q's first (its first word is word `off` of lane `owner`'s
+            // share), and its own
+            int32_t qpre, qv;
+            {
+                const int32_t first = min(lane, nb) * nc, owner = min((int32_t)((first * kInverse[share]) >> 16), 31),
+                              off = first - owner * share;
+                qpre = __shfl_sync(0xffffffffu, end - bits, owner);
+                for (int32_t i = 0; i < off; ++i) qpre += first < words ? __popc(word[(i << 5) + owner]) : 0;
+                if (first >= words) qpre = n;
+                qv = __shfl_down_sync(0xffffffffu, qpre, 1) - qpre;
+                if (lane >= nb) qv = 0;
+                else if (lane == 31) qv = n - qpre;
+            }
+            // every lane expands its share, last word and highest bit first
+            {
+                const uint32_t base = (uint32_t)__cvta_generic_to_shared(word) + 4 * lane;
+                uint32_t pos = (uint32_t)__cvta_generic_to_shared(tab) + 2 * end;
+                uint32_t at = base + 128 * nw, m = 0, tag = (uint32_t)(lane * share + nw) << 5;
+                const int32_t T = __reduce_max_sync(0xffffffffu, steps);
+                for (int32_t t = 0; t < T; t += 4) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) expand_step(base, at, m, tag, pos);
+                }
+            }
+            // the window's runs: start bits and ranks
+            const int32_t wbase = c0 << 5;
+            if (lane < kExpandWin) sm.starts[w][lane] = make_uint2(0u, 0u);
+            __syncwarp();
+            const int32_t at = pre - wbase;
+            if (lane < R && at >= 0 && at < (nc << 5)) atomicOr(&sm.starts[w][at >> 5].x, 1u << (at & 31));
+            const int32_t before = __popc(__ballot_sync(0xffffffffu, lane < R && at < 0));
+            __syncwarp();
+            const int32_t here = lane < kExpandWin ? __popc(sm.starts[w][lane].x) : 0;
+            const int32_t upto = before + warp_inclusive_scan(here) - 1;
+            if (lane < kExpandWin) sm.starts[w][lane].y = (uint32_t)(upto - here);
+            __syncwarp();
+            // the candidate columns, in place of the masks; the loads of each batch issued together so that
+            // their latencies overlap (lanes past the last candidate repeat it)
+            auto gather = [&](int32_t cc0, auto count) {
+                constexpr int N = decltype(count)::value;
+                int32_t jl[N];
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    const int32_t cc = min(cc0 + i, nc - 1);
+                    const uint2 st = sm.starts[w][cc];
+                    const int32_t run = (int32_t)st.y + __popc(st.x & le);
+                    const int32_t j = sm.delta[w][run & 31] + min(wbase + (cc << 5) + lane, M - 1);
+                    jl[i] = TCR_GUARD(j, a.nr) ? __ldg(&a.col_of[j]) : 0;
+                }
+#pragma unroll
+                for (int i = 0; i < N; ++i)
+                    if (cc0 + i < nc) cols[((cc0 + i) << 5) + lane] = jl[i] - rshift;
+            };
+            for (int32_t cc0 = 0; cc0 < nc;) {
+                if (nc - cc0 > 4) {
+                    gather(cc0, std::integral_constant<int, 8>());
+                    cc0 += 8;
                 } else {
+                    gather(cc0, std::integral_constant<int, 4>());
+                    cc0 += 4;
+                }
+            }
+            // per query: the output slot of its table entry 0, and whether all of the window's outputs
+            // fit the output buffer (then the loops write without checks)
+            sm.qcol[w][lane] = reinterpret_cast<long long*>(a.col_out) + (qoff - qpre);
+            const bool fits = __all_sync(0xffffffffu, !mine || qoff + qv <= a.out_cap);
+            qoff += qv;
+            __syncwarp();
+            const uint32_t inc = kInverse[nc], per = (uint32_t)nc << 5;
+            if (fits && !a.row_out) {
 #pragma unroll 4
-                    for (int32_t o = lane; o < n; o += 32) {
-                        const uint32_t v = tab[o];
-                        const uint32_t vq = v >> 9;
-                        const int64_t pos = (sm.qcol[w][vq] - reinterpret_cast<long long*>(a.col_out)) + o;
-                        if (TCR_GUARD(pos, a.out_cap)) {
-                            __stcs(reinterpret_cast<long long*>(&a.col_out[pos]), (long long)cols[v & 0x1ffu]);
-                            if (rows) __stcs(reinterpret_cast<long long*>(&a.row_out[pos]), (long long)sm.qrow[w][vq]);
-                        }
-                    }
+                for (int32_t o = lane; o < n; o += 32) {
+                    const uint32_t v = tab[o], q = ((v >> 5) * inc) >> 16;
+                    __stcs(sm.qcol[w][q] + o, (long long)(uint32_t)cols[v - q * per]);
+                }
+            } else if (fits) {  // COO: the row of an output sits at the same slot of row_out
+                const int64_t rd = ((intptr_t)a.row_out - (intptr_t)a.col_out) / 8;  // both int64-aligned
+#pragma unroll 4
+                for (int32_t o = lane; o < n; o += 32) {
+                    const uint32_t v = tab[o], q = ((v >> 5) * inc) >> 16;
+                    long long* p = sm.qcol[w][q] + o;
+                    __stcs(p, (long long)(uint32_t)cols[v - q * per]);
+                    __stcs(p + rd, (long long)sm.qrow[w][q]);
                 }
             } else {
-                // many outputs: query by query, lanes over the window's chunks
-                for (int32_t qq = 0; qq < nb; ++qq) {
-                    uint32_t m = lane < nc ? __ldcs(&src[lane * nb + qq]) : 0u;
-                    const int32_t cnt = __popc(m);
-                    const int32_t inc = warp_inclusive_scan(cnt);
-                    int64_t pos = sm.qoff[w][qq] + (inc - cnt);
-                    const long long row = sm.qrow[w][qq];
-                    while (m) {
-                        const int bit = __ffs(m) - 1;
-                        m &= m - 1;
-                        if (TCR_GUARD(pos, a.out_cap)) {
-                            a.col_out[pos] = (int64_t)cols[(lane << 5) + bit];
-                            if (a.row_out) a.row_out[pos] = row;
-                        }
-                        ++pos;
+                for (int32_t o = lane; o < n; o += 32) {
+                    const uint32_t v = tab[o], q = ((v >> 5) * inc) >> 16;
+                    const int64_t pos = (sm.qcol[w][q] - reinterpret_cast<long long*>(a.col_out)) + o;
+                    if (TCR_GUARD(pos, a.out_cap)) {
+                        __stcs(reinterpret_cast<long long*>(&a.col_out[pos]), (long long)(uint32_t)cols[v - q * per]);
+                        if (a.row_out) __stcs(reinterpret_cast<long long*>(&a.row_out[pos]), (long long)sm.qrow[w][q]);
                     }
                 }
             }
             __syncwarp();
-            if (g == 0 && qlane) sm.qoff[w][q] += tot;
-            __syncwarp();
         }
+    }
+}
+
+// The caller's id of every sorted reference, for the expansion of a search with ref_ids: composed once
+// here, where composing it per unit read the ids 27 times over in random order (0.25 of 0.43 ms for 500k
+// adaptive points).
+__global__ void compose_ids_kernel(const int32_t* __restrict__ rsidx, const int32_t* __restrict__ ref_ids, int64_t n,
+                                   int32_t* __restrict__ out) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
+        const int32_t p = rsidx[j];
+        out[j] = TCR_GUARD(p, n) ? ref_ids[p] : 0;
     }
 }
 
@@ -3019,7 +3069,7 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
     int rc = upload_table(b, W, st);
     if (rc) return rc;
     const int unit_cap = b.unit_cap;
-    count_init_kernel<<<grid_for(std::max<int64_t>(C, nq), 256), 256, 0, st>>>(W, C, unit_cap, nq);
+    count_init_kernel<<<grid_for(std::max<int64_t>(C, nq), 256), 256, 0, st>>>(W, C, unit_cap, nq, stage_cap);
     note_launches(1);
     if (b.any_query_sup && nq > 0 && !b.same_sorted) {
         support_stats_kernel<<<grid_for(nq, 256, num_sms() * 4), 256, 0, st>>>(
@@ -3102,10 +3152,12 @@ static int emit_impl(const HostBatch& b, const Structure& S, const Scratch& W, c
     a.row_out = row_out;
     a.col_out = col_out;
     a.out_cap = out_capacity;
+    TCR_CUDA(cudaMemsetAsync(W.work, 0, sizeof(int32_t) * kWorkCounters, st));
     if (stage) {
         const int nsm = num_sms();
+        // resident blocks (four an SM), no more than about two units per query group's worth of full ones
         const unsigned blocks = (unsigned)std::max<int64_t>(
-            1, std::min<int64_t>((int64_t)nsm * 16, (nq / 16 + kExpandWarps) / kExpandWarps));
+            1, std::min<int64_t>((int64_t)nsm * 4, (2 * nq / b.unit_cap + kExpandWarps) / kExpandWarps));
         ExpandArgs e;
         e.stage = stage;
         e.rec = W.rec;
@@ -3114,17 +3166,23 @@ static int emit_impl(const HostBatch& b, const Structure& S, const Scratch& W, c
         e.unit_group = W.unit_group;
         e.group_cloud = a.group_cloud;
         e.qsidx = a.qsidx;
-        e.rsidx = S.rsidx;
+        e.col_of = S.rsidx;
+        if (b.ref_ids && b.nr > 0) {  // (the sort's values are spent by now)
+            compose_ids_kernel<<<grid_for(b.nr, 256), 256, 0, st>>>(S.rsidx, b.ref_ids, b.nr, W.vals[0]);
+            note_launches(1);
+            e.col_of = W.vals[0];
+        }
         e.offsets = offsets;
         e.query_ids = b.query_ids;
-        e.ref_ids = b.ref_ids;
+        e.composed = b.ref_ids ? 1 : 0;
         e.table = W.table;
         e.num_clouds = b.C;
         e.local_index = b.local_index;
         e.row_out = row_out;
         e.col_out = col_out;
         e.out_cap = out_capacity;
-        e.stage_cap = 0x7fffffffLL;  // the records lie below the staging capacity of tcr_count (< 2^31 words)
+        e.work = W.work + kExpandCounter;
+        e.stage_cap = W.cursor + 1;
         e.nq = nq;
         e.nr = b.nr;
         static uint64_t expand_attr_done = 0;
@@ -3134,7 +3192,6 @@ static int emit_impl(const HostBatch& b, const Structure& S, const Scratch& W, c
         prof_mark(TCR_PROFILE_EXPAND, 1, st);
         note_launches(1);
     }
-    TCR_CUDA(cudaMemsetAsync(W.work, 0, sizeof(int32_t) * kWorkCounters, st));
     TCR_CUDA(launch_walks<EmitLaunch>(b, a, dim3(walk_blocks(b, nq)), dim3(kWalkWarps * 32), 0, st));
     stray_kernel<true><<<grid_for(nq, 128, num_sms() * 4), 128, 0, st>>>(a);
     note_launches(1);
