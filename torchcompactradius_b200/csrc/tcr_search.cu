@@ -84,7 +84,7 @@ struct Carve {
 // Persistent structure (reference side); kept alive for reuse.
 struct Structure {
     GridParams* grid;         // [C] per cloud
-    int32_t* num_cells;       // [1]
+    int32_t* num_cells;       // [2] cells; set when a one-launch sort gave up waiting
     int32_t* bad_grids;       // [1] clouds with points on both sides and no valid grid
     float4* rsorted;          // [nr] wrapped reference points in (cloud, cell) order, .w = support
     int32_t* rsidx;           // [nr] global index of each sorted point
@@ -101,7 +101,7 @@ static Structure carve_structure(void* buf, int64_t nr, int64_t C, int64_t map_t
     Carve c{(char*)buf, 0};
     Structure s;
     s.grid = c.take<GridParams>(C);
-    s.num_cells = c.take<int32_t>(1);
+    s.num_cells = c.take<int32_t>(2);
     s.bad_grids = c.take<int32_t>(1);
     s.rsorted = c.take<float4>(nr);
     s.rsidx = c.take<int32_t>(nr);
@@ -358,7 +358,7 @@ __global__ void grid_init_kernel(GridParams* g, int C, Structure S, Scratch W) {
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *S.bad_grids = 0;
-        *S.num_cells = 0;
+        S.num_cells[0] = S.num_cells[1] = 0;
         sort_state_reset(reinterpret_cast<SortStateT<K>*>(W.sort_state));
     }
 }
@@ -665,38 +665,37 @@ __device__ __forceinline__ int32_t map_find(const unsigned long long* __restrict
     return -1;
 }
 
-// Run starts of the sorted keys (unique_consecutive, hashTable.py:193).
+// What the build does with its sorted points: places each one (the point, its input index and, for the
+// serving loop, its linear cell and input index), and writes one cell record per run of equal keys
+// (unique_consecutive, hashTable.py:193): begin, lin, cloud, coords of the run's first point, bucket, and
+// the cell's entry in its cloud's map region.
 template <typename K>
-struct RunFlagIn {
-    const K* keys0;
-    const K* keys1;
-    const SortStateT<K>* st;
-    __device__ int32_t operator()(int64_t i) const {
-        const K* k = st->sel[key_passes<K>()] ? keys1 : keys0;
-        return (i == 0 || k[i] != k[i - 1]) ? 1 : 0;
-    }
-};
-
-// Writes one cell record per run start: begin, lin, cloud, coords of the run's first point,
-// bucket, and the cell's entry in its cloud's map region.
-template <typename K>
-struct CellOut {
+struct BuildTail {
+    static constexpr bool kPlace = true, kRuns = true;
+    int32_t* starts;   // cell_start
+    int32_t* num_runs;
+    const float4* __restrict__ pack;
+    float4* sorted;
+    int32_t* sidx;
+    int32_t* lin_out;
+    int32_t* order_out;
     const CloudParams* table;
     const GridParams* grid;
-    const K* keys0;
-    const K* keys1;
-    const SortStateT<K>* st;
-    const float4* rsorted;
-    int32_t* cell_start;
     int32_t* cell_lin;
     int32_t* cell_coords;
     int32_t* cell_bucket;
     int32_t* cell_cloud;
     unsigned long long* map;
-    int32_t n_points;
-    __device__ void write(int64_t i, int32_t ex) const {
-        const K* k = st->sel[key_passes<K>()] ? keys1 : keys0;
-        const K key = k[i];
+    int64_t n;
+    __device__ __forceinline__ void place(int64_t i, K key, int32_t p) const {
+        if (!TCR_GUARD(p, n)) return;
+        sorted[i] = pack[p];
+        sidx[i] = p;
+        if (lin_out) lin_out[i] = (int32_t)(key_low(key) ^ 0x80000000u);
+        if (order_out) order_out[i] = p;
+    }
+    __device__ __forceinline__ void run(const K* keys, int64_t i, int32_t cell) const {
+        const K key = keys[i];
         const int cloud = key_cloud(key);
         const int32_t lin = (int32_t)(key_low(key) ^ 0x80000000u);
         const CloudParams& cp = table[cloud];
@@ -704,83 +703,50 @@ struct CellOut {
         int32_t c[3] = {0, 0, 0};
         uint32_t bucket = 0;
         if (!g.error) {
-            cell_of(cp.dim, cp.dedupe, cp.dmin, g.hcell_d, g.count, rsorted[i], c);
+            cell_of(cp.dim, cp.dedupe, cp.dmin, g.hcell_d, g.count, sorted[i], c);
             bucket = ref_hash(cp.dim, c, cp.hash_len);
-            map_insert(map + cp.map_base, cp.map_cap, lin, ex);
+            map_insert(map + cp.map_base, cp.map_cap, lin, cell);
         }
-        cell_start[ex] = (int32_t)i;
-        cell_lin[ex] = lin;
-        cell_cloud[ex] = cloud;
-        cell_coords[3 * ex + 0] = c[0];
-        cell_coords[3 * ex + 1] = c[1];
-        cell_coords[3 * ex + 2] = c[2];
-        cell_bucket[ex] = (int32_t)bucket;
+        cell_lin[cell] = lin;
+        cell_cloud[cell] = cloud;
+        cell_coords[3 * cell + 0] = c[0];
+        cell_coords[3 * cell + 1] = c[1];
+        cell_coords[3 * cell + 2] = c[2];
+        cell_bucket[cell] = (int32_t)bucket;
     }
 };
 
-// The run-start scan writes only where each cell begins; the cell records are then written by one
-// thread per cell (a run start is one element in 16 here, so doing that work inside the scan left
-// most lanes of every warp idle behind a long chain of dependent loads and the map insert).
-struct CellStartOut {
-    int32_t* cell_start;
-    int32_t n_points;
-    __device__ void operator()(int64_t i, int32_t ex, int32_t flag) const {
-        if (flag && TCR_IN(ex, n_points)) cell_start[ex] = (int32_t)i;
-    }
-};
+// The same for queries sorted by their own cells: one query group per run.
 template <typename K>
-__global__ void cell_records_kernel(CellOut<K> co, const int32_t* __restrict__ num_cells, int64_t n) {
-    const int32_t nc = *num_cells;
-    if (blockIdx.x == 0 && threadIdx.x == 0) co.cell_start[nc] = (int32_t)n;  // end of the last cell
-    for (int32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        const int32_t i = co.cell_start[c];
-        if (TCR_GUARD(i, n)) co.write(i, c);
-    }
-}
-
-// lin_out (optional): the linear cell of each sorted point, the hint of the next incremental build;
-// order_out (optional): a copy of the sort index.
-// The build's consumer of its sort: the sorted points, their input indices and (for the serving
-// loop) each point's linear cell and input index, written as the sort's last pass places them.
-template <typename K>
-struct SortedPointsOut {
-    static constexpr bool kActive = true;
+struct QueryTail {
+    static constexpr bool kPlace = true, kRuns = true;
+    int32_t* starts;   // qgroup_start
+    int32_t* num_runs;
     const float4* __restrict__ pack;
-    float4* __restrict__ sorted;
-    int32_t* __restrict__ sidx;
-    int32_t* __restrict__ lin_out;
-    int32_t* __restrict__ order_out;
+    float4* sorted;
+    int32_t* sidx;
+    const CloudParams* table;
+    const GridParams* grid;
+    int32_t* group_coords;
+    int32_t* group_cloud;
     int64_t n;
-    __device__ __forceinline__ void operator()(int64_t i, K key, int32_t p) const {
-        if (!TCR_IN(p, n)) return;
+    __device__ __forceinline__ void place(int64_t i, K, int32_t p) const {
+        if (!TCR_GUARD(p, n)) return;
         sorted[i] = pack[p];
         sidx[i] = p;
-        if (lin_out) lin_out[i] = (int32_t)(key_low(key) ^ 0x80000000u);
-        if (order_out) order_out[i] = p;
+    }
+    __device__ __forceinline__ void run(const K* keys, int64_t i, int32_t group) const {
+        const int cloud = key_cloud(keys[i]);
+        const CloudParams& cp = table[cloud];
+        const GridParams& g = grid[cloud];
+        int32_t c[3] = {0, 0, 0};
+        if (!g.error) cell_of(cp.dim, cp.dedupe, cp.dmin, g.hcell_d, g.count, sorted[i], c);
+        group_cloud[group] = cloud;
+        group_coords[3 * group + 0] = c[0];
+        group_coords[3 * group + 1] = c[1];
+        group_coords[3 * group + 2] = c[2];
     }
 };
-
-// The same placement when the sort's last pass did not do it (no pass moved the points, or an
-// incremental build's merge ordered them).
-template <typename K>
-__global__ void gather_sorted_kernel(const float4* __restrict__ pack, const int32_t* vals0, const int32_t* vals1,
-                                     const SortStateT<K>* st, int64_t n, float4* __restrict__ sorted,
-                                     int32_t* __restrict__ sidx, const K* keys0 = nullptr, const K* keys1 = nullptr,
-                                     int32_t* __restrict__ lin_out = nullptr,
-                                     int32_t* __restrict__ order_out = nullptr) {
-    if (st->consumed) return;
-    const int32_t* v = st->sel[key_passes<K>()] ? vals1 : vals0;
-    const K* k = st->sel[key_passes<K>()] ? keys1 : keys0;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const int32_t p = v[i];
-        if (!TCR_IN(p, n)) continue;
-        sorted[i] = pack[p];
-        sidx[i] = p;
-        if (lin_out) lin_out[i] = (int32_t)(key_low(k[i]) ^ 0x80000000u);
-        if (order_out) order_out[i] = p;
-    }
-}
 
 // ------------------------------------------------------------------------------------------
 // incremental re-sort
@@ -906,34 +872,6 @@ __global__ void pack_self_queries_kernel(const CloudParams* __restrict__ table, 
         qsidx[t] = i;
     }
 }
-
-template <typename K>
-struct QueryGroupOut {
-    const CloudParams* table;
-    const GridParams* grid;
-    const K* keys0;
-    const K* keys1;
-    const SortStateT<K>* st;
-    const float4* qsorted;
-    int32_t* group_start;
-    int32_t* group_coords;
-    int32_t* group_cloud;
-    int32_t n_points;
-    __device__ void operator()(int64_t i, int32_t ex, int32_t flag) const {
-        if (!flag) return;
-        const K* k = st->sel[key_passes<K>()] ? keys1 : keys0;
-        const int cloud = key_cloud(k[i]);
-        const CloudParams& cp = table[cloud];
-        const GridParams& g = grid[cloud];
-        int32_t c[3] = {0, 0, 0};
-        if (!g.error) cell_of(cp.dim, cp.dedupe, cp.dmin, g.hcell_d, g.count, qsorted[i], c);
-        group_start[ex] = (int32_t)i;
-        group_cloud[ex] = cloud;
-        group_coords[3 * ex + 0] = c[0];
-        group_coords[3 * ex + 1] = c[1];
-        group_coords[3 * ex + 2] = c[2];
-    }
-};
 
 // Group count comes from a device scalar; the scan kernels are launched over the upper bound
 // and read the true count through the functor.  A unit holds at most `cap` (<= 32) queries.
@@ -2618,11 +2556,11 @@ struct OffsetOut {
     }
 };
 
-__global__ void info_kernel(const int32_t* bad_grids, const int64_t* total, const int32_t* num_stray,
+__global__ void info_kernel(const int32_t* bad_grids, const int32_t* num_cells, const int64_t* total, const int32_t* num_stray,
                             const int32_t* exact_clouds, const unsigned long long* cursor, const int32_t* num_flagged,
                             const int32_t* num_exact, const int32_t* inc_count, int64_t n_ref, int64_t* info) {
     info[0] = *total;
-    info[1] = *bad_grids;
+    info[1] = num_cells[1] ? -1 : *bad_grids;  // -1: a wait inside the sort gave up, nothing here is valid
     info[2] = *num_stray;
     info[3] = *exact_clouds;
     info[4] = (int64_t)*cursor;
@@ -3035,27 +2973,21 @@ static int build_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
                                                                    W.inc_count, W.inc_count + 1);
             inc_decide_kernel<K><<<1, 1, 0, st>>>(sw.state, mw.state, W.inc_count, nr);
             note_launches(2);
-            TCR_CUDA(radix_sort_pairs<K>(mw, nr, st));
+            TCR_CUDA(sort_coop<K>(mw, nr, S.num_cells + 1, NoTail(), st));
             inc_merge_kernel<K><<<grid_for(nr, 256), 256, 0, st>>>(
                 reinterpret_cast<const K*>(W.stay_keys), W.stay_idx, mw.keys[0], mw.keys[1], mw.vals[0], mw.vals[1],
                 mw.state, W.inc_count, nr, sw.keys[0], sw.vals[0]);
             note_launches(1);
         }
-        TCR_CUDA(radix_sort_pairs<K>(sw, nr, st, SortedPointsOut<K>{W.pack, S.rsorted, S.rsidx, b.lin_out, b.order_out, nr}));
-        gather_sorted_kernel<K><<<grid_for(nr, 256), 256, 0, st>>>(W.pack, sw.vals[0], sw.vals[1], sw.state, nr,
-                                                                   S.rsorted, S.rsidx, sw.keys[0], sw.keys[1],
-                                                                   b.lin_out, b.order_out);
-        note_launches(1);
-        RunFlagIn<K> fi{sw.keys[0], sw.keys[1], sw.state};
-        TCR_CUDA(device_exclusive_scan<int32_t>(fi, CellStartOut{S.cell_start, (int32_t)nr}, nr, W.scan_tiles32,
-                                                S.num_cells, st));
-        CellOut<K> co{W.table, S.grid, sw.keys[0], sw.keys[1], sw.state, S.rsorted, S.cell_start, S.cell_lin,
-                      S.cell_coords, S.cell_bucket, S.cell_cloud, S.map, (int32_t)nr};
-        cell_records_kernel<K><<<grid_for(nr, 256, num_sms() * 8), 256, 0, st>>>(co, S.num_cells, nr);
+        TCR_CUDA(sort_coop<K>(sw, nr, S.num_cells + 1,
+                              BuildTail<K>{S.cell_start, S.num_cells, W.pack, S.rsorted, S.rsidx, b.lin_out, b.order_out,
+                                           W.table, S.grid, S.cell_lin, S.cell_coords, S.cell_bucket, S.cell_cloud,
+                                           S.map, nr},
+                              st));
     } else {
         finish_cells_kernel<<<1, 1, 0, st>>>(S.cell_start, S.num_cells, nr);
+        note_launches(1);
     }
-    note_launches(1);
     TCR_CUDA(cudaGetLastError());
     return TCR_OK;
 }
@@ -3104,16 +3036,10 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
             pack_points_kernel<K><<<grid_for(nq, 256, num_sms() * 4), 256, 0, st>>>(
                 W.table, S.grid, W.query_prefix, C, nq, 1, 1, 0, W.pack, sw.keys[0], sw.vals[0], sw.state);
             note_launches(1);
-            TCR_CUDA(radix_sort_pairs<K>(sw, nq, st));
-            gather_sorted_kernel<K><<<grid_for(nq, 256), 256, 0, st>>>(W.pack, sw.vals[0], sw.vals[1], sw.state, nq,
-                                                                       W.qsorted, W.qsidx);
-            note_launches(1);
-            QueryGroupOut<K> qo{W.table, S.grid, sw.keys[0], sw.keys[1], sw.state, W.qsorted,
-                                W.qgroup_start, W.qgroup_coords, W.qgroup_cloud, (int32_t)nq};
-            RunFlagIn<K> fi{sw.keys[0], sw.keys[1], sw.state};
-            TCR_CUDA(device_exclusive_scan<int32_t>(fi, qo, nq, W.scan_tiles32, W.num_qgroups, st));
-            finish_cells_kernel<<<1, 1, 0, st>>>(W.qgroup_start, W.num_qgroups, nq);
-            note_launches(1);
+            TCR_CUDA(sort_coop<K>(sw, nq, S.num_cells + 1,
+                                  QueryTail<K>{W.qgroup_start, W.num_qgroups, W.pack, W.qsorted, W.qsidx, W.table,
+                                               S.grid, W.qgroup_coords, W.qgroup_cloud, nq},
+                                  st));
             gstart = W.qgroup_start;
             ngroups = W.num_qgroups;
         }
@@ -3133,7 +3059,7 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
     CountIn ci{W.counts, nq};
     OffsetOut oo{nq, offsets, indptr_out, row_entries_out};
     TCR_CUDA(device_exclusive_scan<int64_t>(ci, oo, nq + 1, W.scan_tiles64, W.total, st));
-    info_kernel<<<1, 1, 0, st>>>(S.bad_grids, W.total, W.num_stray, W.exact_clouds, W.cursor, W.num_flagged,
+    info_kernel<<<1, 1, 0, st>>>(S.bad_grids, S.num_cells, W.total, W.num_stray, W.exact_clouds, W.cursor, W.num_flagged,
                                  W.num_exact, b.lin_hint && b.nr > 0 ? W.inc_count : nullptr, b.nr, W.info);
     note_launches(1);
     if (info_out) TCR_CUDA(cudaMemcpyAsync(info_out, W.info, 8 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
