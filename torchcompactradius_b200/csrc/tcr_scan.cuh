@@ -2,7 +2,9 @@
 //
 // A per-tile reduction, then a per-tile scan that adds the tile's prefix.  Up to kScanDirectTiles
 // tiles, each tile sums the totals of the tiles before it itself (at most 16 KB of reads, from L2);
-// above that a single-CTA scan of the tile totals runs in between.  No block waits for another.
+// above that a single-CTA scan of the tile totals runs in between.  Up to kScanSelfTiles tiles there is no
+// reduction either: each tile sums the elements before it (at most 14k, 56 a thread), which is less
+// than the launch it saves.  No block waits for another.
 // Input and output are functors so that producers (flags, counts) and consumers (cell tables,
 // offsets) fuse into the scan instead of round-tripping through HBM.
 #pragma once
@@ -17,6 +19,8 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 constexpr int64_t kScanDirectTiles = 2048;  // 4M elements
+constexpr int64_t kScanSelfTiles = 8;       // 16k elements
+enum ScanPrefix { kScanPrefixes, kScanTotals, kScanElements };  // what a tile finds its prefix from
 
 template <typename T>
 __device__ __forceinline__ T warp_inclusive_scan(T v) {
@@ -90,9 +94,10 @@ __global__ void __launch_bounds__(1024) scan_tiles_kernel(T* tile_sums, int64_t 
 // scan works in.  A padded index keeps the blocked reads free of bank conflicts.
 __device__ __forceinline__ int scan_pad(int i) { return i + (i >> 5); }
 
-// DIRECT: tile_sums holds the tiles' own totals; the tile's prefix is their sum over the tiles
-// before it, and the last tile stores the grand total.  Otherwise tile_sums holds the prefixes.
-template <typename T, bool DIRECT, typename In, typename Out>
+// kScanTotals: tile_sums holds the tiles' own totals; the tile's prefix is their sum over the tiles
+// before it, and the last tile stores the grand total.  kScanElements: the same from the elements
+// themselves.  kScanPrefixes: tile_sums holds the prefixes.
+template <typename T, ScanPrefix FROM, typename In, typename Out>
 __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(In in, Out out, int64_t n, const T* tile_sums,
                                                                   T* grand_total) {
     __shared__ T sm[kScanThreads / 32 + 1];
@@ -106,9 +111,12 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(In in, Out out
         sval[scan_pad(j)] = i < n ? in(i) : T(0);
     }
     T prefix;
-    if (DIRECT) {
+    if (FROM != kScanPrefixes) {
         T acc = 0;
-        for (int64_t t = threadIdx.x; t < (int64_t)blockIdx.x; t += kScanThreads) acc += tile_sums[t];
+        if (FROM == kScanTotals)
+            for (int64_t t = threadIdx.x; t < (int64_t)blockIdx.x; t += kScanThreads) acc += tile_sums[t];
+        else
+            for (int64_t i = threadIdx.x; i < base; i += kScanThreads) acc += in(i);
         block_exclusive_scan<T, kScanThreads>(acc, sm, prefix);  // (its barriers also publish sval)
     } else {
         prefix = tile_sums[blockIdx.x];
@@ -123,7 +131,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(In in, Out out
     }
     T total;
     T ex = block_exclusive_scan<T, kScanThreads>(s, sm, total) + prefix;
-    if (DIRECT && grand_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *grand_total = prefix + total;
+    if (FROM != kScanPrefixes && grand_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *grand_total = prefix + total;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         sex[scan_pad(threadIdx.x * kScanItems + k)] = ex;
@@ -148,14 +156,19 @@ cudaError_t device_exclusive_scan(In in, Out out, int64_t n, T* tile_sums, T* gr
         if (grand_total) return cudaMemsetAsync(grand_total, 0, sizeof(T), st);
         return cudaSuccess;
     }
+    if (nt <= kScanSelfTiles) {
+        scan_apply_kernel<T, kScanElements><<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, n, tile_sums, grand_total);
+        note_launches(1);
+        return cudaGetLastError();
+    }
     scan_reduce_kernel<T><<<(unsigned)nt, kScanThreads, 0, st>>>(in, n, tile_sums);
     if (nt <= kScanDirectTiles) {
-        scan_apply_kernel<T, true><<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, n, tile_sums, grand_total);
+        scan_apply_kernel<T, kScanTotals><<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, n, tile_sums, grand_total);
         note_launches(2);
         return cudaGetLastError();
     }
     scan_tiles_kernel<T><<<1, 1024, 0, st>>>(tile_sums, nt, grand_total);
-    scan_apply_kernel<T, false><<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, n, tile_sums, nullptr);
+    scan_apply_kernel<T, kScanPrefixes><<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, n, tile_sums, nullptr);
     note_launches(3);
     return cudaGetLastError();
 }

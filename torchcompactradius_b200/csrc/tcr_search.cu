@@ -234,26 +234,42 @@ static SortWorkspaceT<K> sort_workspace(const Scratch& W) {
 // the cloud table
 
 // Host -> device copy of the table as kernel parameters (no pageable copy, so it also records
-// into a CUDA graph): chunks of kUploadChunk clouds per launch.
+// into a CUDA graph): up to kUploadChunk clouds travel with the phase's init kernel; of more, all but the last
+// with launches of up to kWideChunk clouds (kernel parameters hold 32 KB; 24 clouds a launch cost a batch of 256
+// 22 launches, 162 us).
 constexpr int kUploadChunk = 24;
+constexpr int kWideChunk = 220;
+template <int N>
 struct CloudChunk {
     int32_t first, count, n_clouds, query_total, ref_total, pad;
-    CloudParams p[kUploadChunk];
+    CloudParams p[N];
 };
-static_assert(sizeof(CloudChunk) <= 4000, "kernel parameter block too large");
+static_assert(sizeof(CloudChunk<kUploadChunk>) <= 4000 && sizeof(CloudChunk<kWideChunk>) <= 32000,
+              "kernel parameter block too large");
 
-__global__ void upload_clouds_kernel(CloudChunk ch, CloudParams* table, int32_t* query_prefix, int32_t* ref_prefix) {
-    const int i = threadIdx.x;
-    if (i < ch.count) {
+template <int N>
+__device__ __forceinline__ void upload_chunk(const CloudChunk<N>& ch, CloudParams* table, int32_t* query_prefix,
+                                             int32_t* ref_prefix) {
+    for (int i = threadIdx.x; i < ch.count; i += blockDim.x) {
         const int c = ch.first + i;
         table[c] = ch.p[i];
         query_prefix[c] = ch.p[i].query_base;
         ref_prefix[c] = ch.p[i].ref_base;
     }
-    if (i == 0 && ch.first + ch.count == ch.n_clouds) {
+    if (threadIdx.x == 0 && ch.first + ch.count == ch.n_clouds) {
         query_prefix[ch.n_clouds] = ch.query_total;
         ref_prefix[ch.n_clouds] = ch.ref_total;
     }
+}
+// Lanes reading different kernel parameters are served one by one, so the chunk is spread over blocks.
+constexpr int kUploadPerBlock = 8;
+__global__ void upload_clouds_kernel(const __grid_constant__ CloudChunk<kWideChunk> ch, CloudParams* table,
+                                     int32_t* query_prefix, int32_t* ref_prefix) {
+    const int i = blockIdx.x * kUploadPerBlock + threadIdx.x;
+    if (threadIdx.x >= kUploadPerBlock || i >= ch.count) return;
+    table[ch.first + i] = ch.p[i];
+    query_prefix[ch.first + i] = ch.p[i].query_base;
+    ref_prefix[ch.first + i] = ch.p[i].ref_base;
 }
 
 // Cloud of global point index i: the last c with prefix[c] <= i (empty clouds are skipped).
@@ -345,9 +361,11 @@ __global__ void support_stats_kernel(const CloudParams* __restrict__ table, cons
     }
 }
 
-// Start of a build: per-cloud statistics and flags, counters, the sort state.
+// Start of a build: the (last clouds of the) table, per-cloud statistics and flags, counters, the sort
+// state, an empty map.
 template <typename K>
-__global__ void grid_init_kernel(GridParams* g, int C, Structure S, Scratch W) {
+__global__ void grid_init_kernel(const __grid_constant__ CloudChunk<kUploadChunk> ch, GridParams* g, int C, Structure S,
+                                 Scratch W) {
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
         g[c].ref_stats.max_key = 0;
         g[c].ref_stats.bad = 0;
@@ -356,7 +374,13 @@ __global__ void grid_init_kernel(GridParams* g, int C, Structure S, Scratch W) {
         g[c].error = 0;
         g[c].out_of_grid = 0;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ulonglong2* map = reinterpret_cast<ulonglong2*>(S.map);  // capacities are powers of two >= 64
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < S.map_total / 2;
+         i += (int64_t)gridDim.x * blockDim.x)
+        map[i] = make_ulonglong2(~0ull, ~0ull);
+    if (blockIdx.x != 0) return;
+    upload_chunk(ch, W.table, W.query_prefix, W.ref_prefix);
+    if (threadIdx.x == 0) {
         *S.bad_grids = 0;
         S.num_cells[0] = S.num_cells[1] = 0;
         sort_state_reset(reinterpret_cast<SortStateT<K>*>(W.sort_state));
@@ -450,35 +474,40 @@ __global__ void grid_params_kernel(const CloudParams* __restrict__ table, GridPa
     }
 }
 
-// Per cloud: the query-side parameters of the lean test.
-// same_sup: the queries are the reference points with the same support array, whose statistics the
-// build reduced already.
+// One cloud's query-side parameters of the lean test.  same_sup: the queries' supports are the
+// references' array, whose statistics the build reduced already.
+__device__ __forceinline__ void query_params(const CloudParams& cp, const GridParams& g, QueryParams& q,
+                                             int32_t* exact_clouds, int same_sup) {
+    if (same_sup) q.stats = g.ref_stats;
+    const bool has_q = cp.query_sup != nullptr;
+    const float qmax = has_q ? key_float(q.stats.max_key) : 0.0f;
+    q.qmax = (cp.mode == kScatter) ? 0.0f : qmax;
+    const bool qbad = (cp.mode != kScatter) && has_q && q.stats.bad;
+    const bool rbad = (cp.mode != kGather) && g.ref_stats.bad;
+    q.exact_all = (qbad || rbad || !(fabsf(q.qmax) <= 1e18f)) ? 1 : 0;
+    if (q.exact_all && cp.n_query > 0) atomicAdd(exact_clouds, 1);
+}
 __global__ void query_params_kernel(const CloudParams* __restrict__ table, const GridParams* __restrict__ grid, int C,
-                                    QueryParams* qp, int32_t* exact_clouds, int same_sup) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
-        const CloudParams& cp = table[c];
-        QueryParams& q = qp[c];
-        if (same_sup) q.stats = grid[c].ref_stats;
-        const bool has_q = cp.query_sup != nullptr;
-        const float qmax = has_q ? key_float(q.stats.max_key) : 0.0f;
-        q.qmax = (cp.mode == kScatter) ? 0.0f : qmax;
-        const bool qbad = (cp.mode != kScatter) && has_q && q.stats.bad;
-        const bool rbad = (cp.mode != kGather) && grid[c].ref_stats.bad;
-        q.exact_all = (qbad || rbad || !(fabsf(q.qmax) <= 1e18f)) ? 1 : 0;
-        if (q.exact_all && cp.n_query > 0) atomicAdd(exact_clouds, 1);
-    }
+                                    QueryParams* qp, int32_t* exact_clouds) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x)
+        query_params(table[c], grid[c], qp[c], exact_clouds, 0);
 }
 
-// Zeroes the per-search counters, the per-cloud query statistics and the per-query counts.
-__global__ void count_init_kernel(Scratch W, int C, int unit_cap, int64_t nq, int64_t stage_cap) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
+// Start of a count: the (last clouds of the) table; zeroes the per-search counters, the per-cloud query
+// statistics and the per-query counts; with ready also writes the clouds' query parameters (1: the
+// queries' supports are the references', 2: there are none to reduce).
+__global__ void count_init_kernel(const __grid_constant__ CloudChunk<kUploadChunk> ch, const GridParams* grid, Scratch W,
+                                  int C, int unit_cap, int64_t nq, int64_t stage_cap, int ready) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x)
+        W.counts[i] = 0;
+    if (blockIdx.x != 0) return;
+    upload_chunk(ch, W.table, W.query_prefix, W.ref_prefix);
+    for (int c = threadIdx.x; c < C; c += blockDim.x) {
         W.qparams[c].stats.max_key = 0;
         W.qparams[c].stats.bad = 0;
         W.qparams[c].coord_key = 0;
     }
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x)
-        W.counts[i] = 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (threadIdx.x == 0) {
         for (int k = 0; k < kWorkCounters; ++k) W.work[k] = 0;
         *W.num_stray = 0;
         *W.num_units = 0;
@@ -489,6 +518,10 @@ __global__ void count_init_kernel(Scratch W, int C, int unit_cap, int64_t nq, in
         W.cursor[0] = 0ull;
         W.cursor[1] = (unsigned long long)stage_cap;
     }
+    if (!ready) return;
+    __syncthreads();  // (the block's own writes of the table and the counters)
+    for (int c = threadIdx.x; c < C; c += blockDim.x)
+        query_params(W.table[c], grid[c], W.qparams[c], W.exact_clouds, ready == 1);
 }
 
 __device__ __forceinline__ float4 load_point(const float* x, const float* h, int64_t i, int dim) {
@@ -2447,6 +2480,8 @@ __device__ __forceinline__ void decide_band_pair(const WalkArgs& a, const int4& 
 template <bool EMIT>
 __global__ void stray_kernel(WalkArgs a) {
     const int32_t ns = *a.num_stray;
+    // the last launch of a count or an emit leaves the work counters ready for the next emit
+    if (blockIdx.x == 0 && threadIdx.x < kWorkCounters) a.work[threadIdx.x] = 0;
     if (!EMIT) {
         const int64_t nband = min((int64_t)*a.num_exact, a.nq_total);
         for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nband; i += (int64_t)gridDim.x * blockDim.x)
@@ -2549,26 +2584,35 @@ struct OffsetOut {
     int64_t* offsets;
     int32_t* indptr;
     int64_t* entries;
+    // the search's info block, written with the total (element n)
+    const int32_t* bad_grids;
+    const int32_t* num_cells;
+    const int32_t* num_stray;
+    const int32_t* exact_clouds;
+    const unsigned long long* cursor;
+    const int32_t* num_flagged;
+    const int32_t* num_exact;
+    const int32_t* inc_count;
+    int64_t n_ref;
+    int64_t* info;
     __device__ void operator()(int64_t i, int64_t ex, int64_t v) const {
         offsets[i] = ex;
         if (indptr) indptr[i] = (int32_t)ex;
-        if (entries && i < n) entries[i] = v;
+        if (i < n) {
+            if (entries) entries[i] = v;
+            return;
+        }
+        info[0] = ex;
+        info[1] = num_cells[1] ? -1 : *bad_grids;  // -1: a wait inside the sort gave up, nothing here is valid
+        info[2] = *num_stray;
+        info[3] = *exact_clouds;
+        info[4] = (int64_t)*cursor;
+        info[5] = *num_flagged;
+        info[6] = *num_exact;
+        // incremental build: points sorted by the small sort (-1: the full sort ran); -2: no hint
+        info[7] = inc_count ? ((inc_count[1] != 0 || 2 * (int64_t)inc_count[0] < n_ref) ? -1 : n_ref - inc_count[0]) : -2;
     }
 };
-
-__global__ void info_kernel(const int32_t* bad_grids, const int32_t* num_cells, const int64_t* total, const int32_t* num_stray,
-                            const int32_t* exact_clouds, const unsigned long long* cursor, const int32_t* num_flagged,
-                            const int32_t* num_exact, const int32_t* inc_count, int64_t n_ref, int64_t* info) {
-    info[0] = *total;
-    info[1] = num_cells[1] ? -1 : *bad_grids;  // -1: a wait inside the sort gave up, nothing here is valid
-    info[2] = *num_stray;
-    info[3] = *exact_clouds;
-    info[4] = (int64_t)*cursor;
-    info[5] = *num_flagged;
-    info[6] = *num_exact;
-    // incremental build: points sorted by the small sort (-1: the full sort ran); -2: no hint
-    info[7] = inc_count ? ((inc_count[1] != 0 || 2 * (int64_t)inc_count[0] < n_ref) ? -1 : n_ref - inc_count[0]) : -2;
-}
 
 // ------------------------------------------------------------------------------------------
 // host orchestration
@@ -2583,6 +2627,7 @@ struct HostBatch {
     bool any_query_sup = false, any_ref_sup = false;
     bool same_sorted = false;     // self search, no periodic dims, queries are the references (same arrays)
     bool same_positions = false;  // self search, no periodic dims, same position arrays
+    bool same_supports = false;   // self search, the queries' supports are the references' arrays
     int walk_class = 0;           // dim * 2 + (any periodic dim) when every cloud shares it, else 0
     uint32_t class_mask = 0;      // bit cls: some cloud with queries has class cls
     bool wide = false;            // 64-bit (cloud, cell) sort keys
@@ -2625,7 +2670,7 @@ static int check_cloud(const char* who, int dim, int mode, int64_t L, int64_t nq
 
 static int finish_batch(HostBatch& b, int64_t map_min) {
     int64_t qb = 0, rb = 0, mb = 0;
-    bool same_pos = b.self != 0, same_sorted = b.self != 0;
+    bool same_pos = b.self != 0, same_sorted = b.self != 0, same_sup = b.self != 0;
     int cls = -1;
     bool mixed = false;
     b.any_query_sup = b.any_ref_sup = false;
@@ -2642,6 +2687,7 @@ static int finish_batch(HostBatch& b, int64_t map_min) {
         mb += cp.map_cap;
         same_pos = same_pos && cp.periodic_mask == 0 && cp.query_pos == cp.ref_pos;
         same_sorted = same_sorted && cp.periodic_mask == 0 && cp.query_pos == cp.ref_pos && cp.query_sup == cp.ref_sup;
+        same_sup = same_sup && cp.query_sup == cp.ref_sup;
         b.any_query_sup = b.any_query_sup || cp.query_sup != nullptr;
         b.any_ref_sup = b.any_ref_sup || cp.ref_sup != nullptr;
         const int c = cp.dim * 2 + (cp.periodic_mask != 0 ? 1 : 0);
@@ -2654,6 +2700,7 @@ static int finish_batch(HostBatch& b, int64_t map_min) {
     b.map_total = mb;
     b.same_positions = same_pos;
     b.same_sorted = same_sorted;
+    b.same_supports = same_sup;
     b.walk_class = mixed ? 0 : cls;
     b.wide = b.C > 1;
     return TCR_OK;
@@ -2787,19 +2834,28 @@ static void prof_mark(int kernel, int end, cudaStream_t st) {
     if (cudaEventRecordWithFlags(g_prof_ev[kernel][end], st, flags) == cudaSuccess && end) g_prof_recorded[kernel] = 1;
 }
 
-static int upload_table(const HostBatch& b, const Scratch& W, cudaStream_t st) {
-    for (int first = 0; first < b.C; first += kUploadChunk) {
-        CloudChunk ch;
-        memset(&ch, 0, sizeof(ch));
-        ch.first = first;
-        ch.count = std::min(kUploadChunk, b.C - first);
-        ch.n_clouds = b.C;
-        ch.query_total = (int32_t)b.nq;
-        ch.ref_total = (int32_t)b.nr;
-        memcpy(ch.p, &b.clouds[first], sizeof(CloudParams) * ch.count);
-        upload_clouds_kernel<<<1, 32, 0, st>>>(ch, W.table, W.query_prefix, W.ref_prefix);
+template <int N>
+static CloudChunk<N> cloud_chunk(const HostBatch& b, int first, int count) {
+    CloudChunk<N> ch;
+    ch.first = first;
+    ch.count = count;
+    ch.n_clouds = b.C;
+    ch.query_total = (int32_t)b.nq;
+    ch.ref_total = (int32_t)b.nr;
+    ch.pad = 0;
+    memcpy(ch.p, &b.clouds[first], sizeof(CloudParams) * count);
+    return ch;
+}
+// Uploads all but the table's last chunk, which is returned for the phase's init kernel.
+static int upload_table(const HostBatch& b, const Scratch& W, cudaStream_t st, CloudChunk<kUploadChunk>& last) {
+    const int tail = b.C <= kUploadChunk ? b.C : 1, before = b.C - tail;
+    for (int first = 0; first < before; first += kWideChunk) {
+        const int count = std::min(kWideChunk, before - first);
+        upload_clouds_kernel<<<(count + kUploadPerBlock - 1) / kUploadPerBlock, 32, 0, st>>>(
+            cloud_chunk<kWideChunk>(b, first, count), W.table, W.query_prefix, W.ref_prefix);
         note_launches(1);
     }
+    last = cloud_chunk<kUploadChunk>(b, before, tail);
     TCR_CUDA(cudaGetLastError());
     return TCR_OK;
 }
@@ -2932,9 +2988,11 @@ static int build_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
     const SortWorkspaceT<K> sw = sort_workspace<K>(W);
     const int C = b.C;
     const int64_t nr = b.nr, nq = b.nq;
-    int rc = upload_table(b, W, st);
+    CloudChunk<kUploadChunk> chunk;
+    int rc = upload_table(b, W, st, chunk);
     if (rc) return rc;
-    grid_init_kernel<K><<<grid_for(C, 128), 128, 0, st>>>(S.grid, C, S, W);
+    grid_init_kernel<K><<<grid_for(std::max<int64_t>(C, S.map_total / 8), 256, num_sms() * 8), 256, 0, st>>>(
+        chunk, S.grid, C, S, W);
     note_launches(1);
     // computeGridSupport: which supports set hMax depends on the mode
     if (b.any_ref_sup && nr > 0) {
@@ -2943,15 +3001,14 @@ static int build_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
             (int64_t)sizeof(GridParams));
         note_launches(1);
     }
-    if (b.any_query_sup && nq > 0 && !b.same_sorted) {
+    if (b.any_query_sup && nq > 0 && !b.same_supports) {
         support_stats_kernel<<<grid_for(nq, 256, num_sms() * 4), 256, 0, st>>>(
             W.table, W.query_prefix, C, nq, 1,
             reinterpret_cast<char*>(S.grid) + offsetof(GridParams, build_query_stats), (int64_t)sizeof(GridParams));
         note_launches(1);
     }
-    grid_params_kernel<<<grid_for(C, 128), 128, 0, st>>>(W.table, S.grid, C, S.bad_grids, b.same_sorted ? 1 : 0);
+    grid_params_kernel<<<grid_for(C, 128), 128, 0, st>>>(W.table, S.grid, C, S.bad_grids, b.same_supports ? 1 : 0);
     note_launches(1);
-    TCR_CUDA(cudaMemsetAsync(S.map, 0xff, sizeof(unsigned long long) * S.map_total, st));
     if (nr > 0) {
         const bool inc = b.lin_hint != nullptr;
         // few blocks: each ends with one atomic on the key range, so thousands of them would queue
@@ -2998,20 +3055,21 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
                       cudaStream_t st, const F64Args* f64) {
     const int C = b.C;
     const int64_t nq = b.nq;
-    int rc = upload_table(b, W, st);
+    CloudChunk<kUploadChunk> chunk;
+    int rc = upload_table(b, W, st, chunk);
     if (rc) return rc;
     const int unit_cap = b.unit_cap;
-    count_init_kernel<<<grid_for(std::max<int64_t>(C, nq), 256), 256, 0, st>>>(W, C, unit_cap, nq, stage_cap);
+    const bool query_stats = b.any_query_sup && nq > 0 && !b.same_supports;
+    count_init_kernel<<<grid_for(std::max<int64_t>(C, nq), 256), 256, 0, st>>>(chunk, S.grid, W, C, unit_cap, nq, stage_cap,
+                                                                               query_stats ? 0 : (b.same_supports ? 1 : 2));
     note_launches(1);
-    if (b.any_query_sup && nq > 0 && !b.same_sorted) {
+    if (query_stats) {
         support_stats_kernel<<<grid_for(nq, 256, num_sms() * 4), 256, 0, st>>>(
             W.table, W.query_prefix, C, nq, 1, reinterpret_cast<char*>(W.qparams) + offsetof(QueryParams, stats),
             (int64_t)sizeof(QueryParams));
-        note_launches(1);
+        query_params_kernel<<<grid_for(C, 128), 128, 0, st>>>(W.table, S.grid, C, W.qparams, W.exact_clouds);
+        note_launches(2);
     }
-    query_params_kernel<<<grid_for(C, 128), 128, 0, st>>>(W.table, S.grid, C, W.qparams, W.exact_clouds,
-                                                          b.same_sorted ? 1 : 0);
-    note_launches(1);
     if (f64 && (b.nr > 0 || nq > 0)) {
         f64_prep_kernel<<<grid_for(std::max<int64_t>(b.nr, nq * b.clouds[0].dim), 256), 256, 0, st>>>(
             S.rsidx, *f64, b.clouds[0].dim, W.qparams);
@@ -3057,11 +3115,9 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
         note_launches(1);
     }
     CountIn ci{W.counts, nq};
-    OffsetOut oo{nq, offsets, indptr_out, row_entries_out};
+    OffsetOut oo{nq, offsets, indptr_out, row_entries_out, S.bad_grids, S.num_cells, W.num_stray, W.exact_clouds, W.cursor,
+                 W.num_flagged, W.num_exact, b.lin_hint && b.nr > 0 ? W.inc_count : nullptr, b.nr, W.info};
     TCR_CUDA(device_exclusive_scan<int64_t>(ci, oo, nq + 1, W.scan_tiles64, W.total, st));
-    info_kernel<<<1, 1, 0, st>>>(S.bad_grids, S.num_cells, W.total, W.num_stray, W.exact_clouds, W.cursor, W.num_flagged,
-                                 W.num_exact, b.lin_hint && b.nr > 0 ? W.inc_count : nullptr, b.nr, W.info);
-    note_launches(1);
     if (info_out) TCR_CUDA(cudaMemcpyAsync(info_out, W.info, 8 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     return TCR_OK;
 }
@@ -3078,7 +3134,6 @@ static int emit_impl(const HostBatch& b, const Structure& S, const Scratch& W, c
     a.row_out = row_out;
     a.col_out = col_out;
     a.out_cap = out_capacity;
-    TCR_CUDA(cudaMemsetAsync(W.work, 0, sizeof(int32_t) * kWorkCounters, st));
     if (stage) {
         const int nsm = num_sms();
         // resident blocks (four an SM), no more than about two units per query group's worth of full ones

@@ -344,6 +344,8 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     const int64_t per = ((n + G - 1) / G + 31) & ~int64_t(31);
     const int64_t lo = min(n, per * b), hi = min(n, lo + per);
     const unsigned lt = (1u << lane) - 1u;
+    const bool single = per <= kCoopTile;
+    const int rounds = (int)((min(per, (int64_t)kCoopTile) + kCoopThreads - 1) / kCoopThreads);
     unsigned phase = 0;
     int sel = st->sel[0];
     bool placed = false;
@@ -354,16 +356,74 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
         const int32_t* vin = sel ? vals1 : vals0;
         K* kout = sel ? keys0 : keys1;
         int32_t* vout = sel ? vals0 : vals1;
-        // this block's histogram (per-warp copies spread the atomics)
-        for (int i = tid; i < kCoopWarps * kBins; i += kCoopThreads) (&sm.warp_hist[0][0])[i] = 0;
-        __syncthreads();
-        for (int64_t i = lo + tid; i < hi; i += kCoopThreads) atomicAdd(&sm.warp_hist[warp][(int)((kin[i] >> shift) & 0xff)], 1);
-        __syncthreads();
-        if (tid < kBins) {
+        K key[kCoopRounds];
+        int32_t val[kCoopRounds], rank[kCoopRounds];
+        int32_t dtot = 0;  // (thread < 256) the tile's keys of digit tid
+        // loads a tile of the range and ranks its keys: warp w owns keys [32 R w, 32 R (w + 1)); warp_hist
+        // ends as the keys of a digit in the warps before
+        auto rank_tile = [&](int64_t t0, int len, int R) {
+            for (int i = tid; i < kCoopWarps * kBins; i += kCoopThreads) (&sm.warp_hist[0][0])[i] = 0;
+#pragma unroll
+            for (int r = 0; r < kCoopRounds; ++r) {
+                const int i = warp * 32 * R + r * 32 + lane;
+                const bool valid = r < R && i < len;
+                key[r] = valid ? kin[t0 + i] : (K)0;
+                val[r] = valid ? vin[t0 + i] : 0;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < kCoopRounds; ++r) {
+                if (r < R) {
+                    const bool valid = warp * 32 * R + r * 32 + lane < len;
+                    const uint32_t dig = valid ? (uint32_t)((key[r] >> shift) & 0xff) : 0x100u;
+                    const unsigned peers = __match_any_sync(0xffffffffu, dig);
+                    const int ahead = __popc(peers & lt);
+                    const int run = valid ? sm.warp_hist[warp][dig] : 0;
+                    __syncwarp();
+                    if (valid && ahead == 0) sm.warp_hist[warp][dig] = run + __popc(peers);
+                    __syncwarp();
+                    rank[r] = run + ahead;
+                }
+            }
+            __syncthreads();
+            // exclusive over the warps, four groups of threads with eight warps each
+            constexpr int kPer = kCoopWarps / (kCoopThreads / kBins);
+            const int d = tid & (kBins - 1), grp = tid >> 8;
             int32_t c = 0;
+#pragma unroll
+            for (int w = 0; w < kPer; ++w) c += sm.warp_hist[grp * kPer + w][d];
+            sm.part[grp][d] = c;
+            __syncthreads();
+            int32_t acc = 0;
+            for (int g = 0; g < grp; ++g) acc += sm.part[g][d];
+#pragma unroll
+            for (int w = 0; w < kPer; ++w) {
+                const int32_t x = sm.warp_hist[grp * kPer + w][d];
+                sm.warp_hist[grp * kPer + w][d] = acc;
+                acc += x;
+            }
+            dtot = 0;
+            if (tid < kBins)
+                for (int g = 0; g < kCoopThreads / kBins; ++g) dtot += sm.part[g][tid];
+            __syncthreads();
+        };
+        // a range of one tile (up to 1.2M keys on 148 blocks) is ranked at once and stays in registers;
+        // a longer one is counted first and ranked tile by tile
+        if (single) {
+            rank_tile(lo, (int)(hi - lo), rounds);
+            if (tid < kBins) hist[(int64_t)b * kBins + tid] = dtot;
+        } else {
+            for (int i = tid; i < kCoopWarps * kBins; i += kCoopThreads) (&sm.warp_hist[0][0])[i] = 0;
+            __syncthreads();
+            for (int64_t i = lo + tid; i < hi; i += kCoopThreads)
+                atomicAdd(&sm.warp_hist[warp][(int)((kin[i] >> shift) & 0xff)], 1);
+            __syncthreads();
+            if (tid < kBins) {
+                int32_t c = 0;
 #pragma unroll 8
-            for (int w = 0; w < kCoopWarps; ++w) c += sm.warp_hist[w][tid];
-            hist[(int64_t)b * kBins + tid] = c;
+                for (int w = 0; w < kCoopWarps; ++w) c += sm.warp_hist[w][tid];
+                hist[(int64_t)b * kBins + tid] = c;
+            }
         }
         if (!coop_barrier(&st->bar, (unsigned)G * ++phase, failed, &sm.flag)) return;
         // first output slot of every digit of this block: the smaller digits' keys, then this digit's of
@@ -397,42 +457,8 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
         const bool last = Tail::kPlace && !pass_needed(st, shift + 8);
         for (int64_t t0 = lo; t0 < hi; t0 += kCoopTile) {
             const int len = (int)min((int64_t)kCoopTile, hi - t0);
-            const int R = (len + kCoopThreads - 1) / kCoopThreads;  // rounds: warp w owns keys [32 R w, 32 R (w + 1))
-            for (int i = tid; i < kCoopWarps * kBins; i += kCoopThreads) (&sm.warp_hist[0][0])[i] = 0;
-            __syncthreads();
-            K key[kCoopRounds];
-            int32_t val[kCoopRounds], rank[kCoopRounds];
-#pragma unroll
-            for (int r = 0; r < kCoopRounds; ++r) {
-                const int i = warp * 32 * R + r * 32 + lane;
-                const bool valid = r < R && i < len;
-                key[r] = valid ? kin[t0 + i] : (K)0;
-                val[r] = valid ? vin[t0 + i] : 0;
-            }
-#pragma unroll
-            for (int r = 0; r < kCoopRounds; ++r) {
-                if (r < R) {
-                    const bool valid = warp * 32 * R + r * 32 + lane < len;
-                    const uint32_t dig = valid ? (uint32_t)((key[r] >> shift) & 0xff) : 0x100u;
-                    const unsigned peers = __match_any_sync(0xffffffffu, dig);
-                    const int ahead = __popc(peers & lt);
-                    const int run = valid ? sm.warp_hist[warp][dig] : 0;
-                    __syncwarp();
-                    if (valid && ahead == 0) sm.warp_hist[warp][dig] = run + __popc(peers);
-                    __syncwarp();
-                    rank[r] = run + ahead;
-                }
-            }
-            __syncthreads();
-            int32_t dtot = 0;
-            if (tid < kBins) {
-#pragma unroll 8
-                for (int w = 0; w < kCoopWarps; ++w) {
-                    const int c = sm.warp_hist[w][tid];
-                    sm.warp_hist[w][tid] = dtot;
-                    dtot += c;
-                }
-            }
+            const int R = single ? rounds : (len + kCoopThreads - 1) / kCoopThreads;
+            if (!single) rank_tile(t0, len, R);
             int32_t sum;
             const int32_t ex = block_exclusive_scan<int32_t, kCoopThreads>(dtot, sm.scan, sum);
             if (tid < kBins) sm.digit_start[tid] = ex;
