@@ -373,10 +373,39 @@ __device__ __forceinline__ void load_keys(const KT* keys, int64_t base, int64_t 
     }
 }
 
+// A chunk of 64-bit keys that all lie in [0, nslots) and never descend from the key before them: 32-bit
+// differences, one store where a run starts (the usual step of one slot), mark_range where slots are empty.
+// Returns the chunk's descents; nothing is marked when there are any (the fold will not run).
+__device__ __forceinline__ uint32_t mark_chunk32(const int64_t (&v)[kMarkKeys], uint32_t before, int64_t base, int64_t* off,
+                                                 int64_t* gaps, unsigned long long* ngaps, int64_t gap_cap,
+                                                 unsigned long long* dsc) {
+    uint32_t d[kMarkKeys], desc = 0, wide = 0;
+#pragma unroll
+    for (int k = 0; k < kMarkKeys; ++k) {
+        d[k] = (uint32_t)v[k] - (k == 0 ? before : (uint32_t)v[k - 1]);
+        desc += d[k] >> 31;
+        wide |= d[k];
+    }
+    if (desc != 0) return desc;
+    if (wide <= 1) {
+#pragma unroll
+        for (int k = 0; k < kMarkKeys; ++k)
+            if (d[k]) off[(uint32_t)v[k]] = base + k;
+    } else {
+#pragma unroll
+        for (int k = 0; k < kMarkKeys; ++k) {
+            const uint32_t cur = (uint32_t)v[k], prev = k == 0 ? before : (uint32_t)v[k - 1];
+            if (cur != prev) mark_range((int64_t)(prev + 1u), (int64_t)cur, base + k, off, gaps, ngaps, gap_cap, dsc);
+        }
+    }
+    return 0;
+}
+
 // RAW: the keys are the caller's index in its own order (min, max and descents go to stats).
-// Each thread takes kMarkKeys consecutive positions.  Most such chunks lie inside one run (a run
-// of a neighbour list's rows is ~50 long): a chunk that never descends and ends on the key before
-// it marks nothing, so it costs a few compares; only chunks where the key changes mark run starts.
+// Each thread takes kMarkKeys consecutive positions.  The index is read once, 8 bytes an element, which
+// bounds the kernel; a warp meets a run start in nearly every chunk (a run of a neighbour list's rows is
+// ~50 long), so the path with one must be short too: 52M elements took 148 us with 64-bit compares and
+// range loops throughout, now 78, of 65 us the reads take; 3.2M in no order 79, now 16.
 template <typename KT, bool RAW>
 __global__ void __launch_bounds__(kThreads) mark_runs_kernel(const KT* k0, const KT* k1, const int32_t* sel, int64_t M,
                                                              int64_t nslots, int64_t* off, int64_t* gaps,
@@ -386,15 +415,34 @@ __global__ void __launch_bounds__(kThreads) mark_runs_kernel(const KT* k0, const
     const bool aligned = (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
     unsigned long long* dsc = reinterpret_cast<unsigned long long*>(&stats[2]);
     long long lo = LLONG_MAX, hi = LLONG_MIN;
+    uint32_t lo32 = 0xffffffffu, hi32 = 0;
     unsigned long long desc = 0;
     const int64_t nchunks = (M + kMarkKeys - 1) / kMarkKeys;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const bool narrow = nslots <= 0x7ffffffeLL;
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < nchunks; c += stride) {
         const int64_t base = c * kMarkKeys;
         const int nk = M - base < kMarkKeys ? (int)(M - base) : kMarkKeys;
         KT v[kMarkKeys];
         load_keys(keys, base, M, aligned, v);
         const KT pk = base == 0 ? v[0] : keys[base - 1];
+        if constexpr (RAW) {
+            uint64_t bits = base == 0 ? 0ull : (uint64_t)pk;
+            uint32_t mn = 0xffffffffu, mx = 0;
+#pragma unroll
+            for (int k = 0; k < kMarkKeys; ++k) {
+                bits |= (uint64_t)v[k];
+                mn = min(mn, (uint32_t)v[k]);
+                mx = max(mx, (uint32_t)v[k]);
+            }
+            if (narrow && nk == kMarkKeys && base + nk < M && bits <= 0x7fffffffull && mx < (uint32_t)nslots) {
+                lo32 = min(lo32, mn);
+                hi32 = max(hi32, mx);
+                // (the first key follows slot -1)
+                desc += mark_chunk32(v, base == 0 ? 0xffffffffu : (uint32_t)pk, base, off, gaps, ngaps, gap_cap, dsc);
+                continue;
+            }
+        }
         bool mono = true;
         KT last = v[0];
 #pragma unroll
@@ -405,32 +453,22 @@ __global__ void __launch_bounds__(kThreads) mark_runs_kernel(const KT* k0, const
                     mono = false;
                     if (RAW) ++desc;
                 }
-                last = v[k];
-            }
-        }
-        if (RAW) {
-            if (mono) {
-                const long long a = (long long)v[0], b = (long long)last;
-                lo = a < lo ? a : lo;
-                hi = b > hi ? b : hi;
-            } else {
-#pragma unroll
-                for (int k = 0; k < kMarkKeys; ++k) {
-                    if (k < nk) {
-                        const long long x = (long long)v[k];
-                        lo = x < lo ? x : lo;
-                        hi = x > hi ? x : hi;
-                    }
+                if (RAW) {
+                    const long long x = (long long)v[k];
+                    lo = x < lo ? x : lo;
+                    hi = x > hi ? x : hi;
                 }
+                last = v[k];
             }
         }
         if (!(mono && base > 0 && last == pk)) {  // some run starts in this chunk
             int64_t prev = base == 0 ? -1 : key_slot(pk, nslots);
-#pragma unroll
-            for (int k = 0; k < kMarkKeys; ++k) {
+#pragma unroll 1
+            for (int k = 0; k < nk; ++k) {
+                const KT x = k == 0 ? v[0] : keys[base + k];
                 // a key equal to the one before it starts no run (same slot): one compare
-                if (k < nk && (v[k] != (k == 0 ? pk : v[k - 1]) || (k == 0 && base == 0))) {
-                    const int64_t cur = key_slot(v[k], nslots);
+                if (x != (k == 0 ? pk : keys[base + k - 1]) || (k == 0 && base == 0)) {
+                    const int64_t cur = key_slot(x, nslots);
                     mark_range(prev + 1 < 0 ? 0 : prev + 1, cur, base + k, off, gaps, ngaps, gap_cap, dsc);
                     prev = cur;
                 }
@@ -441,7 +479,13 @@ __global__ void __launch_bounds__(kThreads) mark_runs_kernel(const KT* k0, const
             mark_range(cur + 1 < 0 ? 0 : cur + 1, nslots, M, off, gaps, ngaps, gap_cap, dsc);
         }
     }
-    if (RAW) stats_add(stats, lo, hi, desc);
+    if (RAW) {
+        if (lo32 <= hi32) {
+            lo = (long long)lo32 < lo ? (long long)lo32 : lo;
+            hi = (long long)hi32 > hi ? (long long)hi32 : hi;
+        }
+        stats_add(stats, lo, hi, desc);
+    }
 }
 
 // need_sorted: the runs come from the caller's index in its own order, which holds only when it
@@ -513,51 +557,73 @@ __device__ __forceinline__ void fold_write(const FoldArgs& a, T* out, int64_t t,
     }
 }
 
-// Index over e, non-decreasing, one value per (b, e) (K == 1): a block owns kThreads consecutive
-// rows of one b, whose elements are one contiguous range of src.  The range streams through
-// shared memory in tiles with coalesced loads; each thread folds its own row from the tile in
-// order.
-constexpr int kFoldTileBytes = 16384;
+// Index over e, non-decreasing, one value per (b, e) (K == 1): a warp owns 32 consecutive rows of one b,
+// whose elements are one contiguous range of src.  The range streams through the warp's part of shared memory
+// in tiles, with 16-byte loads where src allows them; each lane folds its own row from the tile in
+// order.  The warps do not wait for each other: with a block's 256 rows sharing 16 KB tiles, a third of
+// the threads had a row in the tile and all waited for the longest one (52M float32 values: 75 us, now 43,
+// of 34 us the reads take).
+constexpr int kFoldWarps = 4;
+constexpr int kFoldTileBytes = 8192;  // per warp; 32 rows of ~50 float32 are 6400
 
 template <typename T, int R>
-__global__ void __launch_bounds__(kThreads) fold_rows_kernel(FoldArgs a) {
+__global__ void __launch_bounds__(kFoldWarps * 32) fold_rows_kernel(FoldArgs a) {
     using Nm = Num<T>;
     constexpr int TILE = kFoldTileBytes / (int)sizeof(T);
-    __shared__ __align__(16) unsigned char tile_raw[kFoldTileBytes];
-    T* tile = reinterpret_cast<T*>(tile_raw);
+    constexpr int V = 16 / (int)sizeof(T);
+    __shared__ __align__(16) unsigned char tile_raw[kFoldWarps][kFoldTileBytes];
+    const int lane = threadIdx.x & 31;
+    T* tile = reinterpret_cast<T*>(tile_raw[threadIdx.x >> 5]);
     if (!stats_allow(a.stats, a.N, true)) return;
     const T* __restrict__ src = static_cast<const T*>(a.src);
     T* __restrict__ out = static_cast<T*>(a.out);
     const int64_t M = a.E;
-    const int64_t rb = (a.N + kThreads - 1) / kThreads;
-    for (int64_t blk = blockIdx.x; blk < a.B * rb; blk += gridDim.x) {
-        const int64_t b = blk / rb, n0 = (blk % rb) * kThreads;
-        const int64_t n = n0 + threadIdx.x;
-        const int64_t nend = n0 + kThreads < a.N ? n0 + kThreads : a.N;
-        int64_t E0 = a.off[n0], E1 = a.off[nend];
-        E0 = E0 < 0 ? 0 : (E0 > M ? M : E0);
-        E1 = E1 < E0 ? E0 : (E1 > M ? M : E1);
-        int64_t lo = E1, hi = E1;
-        if (n < a.N) {
-            lo = a.off[n];
-            hi = a.off[n + 1];
-            lo = lo < E0 ? E0 : (lo > E1 ? E1 : lo);
-            hi = hi < lo ? lo : (hi > E1 ? E1 : hi);
-        }
+    const int64_t rb = (a.N + 31) / 32;
+    for (int64_t blk = (int64_t)blockIdx.x * kFoldWarps + (threadIdx.x >> 5); blk < a.B * rb;
+         blk += (int64_t)gridDim.x * kFoldWarps) {
+        const int64_t b = blk / rb, n0 = (blk % rb) * 32;
+        const int64_t n = n0 + lane;
+        int64_t lo = n < a.N ? a.off[n] : M, hi = n < a.N ? a.off[n + 1] : M;
+        lo = lo < 0 ? 0 : (lo > M ? M : lo);
+        hi = hi < lo ? lo : (hi > M ? M : hi);
+        const int64_t E0 = __shfl_sync(0xffffffffu, lo, 0);
+        const int64_t E1 = __shfl_sync(0xffffffffu, hi, (int)(a.N - n0 < 32 ? a.N - n0 - 1 : 31));
         Fold<T, R> f;
         f.acc = (a.accumulate && n < a.N) ? out[b * a.N + n] : reduce_init<T, R>();
         f.cnt = Nm::zero();
         f.arg = a.E;
         const T* s = src + b * a.E;
-        for (int64_t t0 = E0; t0 < E1; t0 += TILE) {
+        const bool wide = (reinterpret_cast<uintptr_t>(s) & 15) == 0;
+        // (with wide loads a tile starts on a 16-byte boundary, up to V - 1 elements early)
+        for (int64_t t0 = wide ? E0 & ~(int64_t)(V - 1) : E0; t0 < E1; t0 += TILE) {
             const int len = (int)(E1 - t0 < TILE ? E1 - t0 : TILE);
-            __syncthreads();  // the previous tile is consumed
-#pragma unroll 8
-            for (int i = threadIdx.x; i < len; i += kThreads) tile[i] = s[t0 + i];
-            __syncthreads();
-            const int64_t j0 = lo > t0 ? lo : t0;
-            const int64_t j1 = hi < t0 + len ? hi : t0 + len;
-            for (int64_t j = j0; j < j1; ++j) f.take(tile[j - t0], j);
+            __syncwarp();  // the previous tile is consumed
+            int i = 0;
+            if (wide) {  // asynchronous copies: a tile's loads are all in flight at once
+                const int nv = len / V;
+                const unsigned to = (unsigned)__cvta_generic_to_shared(tile);
+#pragma unroll 4
+                for (int j = lane; j < nv; j += 32)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to + 16 * j),
+                                 "l"(reinterpret_cast<const uint4*>(s + t0) + j)
+                                 : "memory");
+                i = nv * V;
+            }
+#pragma unroll 4
+            for (int j = i + lane; j < len; j += 32) tile[j] = s[t0 + j];
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+            __syncwarp();
+            const int j0 = (int)((lo > t0 ? lo : t0) - t0 < len ? (lo > t0 ? lo : t0) - t0 : len);
+            const int j1 = (int)((hi < t0 + len ? hi : t0 + len) - t0);
+            int j = j0;
+            for (; j + 4 <= j1; j += 4) {  // four reads in flight, folded in order
+                const T v0 = tile[j], v1 = tile[j + 1], v2 = tile[j + 2], v3 = tile[j + 3];
+                f.take(v0, t0 + j);
+                f.take(v1, t0 + j + 1);
+                f.take(v2, t0 + j + 2);
+                f.take(v3, t0 + j + 3);
+            }
+            for (; j < j1; ++j) f.take(tile[j], t0 + j);
         }
         if (n < a.N) fold_write<T, R>(a, out, b * a.N + n, f);
     }
@@ -604,13 +670,37 @@ __global__ void __launch_bounds__(kThreads) fold_kernel(FoldArgs a) {
             }
             for (; j < hi; ++j) f.take(s[j * a.K], j);
         } else if (P == 1) {
+            // eight positions, then eight values in flight, folded in order: one at a time, each element waited
+            // for two dependent reads (3.2M elements of 8 features: 67 us, now 51)
             const T* s = src + b * a.E * a.K + k;
-            for (int64_t j = lo; j < hi; ++j) {
+            int64_t j = lo;
+            for (; j + 8 <= hi; j += 8) {
+                int32_t e[8];
+                T v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) e[i] = perm[j + i];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = s[(int64_t)e[i] * a.K];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) f.take(v[i], e[i]);
+            }
+            for (; j < hi; ++j) {
                 const int64_t e = perm[j];
                 f.take(s[e * a.K], e);
             }
         } else {
-            for (int64_t j = lo; j < hi; ++j) {
+            int64_t j = lo;
+            for (; j + 4 <= hi; j += 4) {
+                int32_t e[4];
+                T v[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) e[i] = perm[j + i];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = src[e[i]];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) f.take(v[i], (e[i] / a.K) % a.E);
+            }
+            for (; j < hi; ++j) {
                 const int64_t pos = perm[j];
                 f.take(src[pos], (pos / a.K) % a.E);
             }
@@ -622,7 +712,7 @@ __global__ void __launch_bounds__(kThreads) fold_kernel(FoldArgs a) {
 template <typename T, int R, int P>
 void launch_one(const FoldArgs& fa, unsigned grid, cudaStream_t st) {
     if constexpr (P == 3)
-        fold_rows_kernel<T, R><<<grid, kThreads, 0, st>>>(fa);
+        fold_rows_kernel<T, R><<<grid, kFoldWarps * 32, 0, st>>>(fa);
     else
         fold_kernel<T, R, P><<<grid, kThreads, 0, st>>>(fa);
 }
@@ -866,8 +956,10 @@ int tcr_scatter(const tcr_scatter_desc* d, void* scratch, int64_t scratch_bytes,
     fa.accumulate = d->accumulate;
     cudaError_t e;
     if (p.path == 0 && d->K == 1) {
-        const int64_t rows = d->B * ((d->N + kThreads - 1) / kThreads);
-        e = launch_fold<3>(d->dtype, d->reduce, fa, grid_for(rows * kThreads), st);
+        // one warp per 32 rows; at most four times the blocks that are resident at once
+        const int64_t blocks = (d->B * ((d->N + 31) / 32) + kFoldWarps - 1) / kFoldWarps;
+        e = launch_fold<3>(d->dtype, d->reduce, fa,
+                           (unsigned)(blocks < (int64_t)sm_count() * 28 ? blocks : (int64_t)sm_count() * 28), st);
     } else {
         const unsigned grid = grid_for(nout);
         e = p.path == 0   ? launch_fold<0>(d->dtype, d->reduce, fa, grid, st)
