@@ -20,6 +20,7 @@ import torch
 
 from . import _lib
 from . import context as _context
+from .scatter import index_stats
 from .search import _as_f32, _check_device_fault, _domain_host, _ptr, _require_cuda, _to_host
 from .util import DomainDescription, PointCloud, SparseCOO, SparseCSR
 
@@ -308,8 +309,11 @@ def radiusSearchBatch(queryPointClouds: Sequence[PointCloud],
         dims = [pc.positions.shape[1] for pc in queryPointClouds]
         doms = _domain_list(domain, n, dims, device)
         Ls = [hashMapLength] * n if isinstance(hashMapLength, int) else list(hashMapLength)
+        # the table's columns as lists, one row per cloud, assigned once: sixteen field assignments per
+        # cloud and its domain's six tensor operations made 256 clouds 3.5 ms of host work before the first launch
         table = cloud_table(n)
         keep = []
+        rows = []
         for k in range(n):
             q, r = queryPointClouds[k], refs[k]
             dim = dims[k]
@@ -317,36 +321,71 @@ def radiusSearchBatch(queryPointClouds: Sequence[PointCloud],
                 raise ValueError(f"cloud {k}: query and reference dimensions differ")
             xq = _as_f32(q.positions, device)
             xr = xq if self_search else _as_f32(r.positions, device)
+            nq, nr = xq.shape[0], xr.shape[0]
             if supportOverride is not None:
-                hq = torch.full((xq.shape[0],), float(supportOverride), dtype=torch.float32, device=device)
-                hr = hq if self_search else torch.full((xr.shape[0],), float(supportOverride), dtype=torch.float32,
-                                                       device=device)
+                hq = torch.full((nq,), float(supportOverride), dtype=torch.float32, device=device)
+                hr = hq if self_search else torch.full((nr,), float(supportOverride), dtype=torch.float32, device=device)
             else:
                 hq = None if q.supports is None else _as_f32(q.supports, device)
                 hr = hq if self_search else (None if r.supports is None else _as_f32(r.supports, device))
-            if mode in ("gather", "symmetric", "superSymmetric") and hq is None:
+            if hq is None and mode in ("gather", "symmetric", "superSymmetric"):
                 raise AssertionError(f"cloud {k}: query supports must be provided for {mode} mode")
-            if mode in ("scatter", "symmetric", "superSymmetric") and hr is None:
+            if hr is None and mode in ("scatter", "symmetric", "superSymmetric"):
                 raise AssertionError(f"cloud {k}: reference supports must be provided for {mode} mode")
-            keep.extend([xq, xr, hq, hr])
+            keep.append((xq, xr, hq, hr))
             lo, hi, mask = doms[k]
-            table["dim"][k] = dim
-            table["periodic_mask"][k] = mask
-            table["domain_min"][k, :dim] = lo
-            table["domain_max"][k, :dim] = hi
-            table["hash_map_length"][k] = int(Ls[k])
-            table["n_query"][k] = xq.shape[0]
-            table["n_ref"][k] = xr.shape[0]
-            table["query_pos"][k] = xq.data_ptr() if xq.numel() else 0
-            table["ref_pos"][k] = xr.data_ptr() if xr.numel() else 0
-            table["query_sup"][k] = hq.data_ptr() if hq is not None and hq.numel() else 0
-            table["ref_sup"][k] = hr.data_ptr() if hr is not None and hr.numel() else 0
+            pq = xq.data_ptr() if nq else 0
+            sq = hq.data_ptr() if hq is not None and hq.numel() else 0
+            if self_search:
+                pr, sr = pq, sq
+            else:
+                pr = xr.data_ptr() if nr else 0
+                sr = hr.data_ptr() if hr is not None and hr.numel() else 0
+            rows.append((mask, (lo + [0.0, 0.0])[:3], (hi + [1.0, 1.0])[:3], int(Ls[k]), nq, nr, pq, sq, pr, sr))
+        cols = list(zip(*rows))
+        table["dim"] = dims
+        for name, col in zip(("periodic_mask", "domain_min", "domain_max", "hash_map_length", "n_query", "n_ref"), cols):
+            table[name] = col
+        for name, col in zip(("query_pos", "query_sup", "ref_pos", "ref_sup"), cols[6:]):
+            table[name] = np.array(col, dtype=np.uint64)
         if verbose:
             print(f"radiusSearchBatch: {n} clouds, {int(table['n_query'].sum())} queries, "
                   f"{int(table['n_ref'].sum())} references, mode {mode}, format {format}")
         out = run_batch(table, mode, self_search, format, device, local_index=True)
         del keep
         return BatchedAdjacency(format, out, table["n_query"], table["n_ref"])
+
+
+# Batch ids a sorted batch vector may span to be counted by their boundaries (one search per id).
+SORTED_ID_SPAN = 1 << 16
+
+
+def _one_each(x, batch, support):
+    """One batch id (and, where there is a tensor of them, one support) per point."""
+    n = x.shape[0]
+    return batch.dim() == 1 and batch.shape[0] == n and not (
+        torch.is_tensor(support) and support.dim() > 0 and support.shape[0] != n)
+
+
+def _sorted_counts(bx, by, same_cloud):
+    """Points per batch id, int64 [2, ids] (queries, references), when both batch vectors are sorted (as a
+    loader's are) and their ids span little; None otherwise.  One pass over each vector and a binary
+    search per id, where finding the order takes a unique and a stable sort of every id (a 270k-point
+    radius call: 1068 us, now 652)."""
+    parts = (bx,) if same_cloud else (bx, by)
+    if any(t.dim() != 1 or t.numel() == 0 for t in parts):
+        return None
+    parts = tuple(t.contiguous() for t in parts)
+    stats = [index_stats(t) for t in parts]
+    lo, hi = min(s[0] for s in stats), max(s[1] for s in stats)
+    if any(s[2] for s in stats) or hi - lo >= SORTED_ID_SPAN:
+        return None
+    edges = torch.arange(lo, hi + 2, device=bx.device)
+    at = torch.stack([torch.searchsorted(t, edges) for t in parts]).cpu().numpy()
+    counts = np.diff(at.astype(np.int64), axis=1)
+    if same_cloud:
+        counts = np.concatenate([counts, counts])
+    return np.ascontiguousarray(counts[:, counts.any(axis=0)])
 
 
 def radius_batched(xq, xr, support, batch_x, batch_y, mode="gather", domain=None, hashMapLength=4096,
@@ -365,25 +404,38 @@ def radius_batched(xq, xr, support, batch_x, batch_y, mode="gather", domain=None
         batch_y = batch_x if same_cloud else torch.zeros(xr.shape[0], dtype=torch.long, device=xr.device)
     bx = batch_x.to(device=device, dtype=torch.long)
     by = bx if same_cloud else batch_y.to(device=device, dtype=torch.long)
-    ids = torch.unique(torch.cat([bx, by]))
-    C = int(ids.numel())
-    if C == 0:
-        e = torch.empty(0, dtype=torch.long, device=xq.device)
-        return e, e
-    cq = torch.searchsorted(ids, bx)
-    cr = cq if same_cloud else torch.searchsorted(ids, by)
-    oq = torch.argsort(cq, stable=True)
-    orr = oq if same_cloud else torch.argsort(cr, stable=True)
-    nq = torch.bincount(cq, minlength=C)
-    nr = nq if same_cloud else torch.bincount(cr, minlength=C)
-    counts = torch.stack([nq, nr]).cpu().numpy().astype(np.int64)
-    xs = _as_f32(xq, device).index_select(0, oq).contiguous()
-    ys = xs if same_cloud else _as_f32(xr, device).index_select(0, orr).contiguous()
+    counts = None
+    if _one_each(xq, bx, support[0] if isinstance(support, (tuple, list)) else support) and (
+            same_cloud or _one_each(xr, by, support[1] if isinstance(support, (tuple, list)) else None)):
+        counts = _sorted_counts(bx, by, same_cloud)
+    if counts is not None:  # clouds are consecutive already: no order to find, no points to move
+        oq = orr = None
+        C = counts.shape[1]
+    else:
+        ids = torch.unique(torch.cat([bx, by]))
+        C = int(ids.numel())
+        if C == 0:
+            e = torch.empty(0, dtype=torch.long, device=xq.device)
+            return e, e
+        cq = torch.searchsorted(ids, bx)
+        cr = cq if same_cloud else torch.searchsorted(ids, by)
+        oq = torch.argsort(cq, stable=True)
+        orr = oq if same_cloud else torch.argsort(cr, stable=True)
+        nq = torch.bincount(cq, minlength=C)
+        nr = nq if same_cloud else torch.bincount(cr, minlength=C)
+        counts = torch.stack([nq, nr]).cpu().numpy().astype(np.int64)
+
+    def ordered(t, order):
+        t = _as_f32(t, device)
+        return t if order is None else t.index_select(0, order).contiguous()
+
+    xs = ordered(xq, oq)
+    ys = xs if same_cloud else ordered(xr, orr)
     if isinstance(support, (tuple, list)):
-        hq = _as_f32(support[0], device).index_select(0, oq).contiguous()
-        hr = _as_f32(support[1], device).index_select(0, orr).contiguous()
+        hq = ordered(support[0], oq)
+        hr = ordered(support[1], orr)
     elif torch.is_tensor(support) and support.dim() > 0:
-        hq = _as_f32(support, device).index_select(0, oq).contiguous()
+        hq = ordered(support, oq)
         hr = hq if same_cloud else None
     else:
         hq = torch.full((xs.shape[0],), float(support), dtype=torch.float32, device=device)
@@ -409,8 +461,8 @@ def radius_batched(xq, xr, support, batch_x, batch_y, mode="gather", domain=None
         table["query_sup"] = np.where(counts[0] > 0, hq.data_ptr() + qoff * 4, 0)
     if hr is not None and hr.numel():
         table["ref_sup"] = np.where(counts[1] > 0, hr.data_ptr() + roff * 4, 0)
-    qids = oq.to(torch.int32)
-    rids = qids if same_cloud else orr.to(torch.int32)
+    qids = None if oq is None else oq.to(torch.int32)
+    rids = qids if same_cloud else (None if orr is None else orr.to(torch.int32))
     out = run_batch(table, mode, same_cloud, "coo", device, local_index=False, query_ids=qids, ref_ids=rids)
     i, j = out["row"], out["col"]
     if xq.device.type == "cpu":

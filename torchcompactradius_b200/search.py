@@ -61,6 +61,8 @@ def _as_f32(t, device, shape=None):
     process, since the reference searches float64 inputs in double and pairs whose distance lies
     within float32 rounding of the threshold can then differ."""
     global _warned_f64
+    if type(t) is torch.Tensor and t.dtype is torch.float32 and t.device == device and t.is_contiguous():
+        return t
     t = torch.as_tensor(t)
     if t.dtype == torch.float64 and not _warned_f64:
         _warned_f64 = True
@@ -75,12 +77,17 @@ def _ptr(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
+def _flat_list(t):
+    """The values of a tensor (or what becomes one) as a flat list."""
+    if type(t) is torch.Tensor and t.dim() == 1:
+        return t.tolist()
+    return torch.as_tensor(t).detach().cpu().reshape(-1).tolist()
+
+
 def _domain_host(domain, dim):
-    lo = [float(v) for v in torch.as_tensor(domain.min).detach().cpu().reshape(-1).tolist()]
-    hi = [float(v) for v in torch.as_tensor(domain.max).detach().cpu().reshape(-1).tolist()]
-    per = torch.as_tensor(domain.periodic).detach().cpu().reshape(-1).tolist()
-    if isinstance(per, bool):
-        per = [per] * dim
+    lo = [float(v) for v in _flat_list(domain.min)]
+    hi = [float(v) for v in _flat_list(domain.max)]
+    per = _flat_list(domain.periodic)
     if len(per) == 1 and dim > 1:
         per = per * dim
     if len(lo) != dim or len(hi) != dim or len(per) != dim:
