@@ -280,6 +280,24 @@ typedef struct tcr_f64_inputs {
     double domain_max[3];
 } tcr_f64_inputs;
 
+/* What a float64 search needs before its structure: the wrapped positions (queries once, references
+ * twice; wrap is remainder(x - min, max - min) + min on the periodic dimensions), float32 copies of
+ * positions and supports, and four numbers for the cell size.  query_* / ref_* outputs may be NULL when not
+ * wanted; ref_pos NULL with self_search set: the references are the queries.  stats: device, 4 x
+ * uint64; stats_host (pinned, 4 x double, may be NULL) receives, asynchronously, the largest |wrapped
+ * coordinate| of the queries and of the references, the largest query support and the largest reference
+ * support (NaN when one is NaN, -infinity when there is none). */
+typedef struct tcr_f64_prepare_desc {
+    int32_t dim, periodic_mask, self_search, reserved;
+    double domain_min[3], domain_max[3];
+    int64_t n_query, n_ref;
+    const double *query_pos, *query_sup, *ref_pos, *ref_sup; /* device inputs */
+    double *query_wrapped, *ref_wrapped;                     /* device [n * dim] */
+    float *query_pos_f, *query_sup_f, *ref_pos_f, *ref_sup_f;
+    void* stats;
+} tcr_f64_prepare_desc;
+int tcr_f64_prepare(const tcr_f64_prepare_desc* d, double* stats_host, void* stream);
+
 /* countNeighbors at scalar_t = double (neighborhoodDynamic.h:37-74) + the offsets scan; d describes
  * the float32 copies the structure was built from (hcell > 0, clamped_grid 0).  stage and the other
  * arguments as in tcr_count. */

@@ -94,6 +94,16 @@ class F64Inputs(ctypes.Structure):
     ]
 
 
+class F64PrepareDesc(ctypes.Structure):
+    """tcr_f64_prepare_desc (include/tcr_b200.h): wrapping and copying of a float64 search's inputs."""
+    _fields_ = [("dim", ctypes.c_int32), ("periodic_mask", ctypes.c_int32), ("self_search", ctypes.c_int32),
+                ("reserved", ctypes.c_int32), ("domain_min", ctypes.c_double * 3), ("domain_max", ctypes.c_double * 3),
+                ("n_query", ctypes.c_int64), ("n_ref", ctypes.c_int64)] + [
+        (name, ctypes.c_void_p) for name in (
+            "query_pos", "query_sup", "ref_pos", "ref_sup", "query_wrapped", "ref_wrapped", "query_pos_f",
+            "query_sup_f", "ref_pos_f", "ref_sup_f", "stats")]
+
+
 class ScatterDesc(ctypes.Structure):
     """tcr_scatter_desc (include/tcr_b200.h): one reduction of values onto an index."""
     _fields_ = [
@@ -142,6 +152,7 @@ SIGNATURES = {
     "tcr_search_noalloc": (ctypes.c_int, [_desc_p, _vp, _vp, _vp, _vp, _vp, _i64, ctypes.POINTER(_i64), _vp]),
     "tcr_count_f64": (ctypes.c_int, [_desc_p, ctypes.POINTER(F64Inputs), _vp, _vp, _i64, _vp, _i64, _vp, _vp, _vp,
                                      _vp, _vp]),
+    "tcr_f64_prepare": (ctypes.c_int, [ctypes.POINTER(F64PrepareDesc), _vp, _vp]),
     "tcr_emit_f64": (ctypes.c_int, [_desc_p, ctypes.POINTER(F64Inputs), _vp, _vp, _i64, _vp, _vp, _vp, _vp, _i64,
                                     _vp]),
     "tcr_scatter_desc_bytes": (_i64, []),

@@ -5,8 +5,9 @@ for float64 positions its grid, its periodic wrap and every distance test are do
 keeps that arithmetic where it decides pairs and uses float32 only to find candidates:
 
 * positions are wrapped in double exactly as the reference wraps them -- queries once
-  (util.py:375-387), references twice (that, then compactHashing/cppSearch.py:221) -- with the
-  same torch operation, ``remainder(x - min, max - min) + min``;
+  (util.py:375-387), references twice (that, then compactHashing/cppSearch.py:221) -- by
+  ``remainder(x - min, max - min) + min``, in the one pass of ``tcr_f64_prepare`` that also makes the
+  float32 copies and the maxima the cell size needs;
 * the reference's cell size is computed in double (``compute_h``, util.py:28-79, on the mode's
   maximum support, compactHashing/cellTable.py:40-81), then rounded up to float32 and padded by a
   few float32 ulps of the largest coordinate, so that the float32 cell of every point is at least
@@ -21,6 +22,7 @@ dimension (they differ only for a domain extent within a few ulps of a whole num
 """
 import ctypes
 import math
+import threading
 
 import numpy as np
 import torch
@@ -59,13 +61,64 @@ def compute_h64(lo, hi, hmax: float) -> float:
     return float(np.max(h))
 
 
-def grid_support64(hq, hr, mode: str) -> float:
-    """cellTable.py:40-81: the largest support the mode reads."""
+def grid_support64(hq_max: float, hr_max: float, mode: str) -> float:
+    """cellTable.py:40-81: the largest support the mode reads (given the maxima of both arrays)."""
     if mode == "scatter":
-        return float(hr.max())
+        return hr_max
     if mode == "gather":
-        return float(hq.max())
-    return max(float(hr.max()), float(hq.max()))
+        return hq_max
+    return max(hr_max, hq_max)
+
+
+_tls = threading.local()
+
+
+def prepare64(xq, hq, xr, hr, lo, hi, mask, self_search, same_sup):
+    """Wrapped positions, float32 copies and the four maxima of ``tcr_f64_prepare`` (one host wait).  xr None:
+    a search of new queries against a kept structure.  Returns (xq_w, xq_f, hq_f, xr_w, xr_f, hr_f, maxima)."""
+    device, dim, nq = xq.device, xq.shape[1], xq.shape[0]
+    nr = 0 if xr is None else xr.shape[0]
+    if (hq is not None and hq.numel() < nq) or (xr is not None and hr is not None and hr.numel() < nr):
+        raise ValueError("fewer supports than points")
+
+    def new(shape, dtype):
+        return torch.empty(shape, dtype=dtype, device=device)
+
+    xq_w, xq_f = new(xq.shape, torch.float64), new(xq.shape, torch.float32)
+    xr_w = new(xr.shape, torch.float64) if xr is not None else None
+    xr_f = None if xr is None else (xq_f if self_search else new(xr.shape, torch.float32))
+    hq_f = None if hq is None else new(hq.shape, torch.float32)
+    shared = self_search and same_sup
+    hr_f = None if hr is None or xr is None else (hq_f if shared else new(hr.shape, torch.float32))
+    stats = torch.empty(4, dtype=torch.float64, device=device)
+    host = getattr(_tls, "stats", None)
+    if host is None:
+        host = _tls.stats = torch.zeros(4, dtype=torch.float64, pin_memory=True)
+    d = _lib.F64PrepareDesc()
+    d.dim, d.periodic_mask, d.self_search = dim, mask, 1 if (self_search and xr is not None) else 0
+    for k in range(3):
+        d.domain_min[k] = lo[k] if k < dim else 0.0
+        d.domain_max[k] = hi[k] if k < dim else 1.0
+    d.n_query, d.n_ref = nq, nr
+
+    def at(t):
+        return t.data_ptr() if t is not None and t.numel() else None
+
+    d.query_pos, d.query_sup = at(xq), at(hq)
+    d.ref_pos, d.ref_sup = (None if xr is None or self_search else at(xr)), (None if xr is None else at(hr))
+    d.query_wrapped, d.ref_wrapped = at(xq_w), at(xr_w)
+    d.query_pos_f, d.query_sup_f = at(xq_f), at(hq_f)
+    d.ref_pos_f, d.ref_sup_f = (None if self_search else at(xr_f)), (None if shared else at(hr_f))
+    d.stats = stats.data_ptr()
+    stream = torch.cuda.current_stream(device)
+    wait = xr is not None  # (a kept structure has its cell size: nothing is read back)
+    _lib.check(_lib.load().tcr_f64_prepare(ctypes.byref(d), ctypes.c_void_p(host.data_ptr()) if wait else None,
+                                           ctypes.c_void_p(stream.cuda_stream)), "tcr_f64_prepare")
+    maxima = None
+    if wait:
+        stream.synchronize()
+        maxima = host.tolist()
+    return xq_w, xq_f, hq_f, xr_w, xr_f, hr_f, maxima
 
 
 def compact_search_f64(xq, hq, xr, hr, lo, hi, mask, mode, L, fmt, self_search, return_structure=False,
@@ -82,30 +135,25 @@ def compact_search_f64(xq, hq, xr, hr, lo, hi, mask, mode, L, fmt, self_search, 
     nq = xq.shape[0]
     stream = torch.cuda.current_stream(device)
     sptr = ctypes.c_void_p(stream.cuda_stream)
-    xq_w = wrap64(xq, lo, hi, mask)
     if structure is not None:  # references, cell size and float32 copies of an earlier build
         f = structure._f64
         xr_w, hr, xr_f, hr_f, hcell = f["xr_w"], f["hr"], f["xr_f"], f["hr_f"], f["hcell"]
         self_search = False
+        xq_w, xq_f, hq_f, _, _, _, _ = prepare64(xq, hq, None, None, lo, hi, mask, False, False)
     else:
-        xr_w = wrap64(wrap64(xr, lo, hi, mask), lo, hi, mask)
+        xq_w, xq_f, hq_f, xr_w, xr_f, hr_f, maxima = prepare64(xq, hq, xr, hr, lo, hi, mask, self_search, hq is hr)
     nr = xr_w.shape[0]
     if structure is None:
-        hc = compute_h64(lo, hi, grid_support64(hq, hr, mode)) if nq and nr else 1.0
+        hc = compute_h64(lo, hi, grid_support64(maxima[2], maxima[3], mode)) if nq and nr else 1.0
         if not (math.isfinite(hc) and hc > 0.0):
             raise ValueError("no valid cell grid for this domain and support (the support is not smaller than the "
                              "domain extent, or a support/domain value is not finite)")
         big = max([abs(v) for v in lo] + [abs(v) for v in hi] +
-                  [float(t.abs().max()) for t in (xq_w, xr_w) if t.numel()])
+                  [m for m, t in zip(maxima, (xq_w, xr_w)) if t.numel()])
         padded = hc + 8.0 * 2.0 ** -24 * big
         hcell = np.float32(padded)
         if float(hcell) < padded:
             hcell = np.nextafter(hcell, np.float32(np.inf))
-    xq_f = xq_w.float().contiguous()
-    hq_f = None if hq is None else hq.float().contiguous()
-    if structure is None:
-        xr_f = xq_f if self_search else xr_w.float().contiguous()
-        hr_f = None if hr is None else (hq_f if (self_search and hq is hr) else hr.float().contiguous())
     desc = make_desc(dim, mode, mask, lo, hi, L, xq_f, hq_f, xr_f, hr_f, self_search)
     for k in range(dim):
         desc.hcell[k] = float(hcell)
