@@ -84,7 +84,7 @@ struct Carve {
 // Persistent structure (reference side); kept alive for reuse.
 struct Structure {
     GridParams* grid;         // [C] per cloud
-    int32_t* num_cells;       // [2] cells; set when a one-launch sort gave up waiting
+    int32_t* num_cells;       // [3] cells; set when a one-launch sort gave up waiting; blocks of the statistics that finished
     int32_t* bad_grids;       // [1] clouds with points on both sides and no valid grid
     float4* rsorted;          // [nr] wrapped reference points in (cloud, cell) order, .w = support
     int32_t* rsidx;           // [nr] global index of each sorted point
@@ -101,7 +101,7 @@ static Structure carve_structure(void* buf, int64_t nr, int64_t C, int64_t map_t
     Carve c{(char*)buf, 0};
     Structure s;
     s.grid = c.take<GridParams>(C);
-    s.num_cells = c.take<int32_t>(2);
+    s.num_cells = c.take<int32_t>(3);
     s.bad_grids = c.take<int32_t>(1);
     s.rsorted = c.take<float4>(nr);
     s.rsidx = c.take<int32_t>(nr);
@@ -321,86 +321,12 @@ __device__ __forceinline__ void stats_atomic(SupportStats* s, uint32_t kmax, int
     if (bad) atomicOr(&s->bad, 1);
 }
 
-// Per-cloud maximum support (computeGridSupport, cellTable.py:40-81, needs it) and whether every
-// support lies in [1e-18, 1e18] (else the exact test decides every pair).  Each block reduces a
-// contiguous range, so a thread changes cloud only at cloud boundaries; a block that stayed in one
-// cloud issues one atomic per field.  The record of cloud c is at out + c * stride.
-__global__ void support_stats_kernel(const CloudParams* __restrict__ table, const int32_t* __restrict__ prefix, int C,
-                                     int64_t n, int query_side, char* out, int64_t stride) {
-    const int64_t per = (n + gridDim.x - 1) / gridDim.x;
-    const int64_t lo = (int64_t)blockIdx.x * per;
-    const int64_t hi = min(n, lo + per);
-    int cur = -1;
-    int64_t cbase = 0, cend = 0;
-    const float* h = nullptr;
-    uint32_t kmax = 0;
-    int bad = 0;
-    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-        if (cur < 0 || i >= cend) {
-            if (cur >= 0) stats_atomic(stats_at(out, stride, cur), kmax, bad);
-            cur = cloud_of(prefix, C, i);
-            cbase = prefix[cur];
-            cend = prefix[cur + 1];
-            h = query_side ? table[cur].query_sup : table[cur].ref_sup;
-            kmax = 0;
-            bad = 0;
-        }
-        if (h) {
-            const float v = h[i - cbase];
-            kmax = max(kmax, float_key(v));
-            bad |= !(v >= 1e-18f && v <= 1e18f);
-        }
-    }
-    __shared__ int s_cloud;
-    if (threadIdx.x == 0) s_cloud = cur;  // thread 0 holds the block's first point, if it has any
-    __syncthreads();
-    if (__syncthreads_and(cur < 0 || cur == s_cloud)) {
-        if (s_cloud >= 0) block_reduce_stats(kmax, bad, stats_at(out, stride, s_cloud));
-    } else if (cur >= 0) {
-        stats_atomic(stats_at(out, stride, cur), kmax, bad);
-    }
-}
-
-// Start of a build: the (last clouds of the) table, per-cloud statistics and flags, counters, the sort
-// state, an empty map.
-template <typename K>
-__global__ void grid_init_kernel(const __grid_constant__ CloudChunk<kUploadChunk> ch, GridParams* g, int C, Structure S,
-                                 Scratch W) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
-        g[c].ref_stats.max_key = 0;
-        g[c].ref_stats.bad = 0;
-        g[c].build_query_stats.max_key = 0;
-        g[c].build_query_stats.bad = 0;
-        g[c].error = 0;
-        g[c].out_of_grid = 0;
-    }
-    ulonglong2* map = reinterpret_cast<ulonglong2*>(S.map);  // capacities are powers of two >= 64
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < S.map_total / 2;
-         i += (int64_t)gridDim.x * blockDim.x)
-        map[i] = make_ulonglong2(~0ull, ~0ull);
-    if (blockIdx.x != 0) return;
-    upload_chunk(ch, W.table, W.query_prefix, W.ref_prefix);
-    if (threadIdx.x == 0) {
-        *S.bad_grids = 0;
-        S.num_cells[0] = S.num_cells[1] = 0;
-        sort_state_reset(reinterpret_cast<SortStateT<K>*>(W.sort_state));
-    }
-}
-
-template <typename K>
-__global__ void sort_state_init_kernel(SortStateT<K>* st) { sort_state_reset(st); }
-
-// End of the last cell (or query group): cell_start[C] = n.
-__global__ void finish_cells_kernel(int32_t* cell_start, const int32_t* num_cells, int64_t n) {
-    cell_start[*num_cells] = (int32_t)n;
-}
-
 // Per cloud: util.py:28-79 compute_h and cellTable.py:27-29, float32 throughout.
 // same_sup: the query supports are the reference support array (statistics reduced once).
-__global__ void grid_params_kernel(const CloudParams* __restrict__ table, GridParams* grid, int C,
-                                   int32_t* bad_grids, int same_sup) {
+__device__ __forceinline__ void grid_params(const CloudParams* __restrict__ table, GridParams* grid, int C,
+                                            int32_t* bad_grids, int same_sup, int first, int stride) {
     const float grow = 1.00010001659393310546875f;  // fl32(1e-4 + 1)
-    for (int cl = blockIdx.x * blockDim.x + threadIdx.x; cl < C; cl += gridDim.x * blockDim.x) {
+    for (int cl = first; cl < C; cl += stride) {
         const CloudParams& sp = table[cl];
         GridParams* g = &grid[cl];
         if (same_sup) g->build_query_stats = g->ref_stats;
@@ -472,6 +398,96 @@ __global__ void grid_params_kernel(const CloudParams* __restrict__ table, GridPa
         g->error = err;
         if (err && sp.n_query > 0 && sp.n_ref > 0) atomicAdd(bad_grids, 1);
     }
+}
+__global__ void grid_params_kernel(const CloudParams* __restrict__ table, GridParams* grid, int C, int32_t* bad_grids,
+                                   int same_sup) {
+    grid_params(table, grid, C, bad_grids, same_sup, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// Per-cloud maximum support (computeGridSupport, cellTable.py:40-81, needs it) and whether every
+// support lies in [1e-18, 1e18] (else the exact test decides every pair).  Each block reduces a
+// contiguous range, so a thread changes cloud only at cloud boundaries; a block that stayed in one
+// cloud issues one atomic per field.  The record of cloud c is at out + c * stride.  With `done` (a
+// build's last statistics) the last block to finish writes the clouds' grid parameters.
+__global__ void support_stats_kernel(const CloudParams* __restrict__ table, const int32_t* __restrict__ prefix, int C,
+                                     int64_t n, int query_side, char* out, int64_t stride, GridParams* grid = nullptr,
+                                     int32_t* bad_grids = nullptr, int same_sup = 0, int32_t* done = nullptr) {
+    const int64_t per = (n + gridDim.x - 1) / gridDim.x;
+    const int64_t lo = (int64_t)blockIdx.x * per;
+    const int64_t hi = min(n, lo + per);
+    int cur = -1;
+    int64_t cbase = 0, cend = 0;
+    const float* h = nullptr;
+    uint32_t kmax = 0;
+    int bad = 0;
+    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+        if (cur < 0 || i >= cend) {
+            if (cur >= 0) stats_atomic(stats_at(out, stride, cur), kmax, bad);
+            cur = cloud_of(prefix, C, i);
+            cbase = prefix[cur];
+            cend = prefix[cur + 1];
+            h = query_side ? table[cur].query_sup : table[cur].ref_sup;
+            kmax = 0;
+            bad = 0;
+        }
+        if (h) {
+            const float v = h[i - cbase];
+            kmax = max(kmax, float_key(v));
+            bad |= !(v >= 1e-18f && v <= 1e18f);
+        }
+    }
+    __shared__ int s_cloud;
+    if (threadIdx.x == 0) s_cloud = cur;  // thread 0 holds the block's first point, if it has any
+    __syncthreads();
+    if (__syncthreads_and(cur < 0 || cur == s_cloud)) {
+        if (s_cloud >= 0) block_reduce_stats(kmax, bad, stats_at(out, stride, s_cloud));
+    } else if (cur >= 0) {
+        stats_atomic(stats_at(out, stride, cur), kmax, bad);
+    }
+    if (!done) return;
+    __shared__ int s_last;
+    __threadfence();  // this thread's atomics before the block's arrival
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last) grid_params(table, grid, C, bad_grids, same_sup, threadIdx.x, blockDim.x);
+}
+
+// Start of a build: the (last clouds of the) table, per-cloud statistics and flags, counters, the sort
+// state, an empty map.
+template <typename K>
+__global__ void grid_init_kernel(const __grid_constant__ CloudChunk<kUploadChunk> ch, GridParams* g, int C, Structure S,
+                                 Scratch W) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
+        g[c].ref_stats.max_key = 0;
+        g[c].ref_stats.bad = 0;
+        g[c].build_query_stats.max_key = 0;
+        g[c].build_query_stats.bad = 0;
+        g[c].error = 0;
+        g[c].out_of_grid = 0;
+    }
+    ulonglong2* map = reinterpret_cast<ulonglong2*>(S.map);  // capacities are powers of two >= 64
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < S.map_total / 2;
+         i += (int64_t)gridDim.x * blockDim.x)
+        map[i] = make_ulonglong2(~0ull, ~0ull);
+    if (blockIdx.x != 0) return;
+    upload_chunk(ch, W.table, W.query_prefix, W.ref_prefix);
+    if (threadIdx.x == 0) {
+        *S.bad_grids = 0;
+        S.num_cells[0] = S.num_cells[1] = S.num_cells[2] = 0;
+        sort_state_reset(reinterpret_cast<SortStateT<K>*>(W.sort_state));
+    }
+}
+
+template <typename K>
+__global__ void sort_state_init_kernel(SortStateT<K>* st) { sort_state_reset(st); }
+
+// End of the last cell (or query group): cell_start[C] = n.
+__global__ void finish_cells_kernel(int32_t* cell_start, const int32_t* num_cells, int64_t n) {
+    cell_start[*num_cells] = (int32_t)n;
 }
 
 // One cloud's query-side parameters of the lean test.  same_sup: the queries' supports are the
@@ -1989,8 +2005,9 @@ __global__ void __launch_bounds__(kWalkWarps * 32, PERIODIC ? kWalkMinBlocksPeri
     int32_t* counter = &a.work[a.class_filter >= 0 ? 2 + a.class_filter : 0];
     int cur = -1;
     const bool filter = a.class_filter >= 0;
-    int32_t claim = 0;
-    if (lane == 0) claim = atomicAdd(counter, filter ? 32 : 1);
+    // the first claim of every warp is its own number, the counter's come after them
+    const int32_t step = filter ? 32 : 1, first = (int32_t)(gridDim.x * kWalkWarps) * step;
+    int32_t claim = (int32_t)(blockIdx.x * kWalkWarps + w) * step;
     for (;;) {
         const int32_t base = __shfl_sync(0xffffffffu, claim, 0);
         if (base >= nunits) break;
@@ -2003,7 +2020,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, PERIODIC ? kWalkMinBlocksPeri
         }
         // the next claim is issued before this one's units run and read after them, so the
         // atomic's latency overlaps their work
-        if (lane == 0) claim = atomicAdd(counter, filter ? 32 : 1);
+        if (lane == 0) claim = first + atomicAdd(counter, step);
         while (todo) {
             const int32_t unit = base + (__ffs(todo) - 1);
             todo &= todo - 1;
@@ -2240,16 +2257,18 @@ __global__ void __launch_bounds__(kExpandWarps * 32, 4) expand_records_kernel(co
     // A unit is claimed three iterations before it runs, its record offset and first query are read two
     // before, its record's first 64 words (the header and the runs) and query rows (lane < 32 covers every
     // unit size) one before, so a unit starts with them at hand instead of dependent round trips.
-    auto claim = [&]() -> int32_t { return lane == 0 ? atomicAdd(a.work, 1) : 0; };
+    // (the first two are the warp's own number and the next round's, the counter's come after them)
+    const int32_t warps = (int32_t)gridDim.x * kExpandWarps;
+    auto claim = [&]() -> int32_t { return lane == 0 ? 2 * warps + atomicAdd(a.work, 1) : 0; };
     auto words_of = [&](int32_t r0, int32_t k) -> int32_t {
         return (r0 >= 0 && (int64_t)r0 + k < cap) ? a.stage[r0 + k] : 0;
     };
     auto qrows = [&](int32_t v, int32_t t0) -> int32_t {
         return (v < nu && TCR_GUARD(t0 + lane, a.nq)) ? a.qsidx[t0 + lane] : -1;
     };
-    int32_t ua = __shfl_sync(0xffffffffu, claim(), 0);
-    int32_t ub = __shfl_sync(0xffffffffu, claim(), 0);
-    int32_t next = claim();
+    int32_t ua = (int32_t)blockIdx.x * kExpandWarps + w, ub = ua + warps;
+    if (ua >= nu) return;
+    int32_t next = ub < nu ? claim() : nu;
     int32_t r0a = ua < nu ? a.rec[ua] : -1, t0a = ua < nu ? a.unit_t0[ua] : 0;
     int32_t r0b = ub < nu ? a.rec[ub] : -1, t0b = ub < nu ? a.unit_t0[ub] : 0;
     int32_t ha = words_of(r0a, lane), hb = words_of(r0a, 32 + lane), qa = qrows(ua, t0a);
@@ -3079,21 +3098,27 @@ static int build_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
     grid_init_kernel<K><<<grid_for(std::max<int64_t>(C, S.map_total / 8), 256, num_sms() * 8), 256, 0, st>>>(
         chunk, S.grid, C, S, W);
     note_launches(1);
-    // computeGridSupport: which supports set hMax depends on the mode
-    if (b.any_ref_sup && nr > 0) {
+    // computeGridSupport: which supports set hMax depends on the mode; the last statistics also write the
+    // grid parameters
+    const bool ref_stats = b.any_ref_sup && nr > 0, query_stats = b.any_query_sup && nq > 0 && !b.same_supports;
+    const int same_sup = b.same_supports ? 1 : 0;
+    if (ref_stats) {
         support_stats_kernel<<<grid_for(nr, 256, num_sms() * 4), 256, 0, st>>>(
             W.table, W.ref_prefix, C, nr, 0, reinterpret_cast<char*>(S.grid) + offsetof(GridParams, ref_stats),
-            (int64_t)sizeof(GridParams));
+            (int64_t)sizeof(GridParams), S.grid, S.bad_grids, same_sup, query_stats ? nullptr : S.num_cells + 2);
         note_launches(1);
     }
-    if (b.any_query_sup && nq > 0 && !b.same_supports) {
+    if (query_stats) {
         support_stats_kernel<<<grid_for(nq, 256, num_sms() * 4), 256, 0, st>>>(
             W.table, W.query_prefix, C, nq, 1,
-            reinterpret_cast<char*>(S.grid) + offsetof(GridParams, build_query_stats), (int64_t)sizeof(GridParams));
+            reinterpret_cast<char*>(S.grid) + offsetof(GridParams, build_query_stats), (int64_t)sizeof(GridParams),
+            S.grid, S.bad_grids, same_sup, S.num_cells + 2);
         note_launches(1);
     }
-    grid_params_kernel<<<grid_for(C, 128), 128, 0, st>>>(W.table, S.grid, C, S.bad_grids, b.same_supports ? 1 : 0);
-    note_launches(1);
+    if (!ref_stats && !query_stats) {
+        grid_params_kernel<<<grid_for(C, 128), 128, 0, st>>>(W.table, S.grid, C, S.bad_grids, same_sup);
+        note_launches(1);
+    }
     if (nr > 0) {
         const bool inc = b.lin_hint != nullptr;
         // few blocks: each ends with one atomic on the key range, so thousands of them would queue

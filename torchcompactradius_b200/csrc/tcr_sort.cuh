@@ -301,6 +301,7 @@ struct CoopSmem {
 
 __device__ __forceinline__ bool coop_barrier(unsigned* bar, unsigned target, int32_t* failed, int32_t* flag) {
     __syncthreads();
+    if (gridDim.x == 1) return true;
     if (threadIdx.x == 0) {
         __threadfence();
         atomicAdd(bar, 1u);
@@ -346,12 +347,14 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     const unsigned lt = (1u << lane) - 1u;
     const bool single = per <= kCoopTile;
     const int rounds = (int)((min(per, (int64_t)kCoopTile) + kCoopThreads - 1) / kCoopThreads);
+    const K differ = st->key_min ^ st->key_max;
+    const int top = differ == 0 ? -1 : top_bit(differ);  // the highest bit in which two keys differ
     unsigned phase = 0;
     int sel = st->sel[0];
     bool placed = false;
     for (int pass = 0; pass < key_passes<K>(); ++pass) {
         const int shift = 8 * pass;
-        if (!pass_needed(st, shift)) break;
+        if (top < shift) break;
         const K* kin = sel ? keys1 : keys0;
         const int32_t* vin = sel ? vals1 : vals0;
         K* kout = sel ? keys0 : keys1;
@@ -454,7 +457,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
                 continue;
             }
         }
-        const bool last = Tail::kPlace && !pass_needed(st, shift + 8);
+        const bool last = Tail::kPlace && top < shift + 8;
         for (int64_t t0 = lo; t0 < hi; t0 += kCoopTile) {
             const int len = (int)min((int64_t)kCoopTile, hi - t0);
             const int R = single ? rounds : (len + kCoopThreads - 1) / kCoopThreads;
@@ -525,6 +528,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
 }
 
 inline int coop_blocks(int64_t n, int sms) {
+    if (n <= kCoopTile) return 1;  // one tile: no barriers to pay for (about 2 us each)
     const int64_t want = (n + kCoopMinKeys - 1) / kCoopMinKeys;
     return (int)(want < 1 ? 1 : (want < sms ? want : sms));
 }
