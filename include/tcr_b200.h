@@ -164,7 +164,8 @@ int tcr_search_sizes(int64_t n_query, int64_t n_ref, int32_t dim, int64_t* struc
  *   CELL_LIN      int32 [C] linear cell index (cellTable.py:31)
  *   CELL_COORDS   int32 [3*C] integer cell coordinates
  *   CELL_BUCKET   int32 [C] reference hash of the coordinates mod hashMapLength
- *   MAP           uint64 [cap] open-addressing map (lin << 32 | cell), empty = ~0 */
+ *   MAP           uint64 [cap] entries (lin << 32 | cell), empty = ~0: at slot lin when every point lies in a
+ *                 grid of no more cells than slots, else an open-addressing table */
 #define TCR_STRUCT_GRID 0
 #define TCR_STRUCT_NUM_CELLS 1
 #define TCR_STRUCT_SORTED_POINTS 2

@@ -72,3 +72,20 @@ def test_far_domain_and_tiny_supports(mode):
     h = (10.0 ** rng.uniform(-3, -0.7, 4000)).astype(np.float32)
     y = rng.uniform(-1, 1, (4000, 3)).astype(np.float32)
     check(y, h, None, None, [-1.0] * 3, [1.0] * 3, [False] * 3, mode)
+
+
+@pytest.mark.parametrize("mode", ["gather", "superSymmetric"])
+@pytest.mark.parametrize("per", [[0, 0, 0], [1, 1, 0]])
+@pytest.mark.parametrize("h,outside", [(0.3, False), (0.02, False), (0.002, False), (0.3, True), (0.02, True)])
+def test_cell_maps(mode, per, h, outside):
+    """Grids of fewer and of more cells than the map has slots, and points outside a non-periodic domain:
+    cells found in place and through the open-addressing table."""
+    rng = np.random.default_rng(int(1000 * h))
+    n = 1500
+    x = rng.uniform(-1, 1, (n, 3)).astype(np.float32)
+    x[: n // 2] = x[0] + rng.uniform(-2 * h, 2 * h, (n // 2, 3)).astype(np.float32)  # some neighbours in any case
+    x = np.clip(x, -1, 0.9999).astype(np.float32)
+    if outside:
+        x[:5, 2] += np.float32(3.0)
+    hs = rng.uniform(0.7 * h, h, n).astype(np.float32)
+    assert check(x, hs, None, None, [-1.0] * 3, [1.0] * 3, [bool(p) for p in per], mode) > n

@@ -691,6 +691,15 @@ __device__ __forceinline__ uint32_t mix32(uint32_t x) {
     return x;
 }
 
+// A cloud whose points all lie in a grid of no more cells than its map region has slots keeps them in place:
+// slot = linear index (returned: the cells; 0: the region is an open-addressing table).  A unit's 27
+// look-ups then read neighbouring slots, one read each, instead of 27 scattered probe chains.
+__device__ __forceinline__ uint32_t direct_cells(int dim, const int32_t* count, int out_of_grid, int64_t cap) {
+    double cells = 1.0;
+    for (int d = 0; d < dim; ++d) cells *= (double)max(count[d], 1);
+    return (!out_of_grid && cells <= (double)cap && cells < 2147483648.0) ? (uint32_t)cells : 0u;
+}
+
 __device__ __forceinline__ void map_insert(unsigned long long* map, int64_t cap, int32_t lin, int32_t cell) {
     const unsigned long long entry = ((unsigned long long)(uint32_t)lin << 32) | (uint32_t)cell;
     uint64_t slot = mix32((uint32_t)lin) & (cap - 1);
@@ -701,7 +710,12 @@ __device__ __forceinline__ void map_insert(unsigned long long* map, int64_t cap,
     }
 }
 
-__device__ __forceinline__ int32_t map_find(const unsigned long long* __restrict__ map, int64_t cap, int32_t lin) {
+__device__ __forceinline__ int32_t map_find(const unsigned long long* __restrict__ map, int64_t cap, uint32_t direct,
+                                            int32_t lin) {
+    if (direct) {  // (an empty slot holds -1; a linear index outside the grid names no cell)
+        if ((uint32_t)lin >= direct) return -1;
+        return (int32_t)__ldg(reinterpret_cast<const uint2*>(map) + (uint32_t)lin).x;
+    }
     const uint32_t mask = (uint32_t)(cap - 1);  // capacities are at most 2^32
     uint32_t slot = mix32((uint32_t)lin) & mask;
     for (uint32_t probe = 0; probe <= mask; ++probe) {
@@ -754,7 +768,11 @@ struct BuildTail {
         if (!g.error) {
             cell_of(cp.dim, cp.dedupe, cp.dmin, g.hcell_d, g.count, sorted[i], c);
             bucket = ref_hash(cp.dim, c, cp.hash_len);
-            map_insert(map + cp.map_base, cp.map_cap, lin, cell);
+            const uint32_t direct = direct_cells(cp.dim, g.count, g.out_of_grid, cp.map_cap);
+            if (!direct)
+                map_insert(map + cp.map_base, cp.map_cap, lin, cell);
+            else if ((uint32_t)lin < direct)
+                map[cp.map_base + lin] = ((unsigned long long)(uint32_t)lin << 32) | (uint32_t)cell;
         }
         cell_lin[cell] = lin;
         cell_cloud[cell] = cloud;
@@ -1042,6 +1060,7 @@ struct UnitCtx {
     int32_t plain_cells;  // every point lies in the grid and linear indices do not wrap: an in-range cell's linear
                           // index names that cell only, so its bucket needs no check
     int64_t map_base, map_cap;
+    uint32_t map_direct;     // direct_cells of the cloud
 };
 
 struct WalkArgs {
@@ -1055,7 +1074,7 @@ struct WalkArgs {
     int32_t no_stray_check;       // self search, no periodic dims, same positions: a query's cell is its
                                   // group's unless its cloud has points outside the grid (out_of_grid)
     int32_t class_filter;         // >= 0: walk only units of clouds of this class (dim * 2 + periodic)
-    int32_t pad0;
+    int32_t self;                 // self search: sorted query t is sorted reference t, wrapped once less
     const float4* __restrict__ rsorted;
     const int32_t* __restrict__ rsidx;
     const int32_t* __restrict__ cell_start;
@@ -1139,9 +1158,8 @@ __device__ __forceinline__ void load_unit_ctx(UnitCtx& u, const WalkArgs& a, int
     // a float32 copy of a double coordinate x is off by <= |x| 2^-24, the float difference adds one
     // rounding: 2^-21 of the largest |coordinate| bounds a difference's error with room to spare
     u.f64_err = a.f64.qpos ? key_float(q.coord_key) * 4.76837158203125e-7f : 0.0f;
-    double cells = 1.0;
-    for (int d = 0; d < cp.dim; ++d) cells *= (double)max(g.count[d], 1);
-    u.plain_cells = !g.out_of_grid && cells < 2147483648.0;
+    u.plain_cells = direct_cells(cp.dim, g.count, g.out_of_grid, int64_t(1) << 31) != 0;
+    u.map_direct = direct_cells(cp.dim, g.count, g.out_of_grid, cp.map_cap);
     float cell = 0.0f;
     for (int d = 0; d < cp.dim; ++d) cell = fmaxf(cell, g.hcell_d[d]);
     const uint32_t ex = min(max((__float_as_uint(cell) >> 23) & 0xffu, 1u), 253u);
@@ -1197,7 +1215,7 @@ __device__ __forceinline__ void stencil_lookup(const WalkArgs& a, const UnitCtx&
     cnt = 0;
     if (dup) return;
     const int32_t lin = linear_index(DIM, c, u.count);
-    const int32_t cell = map_find(a.map + u.map_base, u.map_cap, lin);
+    const int32_t cell = map_find(a.map + u.map_base, u.map_cap, u.map_direct, lin);
     if (cell < 0 || !TCR_GUARD(cell, a.nr_total)) return;
     const int32_t b = __ldg(&a.cell_start[cell]), e = __ldg(&a.cell_start[cell + 1]);
     // queryHashMap matches the linear index inside bucket hash(c) only.
@@ -1620,7 +1638,14 @@ __device__ __forceinline__ Unit open_unit(const WalkArgs& a, const UnitCtx& u, i
     n.active = false;
     if (qlane) {
         n.active = TCR_IN(n.qorig, a.nq_total);
-        if (n.active && (!a.no_stray_check || u.out_of_grid)) {
+        bool check = !a.no_stray_check || u.out_of_grid;
+        if (check && a.self && !u.out_of_grid) {
+            // the group's cell is the reference's; where the second wrap changed nothing it is the query's
+            // too (three compares instead of three divisions)
+            const float4 r = __ldg(&a.rsorted[t0 + lane]);
+            check = !(r.x == n.q.x && (DIM < 2 || r.y == n.q.y) && (DIM < 3 || r.z == n.q.z));
+        }
+        if (n.active && check) {
             int32_t qc[3];
             cell_of(DIM, u.dedupe, u.dmin, u.hcell, u.count, n.q, qc);
             n.active = same_cell<DIM>(qc, n.gc);
@@ -2975,6 +3000,7 @@ static WalkArgs make_walk(const HostBatch& b, const Structure& S, const Scratch&
     a.local_index = b.local_index;
     a.mode = b.mode;
     a.no_stray_check = b.same_positions ? 1 : 0;
+    a.self = b.self;
     a.rsorted = S.rsorted;
     a.rsidx = S.rsidx;
     a.cell_start = S.cell_start;
