@@ -6,11 +6,12 @@
 // over all clouds, on one CUDA stream, with no host synchronisation inside a phase:
 //   build:  per-cloud support max-reductions -> per-cloud grid parameters (compute_h) -> wrap and
 //           pack reference points into float4 (x, y, z, h) with (cloud, linear cell) sort keys ->
-//           stable radix sort -> run-length cell table (begin, coords, bucket, cloud) and one
-//           open-addressing lin -> cell map region per cloud.
+//           one cooperative launch: stable radix sort, placement, run-length cell table (begin,
+//           coords, bucket, cloud) and one lin -> cell map region per cloud.
 //   count:  query packing (a self search reuses the reference order) -> query groups (cells) ->
 //           work units of <= 32 queries of one group -> warp-per-unit candidate walk that tests
-//           every (query, candidate) pair once, counts, and stages per-unit hit records -> scan.
+//           every (query, candidate) pair once as tensor-core products, counts, and stages
+//           per-unit hit records -> exact decisions of the pairs near the threshold -> scan.
 //   emit:   expansion of the staged records into CSR/COO slots; units that were not staged are
 //           walked again.
 // The candidate set of every query is the reference's (cppSrc/neighborhood.h:73-132): the
@@ -1445,7 +1446,7 @@ __device__ __forceinline__ uint32_t chunk_hits(const WrapCtx& wc, const float4* 
 // N_q = |Q|^2 - (gather hq^2, symmetric hq^2 / 4), N_c = |C|^2 - (scatter hc^2, symmetric hc^2 / 4), and
 // the last term in symmetric mode (thr = (hq + hc) / 2).  Every factor is split into two float16
 // (hi + lo: 22 bits); hi*hi, hi*lo and lo*hi of the three coordinates and the supports and both
-// halves of both norms are 16 products: one mma.m16n8k16 tests 16 queries against 8 candidates, with
+// halves of both norms are 16 products: one mma.m16n8k16 tests 16 candidates against 8 queries, with
 // float32 accumulation.  What bounds the walk is issue slots: the float32x2 form took ~9 instructions a
 // lane and test, the product leaves 1.5 (collect the sign, keep the smallest magnitude), and its
 // accumulator layout hands each lane 4 candidates of two queries, so the hit masks need three

@@ -1,7 +1,8 @@
 // tcr_sort.cuh -- stable LSD radix sort of (key, int32 value) pairs, 32- or 64-bit keys.
 //
-// Per 8-bit digit: a tile histogram kernel, a per-digit scan of the tiles' counts and a stable
-// scatter.  Inside a tile the scatter ranks keys with warp match/ballot so equal digits
+// Per 8-bit digit: a tile histogram, a per-digit scan of the tiles' counts and a stable
+// scatter, as phases of one cooperative launch (sort_coop_kernel, the searches' sorts) or as
+// three launches (radix_sort_pairs, the scatter operators' sort).  Inside a tile the scatter ranks keys with warp match/ballot so equal digits
 // keep their input order; tiles are concatenated in order, so the whole sort is stable.  A pass
 // whose digit is the same for every key is skipped on the device without a host round trip:
 // digits above the highest bit in which two keys differ (from the key range the producer

@@ -123,7 +123,7 @@ class CompactHashMap:
 
     Carries the fields of the reference's ``CompactHashMap`` NamedTuple
     (compactHashing/datastructure.py:8-31).  The device buffer holds the B200 layout (points in
-    cell order as float4, a cell table and an open-addressing linear-index map); the
+    cell order as float4, a cell table and a map from linear index to cell); the
     reference-layout views (``hashTable`` [L,2], ``sortedCellTable`` [C,3], ``numCells``,
     ``hCell``, ...) are derived from it on first access.
     """
