@@ -1,7 +1,7 @@
 """Searches recorded once as CUDA graphs and replayed.
 
 A search (or a batch) whose sizes and buffers stay fixed -- the next timestep of a simulation,
-the next step of a training loop -- repeats the same ~40 kernel launches and their host work.
+the next step of a training loop -- repeats the same ~15 kernel launches and their host work.
 ``SearchPlan`` runs it once eagerly to size the staging list and the output, records the
 ``tcr_batch_build_structure`` / ``tcr_batch_count`` / ``tcr_batch_emit`` sequence into one CUDA
 graph, and from then on launches that graph: one launch and one synchronisation (to read the pair
