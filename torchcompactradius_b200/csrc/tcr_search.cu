@@ -1045,7 +1045,7 @@ constexpr float kMmaFar = 60000.0f;
 struct UnitCtx {
     int32_t cloud, dim, periodic_mask, dedupe;
     uint32_t hash_len;
-    int32_t error, out_of_grid, exact_all;
+    int32_t error, exact_all;
     int32_t count[3];
     int32_t qshift, rshift;  // subtracted from global query / reference indices (cloud-local numbering)
     float dmin[3], hcell[3], ext[3];
@@ -1073,7 +1073,7 @@ struct WalkArgs {
     int32_t local_index;          // 1: rows and columns numbered within each cloud
     int32_t mode;
     int32_t no_stray_check;       // self search, no periodic dims, same positions: a query's cell is its
-                                  // group's unless its cloud has points outside the grid (out_of_grid)
+                                  // group's where linear indices name one cell each (UnitCtx.plain_cells)
     int32_t class_filter;         // >= 0: walk only units of clouds of this class (dim * 2 + periodic)
     int32_t self;                 // self search: sorted query t is sorted reference t, wrapped once less
     const float4* __restrict__ rsorted;
@@ -1124,7 +1124,6 @@ __device__ __forceinline__ void load_unit_ctx(UnitCtx& u, const WalkArgs& a, int
     u.dedupe = cp.dedupe;
     u.hash_len = cp.hash_len;
     u.error = g.error;
-    u.out_of_grid = g.out_of_grid;
     u.exact_all = q.exact_all;
     for (int d = 0; d < 3; ++d) {
         u.count[d] = g.count[d];
@@ -1639,8 +1638,10 @@ __device__ __forceinline__ Unit open_unit(const WalkArgs& a, const UnitCtx& u, i
     n.active = false;
     if (qlane) {
         n.active = TCR_IN(n.qorig, a.nq_total);
-        bool check = !a.no_stray_check || u.out_of_grid;
-        if (check && a.self && !u.out_of_grid) {
+        // (equal positions, and equal cells of the sorted point and its group, are not enough where linear
+        // indices wrap: two cells of the grid can then share one key, one run and one group)
+        bool check = !a.no_stray_check || !u.plain_cells;
+        if (check && a.self && u.plain_cells) {
             // the group's cell is the reference's; where the second wrap changed nothing it is the query's
             // too (three compares instead of three divisions)
             const float4 r = __ldg(&a.rsorted[t0 + lane]);
