@@ -1135,11 +1135,17 @@ __device__ __forceinline__ void load_unit_ctx(UnitCtx& u, const WalkArgs& a, int
     u.rshift = a.local_index ? cp.ref_base : 0;
     u.rmax = key_float(g.ref_stats.max_key);
     u.qmax = q.qmax;
-    // Points of a stencil cell across the periodic seam can be moved by +-ext while staged, so
-    // the fast test needs no wrap: with >= 5 cells on every periodic dimension no candidate of the stencil
-    // (at most two cells away) is near half the extent away, so the reference's moduloOp wraps exactly
-    // the shifted cells; with 4 cells the two differ only for candidates at least 2 cells away, beyond
-    // every threshold when those stay below 1.5 cells.  A shift
+    // a float32 copy of a double coordinate x is off by <= |x| 2^-24, the float difference adds one
+    // rounding: 2^-21 of the largest |coordinate| bounds a difference's error with room to spare
+    u.f64_err = a.f64.qpos ? key_float(q.coord_key) * 4.76837158203125e-7f : 0.0f;
+    // Candidates of a stencil cell across the periodic seam can be moved by +-ext, so that the fast test
+    // needs no wrap, where the reference's moduloOp wraps exactly the moved cells.  Two points of a
+    // stencil are less than 2 cells apart.  With five cells or more on a dimension that is at most half the
+    // extent (the last cell may be a sliver: ext > 4 cells), so only moved candidates wrap.  With four
+    // cells (3 cells < ext <= 4 cells) a difference D between ext / 2 and 2 cells wraps too, to
+    // ext - D >= ext - 2 cells: beyond every threshold, and so is D, when thresholds end at ext - 2 cells
+    // (less what rounding a coordinate to its cell can add).  A moved candidate is at most 2 cells away
+    // with five cells, ext - 2 cells with four: ext / 2 at most.  A shift
     // changes a difference by at most one rounding of the shifted coordinate plus the reference's
     // own rounding of q - c before its exact wrap: shift_delta bounds both.
     bool ok = cp.periodic_mask != 0;
@@ -1147,17 +1153,16 @@ __device__ __forceinline__ void load_unit_ctx(UnitCtx& u, const WalkArgs& a, int
     const float tmax = fmaxf(a.mode == kScatter ? 0.0f : u.qmax, a.mode == kGather ? 0.0f : u.rmax);
     for (int d = 0; d < cp.dim; ++d)
         if ((cp.periodic_mask >> d) & 1) {
-            ok = ok && (g.count[d] >= 5 || (g.count[d] == 4 && tmax <= 1.5f * g.hcell_d[d]));
             // two roundings of magnitude <= half an ulp of (|coordinate| + ext) each: <= 2^-23 of it
-            delta = fmaxf(delta, (fmaxf(fabsf(cp.dmin[d]), fabsf(cp.dmax[d])) + cp.ext[d]) * 1.1920928955078125e-7f);
+            const float one = (fmaxf(fabsf(cp.dmin[d]), fabsf(cp.dmax[d])) + cp.ext[d]) * 1.1920928955078125e-7f;
+            const float room = fmaf(-2.0f, g.hcell_d[d], cp.ext[d]) - fmaf(4.0f, one, 2.0f * u.f64_err);
+            ok = ok && (g.count[d] >= 5 || (g.count[d] == 4 && tmax <= room));
+            delta = fmaxf(delta, one);
         }
     u.shift_ok = ok && isfinite(delta);
     u.shift_delta = delta;
     u.map_base = cp.map_base;
     u.map_cap = cp.map_cap;
-    // a float32 copy of a double coordinate x is off by <= |x| 2^-24, the float difference adds one
-    // rounding: 2^-21 of the largest |coordinate| bounds a difference's error with room to spare
-    u.f64_err = a.f64.qpos ? key_float(q.coord_key) * 4.76837158203125e-7f : 0.0f;
     u.plain_cells = direct_cells(cp.dim, g.count, g.out_of_grid, int64_t(1) << 31) != 0;
     u.map_direct = direct_cells(cp.dim, g.count, g.out_of_grid, cp.map_cap);
     float cell = 0.0f;
