@@ -133,6 +133,7 @@ struct Scratch {
     int32_t* num_flagged;   // [1]
     int32_t* exact_clouds;  // [1] clouds whose every pair takes the exact test
     int32_t* num_exact;     // [1] pairs inside the count walk's band, decided exactly
+    int32_t* pack_done;     // [1] blocks of the self queries' packing that finished
     int32_t* unit_cap;      // [1] queries per work unit of this search (set by the count phase)
     unsigned long long* cursor;  // [2] staging fill, staging capacity
     float4* pack;           // [max(nq,nr)] packed input points before sorting
@@ -180,7 +181,8 @@ static Scratch carve_scratch(void* buf, int64_t nq, int64_t nr, int64_t C, bool 
     s.info = c.take<int64_t>(8);
     s.num_flagged = c.take<int32_t>(1);
     s.exact_clouds = c.take<int32_t>(1);
-    s.num_exact = c.take<int32_t>(1);
+    s.num_exact = c.take<int32_t>(2);
+    s.pack_done = s.num_exact ? s.num_exact + 1 : nullptr;
     s.unit_cap = c.take<int32_t>(1);
     s.cursor = c.take<unsigned long long>(2);
     s.pack = c.take<float4>(nmax);
@@ -322,6 +324,35 @@ __device__ __forceinline__ void stats_atomic(SupportStats* s, uint32_t kmax, int
     if (bad) atomicOr(&s->bad, 1);
 }
 
+__device__ __forceinline__ void support_stat(float v, uint32_t& kmax, int& bad) {
+    kmax = max(kmax, float_key(v));
+    bad |= !(v >= 1e-18f && v <= 1e18f);
+}
+// The threads' statistics of the cloud each ended in (-1: it had no point): one atomic per block and field
+// where the block stayed in one cloud.
+__device__ __forceinline__ void block_stats(int cur, uint32_t kmax, int bad, char* out, int64_t stride) {
+    __shared__ int s_cloud;
+    if (threadIdx.x == 0) s_cloud = cur;  // thread 0 holds the block's first point, if it has any
+    __syncthreads();
+    if (__syncthreads_and(cur < 0 || cur == s_cloud)) {
+        if (s_cloud >= 0) block_reduce_stats(kmax, bad, stats_at(out, stride, s_cloud));
+    } else if (cur >= 0) {
+        stats_atomic(stats_at(out, stride, cur), kmax, bad);
+    }
+}
+// Whether this block is the last of its launch to get here; the others' writes before are visible then.
+__device__ __forceinline__ bool last_block(int32_t* done) {
+    __shared__ int s_last;
+    __threadfence();  // this thread's atomics before the block's arrival
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last != 0;
+}
+
 // Per cloud: util.py:28-79 compute_h and cellTable.py:27-29, float32 throughout.
 // same_sup: the query supports are the reference support array (statistics reduced once).
 __device__ __forceinline__ void grid_params(const CloudParams* __restrict__ table, GridParams* grid, int C,
@@ -431,30 +462,10 @@ __global__ void support_stats_kernel(const CloudParams* __restrict__ table, cons
             kmax = 0;
             bad = 0;
         }
-        if (h) {
-            const float v = h[i - cbase];
-            kmax = max(kmax, float_key(v));
-            bad |= !(v >= 1e-18f && v <= 1e18f);
-        }
+        if (h) support_stat(h[i - cbase], kmax, bad);
     }
-    __shared__ int s_cloud;
-    if (threadIdx.x == 0) s_cloud = cur;  // thread 0 holds the block's first point, if it has any
-    __syncthreads();
-    if (__syncthreads_and(cur < 0 || cur == s_cloud)) {
-        if (s_cloud >= 0) block_reduce_stats(kmax, bad, stats_at(out, stride, s_cloud));
-    } else if (cur >= 0) {
-        stats_atomic(stats_at(out, stride, cur), kmax, bad);
-    }
-    if (!done) return;
-    __shared__ int s_last;
-    __threadfence();  // this thread's atomics before the block's arrival
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
-        __threadfence();
-    }
-    __syncthreads();
-    if (s_last) grid_params(table, grid, C, bad_grids, same_sup, threadIdx.x, blockDim.x);
+    block_stats(cur, kmax, bad, out, stride);
+    if (done && last_block(done)) grid_params(table, grid, C, bad_grids, same_sup, threadIdx.x, blockDim.x);
 }
 
 // Start of a build: the (last clouds of the) table, per-cloud statistics and flags, counters, the sort
@@ -512,7 +523,7 @@ __global__ void query_params_kernel(const CloudParams* __restrict__ table, const
 
 // Start of a count: the (last clouds of the) table; zeroes the per-search counters, the per-cloud query
 // statistics and the per-query counts; with ready also writes the clouds' query parameters (1: the
-// queries' supports are the references', 2: there are none to reduce).
+// queries are the structure's sorted points, 2: there are no supports to reduce).
 __global__ void count_init_kernel(const __grid_constant__ CloudChunk<kUploadChunk> ch, const GridParams* grid, Scratch W,
                                   int C, int unit_cap, int64_t nq, int64_t stage_cap, int ready) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x)
@@ -531,6 +542,7 @@ __global__ void count_init_kernel(const __grid_constant__ CloudChunk<kUploadChun
         *W.num_flagged = 0;
         *W.exact_clouds = 0;
         *W.num_exact = 0;
+        *W.pack_done = 0;
         *W.unit_cap = unit_cap;
         W.cursor[0] = 0ull;
         W.cursor[1] = (unsigned long long)stage_cap;
@@ -923,22 +935,40 @@ __global__ void inc_merge_kernel(const K* __restrict__ stay_keys, const int32_t*
 // query side
 
 // Self search: query i is reference i, so the reference order and cells group the queries.
-// Positions are the once-wrapped query coordinates (only periodic dims differ from rsorted).
+// Positions are the once-wrapped query coordinates (only periodic dims differ from rsorted), supports the
+// caller's of this call: a kept structure may be searched with others than it was built from.  Their
+// statistics are reduced on the way, as support_stats_kernel does, and the last block to finish writes the clouds'
+// query parameters.
 __global__ void pack_self_queries_kernel(const CloudParams* __restrict__ table, const GridParams* grid,
                                          const int32_t* __restrict__ prefix, int C, const int32_t* __restrict__ rsidx,
-                                         int64_t n, float4* __restrict__ qsorted, int32_t* __restrict__ qsidx) {
+                                         int64_t n, float4* __restrict__ qsorted, int32_t* __restrict__ qsidx,
+                                         QueryParams* qp, int32_t* exact_clouds, int32_t* done) {
     const int64_t per = (n + gridDim.x - 1) / gridDim.x;
     const int64_t lo = (int64_t)blockIdx.x * per;
     const int64_t hi = min(n, lo + per);
+    char* const out = reinterpret_cast<char*>(&qp->stats);
+    constexpr int64_t stride = (int64_t)sizeof(QueryParams);
     PointCtx p;
     p.cloud = -1;
     p.base = p.end = 0;
+    uint32_t kmax = 0;
+    int bad = 0;
     for (int64_t t = lo + threadIdx.x; t < hi; t += blockDim.x) {
         const int32_t i = rsidx[t];
-        if (p.cloud < 0 || i < p.base || i >= p.end) load_point_ctx(p, table, grid, prefix, cloud_of(prefix, C, i), true);
-        qsorted[t] = wrap_point(p.dim, p.periodic_mask, p.dmin, p.ext, load_point(p.pos, p.sup, i - p.base, p.dim), 1);
+        if (p.cloud < 0 || i < p.base || i >= p.end) {
+            if (p.cloud >= 0) stats_atomic(stats_at(out, stride, p.cloud), kmax, bad);
+            load_point_ctx(p, table, grid, prefix, cloud_of(prefix, C, i), true);
+            kmax = 0;
+            bad = 0;
+        }
+        const float4 v = load_point(p.pos, p.sup, i - p.base, p.dim);
+        if (p.sup) support_stat(v.w, kmax, bad);
+        qsorted[t] = wrap_point(p.dim, p.periodic_mask, p.dmin, p.ext, v, 1);
         qsidx[t] = i;
     }
+    block_stats(p.cloud, kmax, bad, out, stride);
+    if (last_block(done))
+        for (int c = threadIdx.x; c < C; c += blockDim.x) query_params(table[c], grid[c], qp[c], exact_clouds, 0);
 }
 
 // Group count comes from a device scalar; the scan kernels are launched over the upper bound
@@ -3202,9 +3232,12 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
     int rc = upload_table(b, W, st, chunk);
     if (rc) return rc;
     const int unit_cap = b.unit_cap;
-    const bool query_stats = b.any_query_sup && nq > 0 && !b.same_supports;
-    count_init_kernel<<<grid_for(std::max<int64_t>(C, nq), 256), 256, 0, st>>>(chunk, S.grid, W, C, unit_cap, nq, stage_cap,
-                                                                               query_stats ? 0 : (b.same_supports ? 1 : 2));
+    // Query parameters: from the structure's statistics where the queries are its sorted points
+    // themselves (same_sorted), with the packing of other self searches, else by launches of their own.
+    const bool packed = b.self && !b.same_sorted && nq > 0;
+    const bool query_stats = b.any_query_sup && nq > 0 && !b.self;
+    count_init_kernel<<<grid_for(std::max<int64_t>(C, nq), 256), 256, 0, st>>>(
+        chunk, S.grid, W, C, unit_cap, nq, stage_cap, packed || query_stats ? 0 : (b.same_sorted ? 1 : 2));
     note_launches(1);
     if (query_stats) {
         support_stats_kernel<<<grid_for(nq, 256, num_sms() * 4), 256, 0, st>>>(
@@ -3222,9 +3255,10 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
         const int32_t* gstart;
         const int32_t* ngroups;
         if (b.self) {
-            if (!b.same_sorted) {
-                pack_self_queries_kernel<<<grid_for(nq, 256), 256, 0, st>>>(W.table, S.grid, W.query_prefix, C, S.rsidx,
-                                                                            nq, W.qsorted, W.qsidx);
+            if (packed) {
+                pack_self_queries_kernel<<<grid_for(nq, 256, num_sms() * 8), 256, 0, st>>>(
+                    W.table, S.grid, W.query_prefix, C, S.rsidx, nq, W.qsorted, W.qsidx, W.qparams, W.exact_clouds,
+                    W.pack_done);
                 note_launches(1);
             }
             gstart = S.cell_start;
