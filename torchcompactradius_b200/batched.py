@@ -360,11 +360,11 @@ def radiusSearchBatch(queryPointClouds: Sequence[PointCloud],
 SORTED_ID_SPAN = 1 << 16
 
 
-def _one_each(x, batch, support):
-    """One batch id (and, where there is a tensor of them, one support) per point."""
+def _one_each(x, batch, support=None):
+    """One batch id and, where supports are given, one support per point (None: none are given)."""
     n = x.shape[0]
-    return batch.dim() == 1 and batch.shape[0] == n and not (
-        torch.is_tensor(support) and support.dim() > 0 and support.shape[0] != n)
+    return batch.dim() == 1 and batch.shape[0] == n and (
+        support is None or (torch.is_tensor(support) and support.dim() > 0 and support.shape[0] == n))
 
 
 def _sorted_counts(bx, by, same_cloud):
@@ -404,9 +404,11 @@ def radius_batched(xq, xr, support, batch_x, batch_y, mode="gather", domain=None
         batch_y = batch_x if same_cloud else torch.zeros(xr.shape[0], dtype=torch.long, device=xr.device)
     bx = batch_x.to(device=device, dtype=torch.long)
     by = bx if same_cloud else batch_y.to(device=device, dtype=torch.long)
+    pair = isinstance(support, (tuple, list))
+    sq = support[0] if pair else (support if torch.is_tensor(support) and support.dim() > 0 else None)
+    sr = support[1] if pair else None
     counts = None
-    if _one_each(xq, bx, support[0] if isinstance(support, (tuple, list)) else support) and (
-            same_cloud or _one_each(xr, by, support[1] if isinstance(support, (tuple, list)) else None)):
+    if _one_each(xq, bx, sq) and _one_each(xq if same_cloud else xr, by, sr):
         counts = _sorted_counts(bx, by, same_cloud)
     if counts is not None:  # clouds are consecutive already: no order to find, no points to move
         oq = orr = None
@@ -427,15 +429,19 @@ def radius_batched(xq, xr, support, batch_x, batch_y, mode="gather", domain=None
 
     def ordered(t, order):
         t = _as_f32(t, device)
-        return t if order is None else t.index_select(0, order).contiguous()
+        if order is None:
+            return t
+        if (t.shape[0] if t.dim() else 1) < order.shape[0]:
+            raise ValueError(f"{t.shape[0] if t.dim() else 1} positions or supports for {order.shape[0]} batch ids")
+        return t.index_select(0, order).contiguous()
 
     xs = ordered(xq, oq)
     ys = xs if same_cloud else ordered(xr, orr)
-    if isinstance(support, (tuple, list)):
-        hq = ordered(support[0], oq)
-        hr = ordered(support[1], orr)
-    elif torch.is_tensor(support) and support.dim() > 0:
-        hq = ordered(support, oq)
+    if pair:
+        hq = ordered(sq, oq)
+        hr = ordered(sr, orr)
+    elif sq is not None:
+        hq = ordered(sq, oq)
         hr = hq if same_cloud else None
     else:
         hq = torch.full((xs.shape[0],), float(support), dtype=torch.float32, device=device)
