@@ -1,5 +1,5 @@
 """radius() with batch vectors: which calls take their points in place, and what calls with too few supports
-do."""
+or with batch ids at the end of int64 do."""
 import numpy as np
 import pytest
 import torch
@@ -29,6 +29,18 @@ def test_too_few_supports_are_refused(same, short):
                    scalar=(h, torch.tensor(0.1)))[short]
     with pytest.raises(ValueError):
         tcr.radius(x, None if same else x.clone(), support, batch, batch, mode="symmetric")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("last", [2 ** 62, 2 ** 63 - 3, 2 ** 63 - 2, 2 ** 63 - 1])
+def test_ids_at_the_end_of_int64(last):
+    import torchcompactradius_b200 as tcr
+    g = torch.Generator().manual_seed(1)
+    x = torch.rand(400, 3, generator=g).cuda()
+    low = torch.arange(2).repeat_interleave(200)
+    i, j = tcr.radius(x, None, 0.2, low.cuda())
+    a, b = tcr.radius(x, None, 0.2, (low + (last - 1)).cuda())
+    assert i.numel() > 400 and torch.equal(i, a) and torch.equal(j, b)
 
 
 @pytest.mark.gpu

@@ -378,7 +378,7 @@ def _sorted_counts(bx, by, same_cloud):
     parts = tuple(t.contiguous() for t in parts)
     stats = [index_stats(t) for t in parts]
     lo, hi = min(s[0] for s in stats), max(s[1] for s in stats)
-    if any(s[2] for s in stats) or hi - lo >= SORTED_ID_SPAN:
+    if any(s[2] for s in stats) or hi - lo >= SORTED_ID_SPAN or hi + 2 > torch.iinfo(torch.int64).max:
         return None
     edges = torch.arange(lo, hi + 2, device=bx.device)
     at = torch.stack([torch.searchsorted(t, edges) for t in parts]).cpu().numpy()
