@@ -27,6 +27,7 @@
 
 #include "tcr_common.cuh"
 #include "tcr_scan.cuh"
+#include "tcr_fold_span.cuh"
 #include "tcr_sort.cuh"
 #include "../../include/tcr_b200.h"
 
@@ -613,8 +614,7 @@ __global__ void __launch_bounds__(kFoldWarps * 32) fold_rows_kernel(FoldArgs a) 
             for (int j = i + lane; j < len; j += 32) tile[j] = s[t0 + j];
             asm volatile("cp.async.wait_all;\n" ::: "memory");
             __syncwarp();
-            const int j0 = (int)((lo > t0 ? lo : t0) - t0 < len ? (lo > t0 ? lo : t0) - t0 : len);
-            const int j1 = (int)((hi < t0 + len ? hi : t0 + len) - t0);
+            const int j0 = tile_offset(lo, t0, len), j1 = tile_offset(hi, t0, len);
             int j = j0;
             for (; j + 4 <= j1; j += 4) {  // four reads in flight, folded in order
                 const T v0 = tile[j], v1 = tile[j + 1], v2 = tile[j + 2], v3 = tile[j + 3];
