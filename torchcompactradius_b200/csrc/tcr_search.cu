@@ -343,9 +343,9 @@ __device__ __forceinline__ void block_stats(int cur, uint32_t kmax, int bad, cha
 // Whether this block is the last of its launch to get here; the others' writes before are visible then.
 __device__ __forceinline__ bool last_block(int32_t* done) {
     __shared__ int s_last;
-    __threadfence();  // this thread's atomics before the block's arrival
     __syncthreads();
     if (threadIdx.x == 0) {
+        __threadfence();  // (cumulative: the block's atomics before its arrival)
         s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
         __threadfence();
     }
