@@ -2494,7 +2494,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32, 4) expand_records_kernel(co
 #pragma unroll 4
                 for (int32_t o = lane; o < n; o += 32) {
                     const uint32_t v = tab[o], q = ((v >> 5) * inc) >> 16;
-                    __stcs(sm.qcol[w][q] + o, (long long)(uint32_t)cols[v - q * per]);
+                    __stcs(sm.qcol[w][q] + o, (long long)cols[v - q * per]);
                 }
             } else if (fits) {  // COO: the row of an output sits at the same slot of row_out
                 const int64_t rd = ((intptr_t)a.row_out - (intptr_t)a.col_out) / 8;  // both int64-aligned
@@ -2502,7 +2502,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32, 4) expand_records_kernel(co
                 for (int32_t o = lane; o < n; o += 32) {
                     const uint32_t v = tab[o], q = ((v >> 5) * inc) >> 16;
                     long long* p = sm.qcol[w][q] + o;
-                    __stcs(p, (long long)(uint32_t)cols[v - q * per]);
+                    __stcs(p, (long long)cols[v - q * per]);
                     __stcs(p + rd, (long long)sm.qrow[w][q]);
                 }
             } else {
@@ -2510,7 +2510,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32, 4) expand_records_kernel(co
                     const uint32_t v = tab[o], q = ((v >> 5) * inc) >> 16;
                     const int64_t pos = (sm.qcol[w][q] - reinterpret_cast<long long*>(a.col_out)) + o;
                     if (TCR_GUARD(pos, a.out_cap)) {
-                        __stcs(reinterpret_cast<long long*>(&a.col_out[pos]), (long long)(uint32_t)cols[v - q * per]);
+                        __stcs(reinterpret_cast<long long*>(&a.col_out[pos]), (long long)cols[v - q * per]);
                         if (a.row_out) __stcs(reinterpret_cast<long long*>(&a.row_out[pos]), (long long)sm.qrow[w][q]);
                     }
                 }
