@@ -554,10 +554,16 @@ inline cudaError_t sort_coop(const SortWorkspaceT<K>& w, int64_t n, int32_t* fai
     int32_t *v0 = w.vals[0], *v1 = w.vals[1], *hist = w.hist;
     SortStateT<K>* state = w.state;
     void* args[] = {&k0, &k1, &v0, &v1, &n, &state, &hist, &failed, &tail};
+    // One block per SM is resident on the whole device; a stream that is given fewer SMs (a partition of
+    // them) refuses that many.  Any number of blocks sorts, in longer ranges.
+    for (int blocks = coop_blocks(n, sms);; blocks = (blocks + 1) / 2) {
+        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(sort_coop_kernel<K, Tail>), dim3((unsigned)blocks),
+                                        dim3(kCoopThreads), args, sizeof(CoopSmem<K>), st);
+        if (e != cudaErrorCooperativeLaunchTooLarge || blocks == 1) break;
+        (void)cudaGetLastError();
+    }
     note_launches(1);
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(sort_coop_kernel<K, Tail>),
-                                       dim3((unsigned)coop_blocks(n, sms)), dim3(kCoopThreads), args,
-                                       sizeof(CoopSmem<K>), st);
+    return e;
 }
 
 }  // namespace tcr
