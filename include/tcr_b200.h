@@ -202,7 +202,11 @@ int tcr_build_structure(const tcr_search_desc* d, void* structure, int64_t struc
  * decided again by the exact test because they lay within the fast test's rounding band, and
  * for a batch built with a linear-cell hint the points its incremental re-sort sorted (-1: it fell
  * back to the full sort; -2: no hint)};
- * a caller sizes the next search's staging list from entry 4. */
+ * a caller sizes the next search's staging list from entry 4.
+ * Entry 1 is -1 when a sort on the device gave up waiting for its own blocks (each wait is bounded; about a
+ * second and a half): the offsets are then all 0, and an emit enqueued behind the count writes nothing.  When it was
+ * the build's sort, the structure holds nothing and every count of it reports -1 until it is built again; when
+ * it was the queries' sort, the structure is as good as before. */
 int tcr_count(const tcr_search_desc* d, const void* structure, void* scratch, int64_t scratch_bytes, int32_t* stage,
               int64_t stage_capacity, int64_t* offsets, int32_t* indptr_out, int64_t* row_entries_out,
               int64_t* info_out, void* stream);

@@ -85,7 +85,7 @@ struct Carve {
 // Persistent structure (reference side); kept alive for reuse.
 struct Structure {
     GridParams* grid;         // [C] per cloud
-    int32_t* num_cells;       // [3] cells; set when a one-launch sort gave up waiting; blocks of the statistics that finished
+    int32_t* num_cells;       // [3] cells; set when the build's sort gave up waiting; blocks of the statistics that finished
     int32_t* bad_grids;       // [1] clouds with points on both sides and no valid grid
     float4* rsorted;          // [nr] wrapped reference points in (cloud, cell) order, .w = support
     int32_t* rsidx;           // [nr] global index of each sorted point
@@ -124,7 +124,7 @@ struct Scratch {
     int32_t* ref_prefix;    // [C+1] the same for reference points
     QueryParams* qparams;   // [C]
     void* sort_state;       // SortState32 or SortState64
-    int32_t* num_qgroups;   // [1]
+    int32_t* num_qgroups;   // [2] query groups; set when this search's query sort gave up waiting
     int32_t* num_units;     // [1]
     int32_t* num_stray;     // [1]
     int32_t* work;          // [kWorkCounters] work distribution counters
@@ -173,7 +173,7 @@ static Scratch carve_scratch(void* buf, int64_t nq, int64_t nr, int64_t C, bool 
     s.ref_prefix = c.take<int32_t>(C + 1);
     s.qparams = c.take<QueryParams>(C);
     s.sort_state = c.take<SortState64>(1);
-    s.num_qgroups = c.take<int32_t>(1);
+    s.num_qgroups = c.take<int32_t>(2);
     s.num_units = c.take<int32_t>(1);
     s.num_stray = c.take<int32_t>(1);
     s.work = c.take<int32_t>(kWorkCounters);
@@ -537,6 +537,7 @@ __global__ void count_init_kernel(const __grid_constant__ CloudChunk<kUploadChun
     }
     if (threadIdx.x == 0) {
         for (int k = 0; k < kWorkCounters; ++k) W.work[k] = 0;
+        W.num_qgroups[0] = W.num_qgroups[1] = 0;
         *W.num_stray = 0;
         *W.num_units = 0;
         *W.num_flagged = 0;
@@ -796,7 +797,18 @@ struct BuildTail {
     }
 };
 
-// The same for queries sorted by their own cells: one query group per run.
+// The order and cells a caller of the incremental build receives when the sort gave up: the order it came
+// in, and its hint.
+__global__ void abandoned_order_kernel(const int32_t* __restrict__ failed, int64_t n, const int32_t* __restrict__ hint,
+                                       int32_t* lin_out, int32_t* order_out) {
+    if (!*failed) return;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        if (lin_out) lin_out[i] = hint ? hint[i] : 0;
+        if (order_out) order_out[i] = (int32_t)i;
+    }
+}
+
+// What BuildTail does, for queries sorted by their own cells: one query group per run.
 template <typename K>
 struct QueryTail {
     static constexpr bool kPlace = true, kRuns = true;
@@ -955,6 +967,7 @@ __global__ void pack_self_queries_kernel(const CloudParams* __restrict__ table, 
     int bad = 0;
     for (int64_t t = lo + threadIdx.x; t < hi; t += blockDim.x) {
         const int32_t i = rsidx[t];
+        if (!TCR_GUARD(i, n)) continue;  // (the build's sort gave up)
         if (p.cloud < 0 || i < p.base || i >= p.end) {
             if (p.cloud >= 0) stats_atomic(stats_at(out, stride, p.cloud), kmax, bad);
             load_point_ctx(p, table, grid, prefix, cloud_of(prefix, C, i), true);
@@ -973,28 +986,32 @@ __global__ void pack_self_queries_kernel(const CloudParams* __restrict__ table, 
 
 // Group count comes from a device scalar; the scan kernels are launched over the upper bound
 // and read the true count through the functor.  A unit holds at most `cap` (<= 32) queries.
+// After a sort that gave up there are no groups and so no units: nothing is walked, counted or emitted.
 struct BoundedUnitCountIn {
     const int32_t* group_start;
     const int32_t* num_groups;
     int32_t cap;
+    const int32_t* build_failed;
+    const int32_t* sort_failed;
     __device__ int32_t operator()(int64_t g) const {
-        if (g >= *num_groups) return 0;
-        int32_t n = group_start[g + 1] - group_start[g];
+        // (read-only loads, so that a thread's elements share them and none waits for another)
+        const int32_t groups = __ldg(num_groups), failed = __ldg(build_failed) | __ldg(sort_failed);
+        if (failed != 0 || g >= groups) return 0;
+        const int32_t n = __ldg(&group_start[g + 1]) - __ldg(&group_start[g]);
         return (n + cap - 1) / cap;
     }
 };
 struct BoundedUnitOut {
     const int32_t* group_start;
-    const int32_t* num_groups;
     int32_t* unit_group;
     int32_t* unit_t0;
     int32_t cap;
-    int64_t bound = 1ll << 62;  // entries of unit_group / unit_t0 (checked build)
+    int64_t bound;  // entries of unit_group / unit_t0
     __device__ void operator()(int64_t g, int32_t ex, int32_t nunits) const {
-        if (g >= *num_groups) return;
+        if (nunits <= 0) return;
         const int32_t s = group_start[g];
         for (int32_t u = 0; u < nunits; ++u) {
-            if (!TCR_IN(ex + u, bound)) break;
+            if (!TCR_GUARD(ex + u, bound)) break;
             unit_group[ex + u] = (int32_t)g;
             unit_t0[ex + u] = s + u * cap;
         }
@@ -2640,6 +2657,7 @@ __global__ void f64_prep_kernel(const int32_t* __restrict__ rsidx, F64Args f, in
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < f.nr; j += stride) {
         const int64_t jl = rsidx[j];
+        if (!TCR_GUARD(jl, f.nr)) continue;  // (the build's sort gave up)
         double4 v = make_double4(0.0, 0.0, 0.0, f.rsup ? f.rsup[jl] : 0.0);
         v.x = f.rpos[jl * dim];
         if (dim > 1) v.y = f.rpos[jl * dim + 1];
@@ -2752,7 +2770,8 @@ struct OffsetOut {
     int64_t* entries;
     // the search's info block, written with the total (element n)
     const int32_t* bad_grids;
-    const int32_t* num_cells;
+    const int32_t* build_failed;
+    const int32_t* sort_failed;
     const int32_t* num_stray;
     const int32_t* exact_clouds;
     const unsigned long long* cursor;
@@ -2769,7 +2788,7 @@ struct OffsetOut {
             return;
         }
         info[0] = ex;
-        info[1] = num_cells[1] ? -1 : *bad_grids;  // -1: a wait inside the sort gave up, nothing here is valid
+        info[1] = *build_failed || *sort_failed ? -1 : *bad_grids;  // -1: a sort gave up waiting, nothing was searched
         info[2] = *num_stray;
         info[3] = *exact_clouds;
         info[4] = (int64_t)*cursor;
@@ -3214,6 +3233,11 @@ static int build_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
                                            W.table, S.grid, S.cell_lin, S.cell_coords, S.cell_bucket, S.cell_cloud,
                                            S.map, nr},
                               st));
+        if (b.lin_out || b.order_out) {
+            abandoned_order_kernel<<<grid_for(nr, 256, num_sms()), 256, 0, st>>>(S.num_cells + 1, nr, b.lin_hint,
+                                                                               b.lin_out, b.order_out);
+            note_launches(1);
+        }
     } else {
         finish_cells_kernel<<<1, 1, 0, st>>>(S.cell_start, S.num_cells, nr);
         note_launches(1);
@@ -3271,15 +3295,15 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
             pack_points_kernel<K><<<grid_for(nq, 256, num_sms() * 4), 256, 0, st>>>(
                 W.table, S.grid, W.query_prefix, C, nq, 1, 1, 0, W.pack, sw.keys[0], sw.vals[0], sw.state);
             note_launches(1);
-            TCR_CUDA(sort_coop<K>(sw, nq, S.num_cells + 1,
+            TCR_CUDA(sort_coop<K>(sw, nq, W.num_qgroups + 1,
                                   QueryTail<K>{W.qgroup_start, W.num_qgroups, W.pack, W.qsorted, W.qsidx, W.table,
                                                S.grid, W.qgroup_coords, W.qgroup_cloud, nq},
                                   st));
             gstart = W.qgroup_start;
             ngroups = W.num_qgroups;
         }
-        BoundedUnitCountIn ui{gstart, ngroups, unit_cap};
-        BoundedUnitOut uo{gstart, ngroups, W.unit_group, W.unit_t0, unit_cap, nq};
+        BoundedUnitCountIn ui{gstart, ngroups, unit_cap, S.num_cells + 1, W.num_qgroups + 1};
+        BoundedUnitOut uo{gstart, W.unit_group, W.unit_t0, unit_cap, nq};
         TCR_CUDA(device_exclusive_scan<int32_t>(ui, uo, nq, W.scan_tiles32, W.num_units, st));
         WalkArgs a = make_walk(b, S, W);
         if (f64) a.f64 = f64_walk(*f64);
@@ -3292,7 +3316,7 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
         note_launches(1);
     }
     CountIn ci{W.counts, nq};
-    OffsetOut oo{nq, offsets, indptr_out, row_entries_out, S.bad_grids, S.num_cells, W.num_stray, W.exact_clouds, W.cursor,
+    OffsetOut oo{nq, offsets, indptr_out, row_entries_out, S.bad_grids, S.num_cells + 1, W.num_qgroups + 1, W.num_stray, W.exact_clouds, W.cursor,
                  W.num_flagged, W.num_exact, b.lin_hint && b.nr > 0 ? W.inc_count : nullptr, b.nr, W.info};
     TCR_CUDA(device_exclusive_scan<int64_t>(ci, oo, nq + 1, W.scan_tiles64, W.total, st));
     if (info_out) TCR_CUDA(cudaMemcpyAsync(info_out, W.info, 8 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -3706,6 +3730,7 @@ extern "C" int tcr_search_noalloc(const tcr_search_desc* d, int64_t* offsets, in
     if (rc) return rc;
     TCR_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     if (total_out) *total_out = info[0];
+    if (info[1] < 0) return set_error(TCR_ERR_CUDA, "tcr_search_noalloc: a sort on the device gave up waiting; nothing was searched");
     if (info[1]) return set_error(TCR_ERR_INVALID, "no valid cell grid for this domain and support");
     if (info[0] > pair_capacity)
         return set_error(TCR_ERR_INVALID, "tcr_search_noalloc: %lld pairs do not fit the %lld-entry output",

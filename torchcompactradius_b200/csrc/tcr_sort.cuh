@@ -280,7 +280,9 @@ inline cudaError_t radix_sort_pairs(const SortWorkspaceT<K>& w, int64_t n, cudaS
 // everything after the sort (placement, run-start scan, run records) four launches more.
 //
 // One block of 32 warps per SM: a launch is cooperative, so all blocks are resident, and each wait on
-// the barrier is bounded: a block that gives up sets *failed and returns (the host reports it).
+// the barrier is bounded: a block that gives up sets *failed and returns, and the others follow at their
+// next wait.  What the sort should have written is then there in part: the kernels behind it check every index
+// that they take from it, make no work units where the flag is set, and the host reports it.
 constexpr int kCoopThreads = 1024;
 constexpr int kCoopWarps = kCoopThreads / 32;
 constexpr int kCoopRounds = 8;
@@ -342,6 +344,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     CoopSmem<K>& sm = *reinterpret_cast<CoopSmem<K>*>(coop_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, b = blockIdx.x;
+    const int32_t gone = *(volatile int32_t*)failed;  // a sort before this one gave up: its pairs are not there
     const int64_t n = (st->n_dev >= 0 && st->n_dev < n_all) ? st->n_dev : n_all;
     const int64_t per = ((n + G - 1) / G + 31) & ~int64_t(31);
     const int64_t lo = min(n, per * b), hi = min(n, lo + per);
@@ -352,6 +355,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     const int top = differ == 0 ? -1 : top_bit(differ);  // the highest bit in which two keys differ
     unsigned phase = 0;
     int sel = st->sel[0];
+    if (gone) return;  // (here, so that the loads above are in flight together)
     bool placed = false;
     for (int pass = 0; pass < key_passes<K>(); ++pass) {
         const int shift = 8 * pass;

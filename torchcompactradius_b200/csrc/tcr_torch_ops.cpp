@@ -115,6 +115,10 @@ Tensor bytes_on(const Tensor& like, int64_t n) {
     return at::empty({std::max<int64_t>(n, 1)}, like.options().dtype(at::kByte));
 }
 
+void check_device(const int64_t* info) {
+    TORCH_CHECK(info[1] >= 0, "a device-wide sort of the search did not complete (a bounded wait gave up); nothing was searched");
+}
+
 // Count phase: offsets [nq+1], optional indptr/rowEntries; returns the info block (host).
 std::vector<int64_t> count_phase(const Search& s, const Tensor& structure, const Tensor& scratch, const Tensor& stage,
                                  const Tensor& offsets, int32_t* indptr, int64_t* rowEntries, cudaStream_t st) {
@@ -125,6 +129,7 @@ std::vector<int64_t> count_phase(const Search& s, const Tensor& structure, const
              "tcr_count");
     C10_CUDA_CHECK(cudaStreamSynchronize(st));
     std::vector<int64_t> out(info.data_ptr<int64_t>(), info.data_ptr<int64_t>() + 8);
+    check_device(out.data());
     TORCH_CHECK(out[1] == 0, out[1], " cloud(s) have no valid cell grid for their domain and support (the support "
                 "is not smaller than the domain extent, or a support/domain value is not finite)");
     return out;
@@ -308,6 +313,7 @@ std::tuple<Tensor, Tensor, Tensor> radiusSearchBatched(Tensor queryPositions, st
                              st),
              "tcr_batch_count");
     C10_CUDA_CHECK(cudaStreamSynchronize(st));
+    check_device(info.data_ptr<int64_t>());
     TORCH_CHECK(info.data_ptr<int64_t>()[1] == 0, "a cloud has no valid cell grid for its domain and support");
     const int64_t total = info.data_ptr<int64_t>()[0];
     Tensor row = at::empty({total}, all.xq.options().dtype(at::kLong));
