@@ -49,7 +49,8 @@ static int sort_on(void* keys0, void* keys1, int32_t* vals0, int32_t* vals1, int
     if (e != cudaSuccess) return (int)e;
     K *k0 = (K*)keys0, *k1 = (K*)keys1;
     PlainTail<K> tail{starts, num_runs, placed, (K*)run_key};
-    void* args[] = {&k0, &k1, &vals0, &vals1, &n, &state, &hist, &failed, &tail};
+    int chained = 1;
+    void* args[] = {&k0, &k1, &vals0, &vals1, &n, &state, &hist, &failed, &chained, &tail};
     return (int)cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(sort_coop_kernel<K, PlainTail<K>>),
                                             dim3((unsigned)blocks), dim3(kCoopThreads), args, sizeof(CoopSmem<K>), st);
 }

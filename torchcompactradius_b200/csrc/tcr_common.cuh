@@ -116,11 +116,9 @@ struct GridParams {
     SupportStats build_query_stats;  // over the query supports seen at build time
 };
 
-// Per-search query-side parameters of the lean test (scratch).
+// Per-search query-side reductions (scratch).
 struct QueryParams {
     SupportStats stats;      // over this search's query supports
-    float qmax;              // largest query support (band of the fast test)
-    int32_t exact_all;       // decide every pair with the exact reference test
     uint32_t coord_key;      // float64 inputs: float_key of the largest |coordinate| of the double positions
     int32_t pad;
 };

@@ -133,7 +133,6 @@ struct Scratch {
     int32_t* num_flagged;   // [1]
     int32_t* exact_clouds;  // [1] clouds whose every pair takes the exact test
     int32_t* num_exact;     // [1] pairs inside the count walk's band, decided exactly
-    int32_t* pack_done;     // [1] blocks of the self queries' packing that finished
     int32_t* unit_cap;      // [1] queries per work unit of this search (set by the count phase)
     unsigned long long* cursor;  // [2] staging fill, staging capacity
     float4* pack;           // [max(nq,nr)] packed input points before sorting
@@ -181,8 +180,7 @@ static Scratch carve_scratch(void* buf, int64_t nq, int64_t nr, int64_t C, bool 
     s.info = c.take<int64_t>(8);
     s.num_flagged = c.take<int32_t>(1);
     s.exact_clouds = c.take<int32_t>(1);
-    s.num_exact = c.take<int32_t>(2);
-    s.pack_done = s.num_exact ? s.num_exact + 1 : nullptr;
+    s.num_exact = c.take<int32_t>(1);
     s.unit_cap = c.take<int32_t>(1);
     s.cursor = c.take<unsigned long long>(2);
     s.pack = c.take<float4>(nmax);
@@ -502,37 +500,27 @@ __global__ void finish_cells_kernel(int32_t* cell_start, const int32_t* num_cell
     cell_start[*num_cells] = (int32_t)n;
 }
 
-// One cloud's query-side parameters of the lean test.  same_sup: the queries' supports are the
-// references' array, whose statistics the build reduced already.
-__device__ __forceinline__ void query_params(const CloudParams& cp, const GridParams& g, QueryParams& q,
-                                             int32_t* exact_clouds, int same_sup) {
-    if (same_sup) q.stats = g.ref_stats;
-    const bool has_q = cp.query_sup != nullptr;
-    const float qmax = has_q ? key_float(q.stats.max_key) : 0.0f;
-    q.qmax = (cp.mode == kScatter) ? 0.0f : qmax;
-    const bool qbad = (cp.mode != kScatter) && has_q && q.stats.bad;
-    const bool rbad = (cp.mode != kGather) && g.ref_stats.bad;
-    q.exact_all = (qbad || rbad || !(fabsf(q.qmax) <= 1e18f)) ? 1 : 0;
-    if (q.exact_all && cp.n_query > 0) atomicAdd(exact_clouds, 1);
-}
-__global__ void query_params_kernel(const CloudParams* __restrict__ table, const GridParams* __restrict__ grid, int C,
-                                    QueryParams* qp, int32_t* exact_clouds) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x)
-        query_params(table[c], grid[c], qp[c], exact_clouds, 0);
+// A cloud's largest query support, as the lean test's band takes it, and whether every pair takes the exact
+// test; derived from the statistics by whoever reads them.
+__device__ __forceinline__ bool query_limits(const CloudParams& cp, const GridParams& g, const QueryParams& q,
+                                             float& qmax) {
+    const bool has_q = cp.query_sup != nullptr && cp.mode != kScatter;
+    qmax = has_q ? key_float(q.stats.max_key) : 0.0f;
+    return (has_q && q.stats.bad) || (cp.mode != kGather && g.ref_stats.bad) || !(fabsf(qmax) <= 1e18f);
 }
 
 // Start of a count: the (last clouds of the) table; zeroes the per-search counters, the per-cloud query
-// statistics and the per-query counts; with ready also writes the clouds' query parameters (1: the
-// queries are the structure's sorted points, 2: there are no supports to reduce).
+// statistics and the per-query counts.  same_sorted: the queries are the structure's sorted points, whose
+// statistics are there.
 __global__ void count_init_kernel(const __grid_constant__ CloudChunk<kUploadChunk> ch, const GridParams* grid, Scratch W,
-                                  int C, int unit_cap, int64_t nq, int64_t stage_cap, int ready) {
+                                  int C, int unit_cap, int64_t nq, int64_t stage_cap, int same_sorted) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x)
         W.counts[i] = 0;
     if (blockIdx.x != 0) return;
     upload_chunk(ch, W.table, W.query_prefix, W.ref_prefix);
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
-        W.qparams[c].stats.max_key = 0;
-        W.qparams[c].stats.bad = 0;
+        const SupportStats none = {0u, 0};
+        W.qparams[c].stats = same_sorted ? grid[c].ref_stats : none;
         W.qparams[c].coord_key = 0;
     }
     if (threadIdx.x == 0) {
@@ -543,15 +531,10 @@ __global__ void count_init_kernel(const __grid_constant__ CloudChunk<kUploadChun
         *W.num_flagged = 0;
         *W.exact_clouds = 0;
         *W.num_exact = 0;
-        *W.pack_done = 0;
         *W.unit_cap = unit_cap;
         W.cursor[0] = 0ull;
         W.cursor[1] = (unsigned long long)stage_cap;
     }
-    if (!ready) return;
-    __syncthreads();  // (the block's own writes of the table and the counters)
-    for (int c = threadIdx.x; c < C; c += blockDim.x)
-        query_params(W.table[c], grid[c], W.qparams[c], W.exact_clouds, ready == 1);
 }
 
 __device__ __forceinline__ float4 load_point(const float* x, const float* h, int64_t i, int dim) {
@@ -949,12 +932,11 @@ __global__ void inc_merge_kernel(const K* __restrict__ stay_keys, const int32_t*
 // Self search: query i is reference i, so the reference order and cells group the queries.
 // Positions are the once-wrapped query coordinates (only periodic dims differ from rsorted), supports the
 // caller's of this call: a kept structure may be searched with others than it was built from.  Their
-// statistics are reduced on the way, as support_stats_kernel does, and the last block to finish writes the clouds'
-// query parameters.
+// statistics are reduced on the way, as support_stats_kernel does.
 __global__ void pack_self_queries_kernel(const CloudParams* __restrict__ table, const GridParams* grid,
                                          const int32_t* __restrict__ prefix, int C, const int32_t* __restrict__ rsidx,
                                          int64_t n, float4* __restrict__ qsorted, int32_t* __restrict__ qsidx,
-                                         QueryParams* qp, int32_t* exact_clouds, int32_t* done) {
+                                         QueryParams* qp) {
     const int64_t per = (n + gridDim.x - 1) / gridDim.x;
     const int64_t lo = (int64_t)blockIdx.x * per;
     const int64_t hi = min(n, lo + per);
@@ -980,8 +962,6 @@ __global__ void pack_self_queries_kernel(const CloudParams* __restrict__ table, 
         qsidx[t] = i;
     }
     block_stats(p.cloud, kmax, bad, out, stride);
-    if (last_block(done))
-        for (int c = threadIdx.x; c < C; c += blockDim.x) query_params(table[c], grid[c], qp[c], exact_clouds, 0);
 }
 
 // Group count comes from a device scalar; the scan kernels are launched over the upper bound
@@ -1147,6 +1127,7 @@ struct WalkArgs {
     int32_t* flagged;             // [units] units to re-walk in the emit pass
     int32_t* num_flagged;
     int32_t* num_exact;           // pairs inside the product's band, decided after the walk
+    int32_t* exact_clouds;
     int4* band_pairs;             // [nq] (sorted query, sorted reference, mask word of the staging list, bit)
     unsigned long long* cursor;   // staging list fill
     int32_t* stage;               // staging list
@@ -1171,7 +1152,7 @@ __device__ __forceinline__ void load_unit_ctx(UnitCtx& u, const WalkArgs& a, int
     u.dedupe = cp.dedupe;
     u.hash_len = cp.hash_len;
     u.error = g.error;
-    u.exact_all = q.exact_all;
+    u.exact_all = query_limits(cp, g, q, u.qmax);
     for (int d = 0; d < 3; ++d) {
         u.count[d] = g.count[d];
         u.dmin[d] = cp.dmin[d];
@@ -1181,7 +1162,6 @@ __device__ __forceinline__ void load_unit_ctx(UnitCtx& u, const WalkArgs& a, int
     u.qshift = a.local_index ? cp.query_base : 0;
     u.rshift = a.local_index ? cp.ref_base : 0;
     u.rmax = key_float(g.ref_stats.max_key);
-    u.qmax = q.qmax;
     // a float32 copy of a double coordinate x is off by <= |x| 2^-24, the float difference adds one
     // rounding: 2^-21 of the largest |coordinate| bounds a difference's error with room to spare
     u.f64_err = a.f64.qpos ? key_float(q.coord_key) * 4.76837158203125e-7f : 0.0f;
@@ -2581,6 +2561,10 @@ __global__ void stray_kernel(WalkArgs a) {
     // the last launch of a count or an emit leaves the work counters ready for the next emit
     if (blockIdx.x == 0 && threadIdx.x < kWorkCounters) a.work[threadIdx.x] = 0;
     if (!EMIT) {
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.num_clouds; c += gridDim.x * blockDim.x) {
+            float qmax;
+            if (a.table[c].n_query > 0 && query_limits(a.table[c], a.grid[c], a.qparams[c], qmax)) atomicAdd(a.exact_clouds, 1);
+        }
         const int64_t nband = min((int64_t)*a.num_exact, a.nq_total);
         for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nband; i += (int64_t)gridDim.x * blockDim.x)
             decide_band_pair(a, a.band_pairs[i]);
@@ -3081,6 +3065,7 @@ static WalkArgs make_walk(const HostBatch& b, const Structure& S, const Scratch&
     a.flagged = W.flagged;
     a.num_flagged = W.num_flagged;
     a.num_exact = W.num_exact;
+    a.exact_clouds = W.exact_clouds;
     a.band_pairs = reinterpret_cast<int4*>(W.pack);  // the packed points are sorted away by now
     a.cursor = W.cursor;
     a.query_ids = b.query_ids;
@@ -3222,13 +3207,13 @@ static int build_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
                                                                    W.inc_count, W.inc_count + 1);
             inc_decide_kernel<K><<<1, 1, 0, st>>>(sw.state, mw.state, W.inc_count, nr);
             note_launches(2);
-            TCR_CUDA(sort_coop<K>(mw, nr, S.num_cells + 1, NoTail(), st));
+            TCR_CUDA(sort_coop<K>(mw, nr, S.num_cells + 1, 0, NoTail(), st));
             inc_merge_kernel<K><<<grid_for(nr, 256), 256, 0, st>>>(
                 reinterpret_cast<const K*>(W.stay_keys), W.stay_idx, mw.keys[0], mw.keys[1], mw.vals[0], mw.vals[1],
                 mw.state, W.inc_count, nr, sw.keys[0], sw.vals[0]);
             note_launches(1);
         }
-        TCR_CUDA(sort_coop<K>(sw, nr, S.num_cells + 1,
+        TCR_CUDA(sort_coop<K>(sw, nr, S.num_cells + 1, inc ? 1 : 0,
                               BuildTail<K>{S.cell_start, S.num_cells, W.pack, S.rsorted, S.rsidx, b.lin_out, b.order_out,
                                            W.table, S.grid, S.cell_lin, S.cell_coords, S.cell_bucket, S.cell_cloud,
                                            S.map, nr},
@@ -3256,19 +3241,17 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
     int rc = upload_table(b, W, st, chunk);
     if (rc) return rc;
     const int unit_cap = b.unit_cap;
-    // Query parameters: from the structure's statistics where the queries are its sorted points
-    // themselves (same_sorted), with the packing of other self searches, else by launches of their own.
+    // The query supports' statistics: the structure's where the queries are its sorted points themselves, with
+    // the packing of other self searches, else by a launch of their own.
     const bool packed = b.self && !b.same_sorted && nq > 0;
-    const bool query_stats = b.any_query_sup && nq > 0 && !b.self;
-    count_init_kernel<<<grid_for(std::max<int64_t>(C, nq), 256), 256, 0, st>>>(
-        chunk, S.grid, W, C, unit_cap, nq, stage_cap, packed || query_stats ? 0 : (b.same_sorted ? 1 : 2));
+    count_init_kernel<<<grid_for(std::max<int64_t>(C, nq), 256), 256, 0, st>>>(chunk, S.grid, W, C, unit_cap, nq, stage_cap,
+                                                                               b.same_sorted ? 1 : 0);
     note_launches(1);
-    if (query_stats) {
+    if (b.any_query_sup && nq > 0 && !b.self) {
         support_stats_kernel<<<grid_for(nq, 256, num_sms() * 4), 256, 0, st>>>(
             W.table, W.query_prefix, C, nq, 1, reinterpret_cast<char*>(W.qparams) + offsetof(QueryParams, stats),
             (int64_t)sizeof(QueryParams));
-        query_params_kernel<<<grid_for(C, 128), 128, 0, st>>>(W.table, S.grid, C, W.qparams, W.exact_clouds);
-        note_launches(2);
+        note_launches(1);
     }
     if (f64 && (b.nr > 0 || nq > 0)) {
         f64_prep_kernel<<<grid_for(std::max<int64_t>(b.nr, nq * b.clouds[0].dim), 256), 256, 0, st>>>(
@@ -3281,8 +3264,7 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
         if (b.self) {
             if (packed) {
                 pack_self_queries_kernel<<<grid_for(nq, 256, num_sms() * 8), 256, 0, st>>>(
-                    W.table, S.grid, W.query_prefix, C, S.rsidx, nq, W.qsorted, W.qsidx, W.qparams, W.exact_clouds,
-                    W.pack_done);
+                    W.table, S.grid, W.query_prefix, C, S.rsidx, nq, W.qsorted, W.qsidx, W.qparams);
                 note_launches(1);
             }
             gstart = S.cell_start;
@@ -3295,7 +3277,7 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
             pack_points_kernel<K><<<grid_for(nq, 256, num_sms() * 4), 256, 0, st>>>(
                 W.table, S.grid, W.query_prefix, C, nq, 1, 1, 0, W.pack, sw.keys[0], sw.vals[0], sw.state);
             note_launches(1);
-            TCR_CUDA(sort_coop<K>(sw, nq, W.num_qgroups + 1,
+            TCR_CUDA(sort_coop<K>(sw, nq, W.num_qgroups + 1, 0,
                                   QueryTail<K>{W.qgroup_start, W.num_qgroups, W.pack, W.qsorted, W.qsidx, W.table,
                                                S.grid, W.qgroup_coords, W.qgroup_cloud, nq},
                                   st));

@@ -339,12 +339,13 @@ struct NoTail {
 template <typename K, typename Tail>
 __global__ void __launch_bounds__(kCoopThreads, 1)
     sort_coop_kernel(K* keys0, K* keys1, int32_t* vals0, int32_t* vals1, int64_t n_all, SortStateT<K>* st,
-                     int32_t* hist, int32_t* failed, Tail tail) {
+                     int32_t* hist, int32_t* failed, int chained, Tail tail) {
     extern __shared__ __align__(16) unsigned char coop_raw[];
     CoopSmem<K>& sm = *reinterpret_cast<CoopSmem<K>*>(coop_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, b = blockIdx.x;
-    const int32_t gone = *(volatile int32_t*)failed;  // a sort before this one gave up: its pairs are not there
+    // a sort before this one gave up: its pairs are not there
+    const int32_t gone = chained ? *(volatile int32_t*)failed : 0;
     const int64_t n = (st->n_dev >= 0 && st->n_dev < n_all) ? st->n_dev : n_all;
     const int64_t per = ((n + G - 1) / G + 31) & ~int64_t(31);
     const int64_t lo = min(n, per * b), hi = min(n, lo + per);
@@ -539,9 +540,11 @@ inline int coop_blocks(int64_t n, int sms) {
 }
 
 // Launches the one-launch sort of keys[0] / vals[0] (the selector and the key range as for
-// radix_sort_pairs; the sorted keys end in buffer state->sel[key_passes<K>()]).
+// radix_sort_pairs; the sorted keys end in buffer state->sel[key_passes<K>()]).  chained: the pairs come from
+// a sort with the same flag.
 template <typename K, typename Tail>
-inline cudaError_t sort_coop(const SortWorkspaceT<K>& w, int64_t n, int32_t* failed, Tail tail, cudaStream_t st) {
+inline cudaError_t sort_coop(const SortWorkspaceT<K>& w, int64_t n, int32_t* failed, int chained, Tail tail,
+                             cudaStream_t st) {
     int dev = 0, sms = 148;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -557,7 +560,7 @@ inline cudaError_t sort_coop(const SortWorkspaceT<K>& w, int64_t n, int32_t* fai
     K *k0 = w.keys[0], *k1 = w.keys[1];
     int32_t *v0 = w.vals[0], *v1 = w.vals[1], *hist = w.hist;
     SortStateT<K>* state = w.state;
-    void* args[] = {&k0, &k1, &v0, &v1, &n, &state, &hist, &failed, &tail};
+    void* args[] = {&k0, &k1, &v0, &v1, &n, &state, &hist, &failed, &chained, &tail};
     // One block per SM is resident on the whole device; a stream that is given fewer SMs (a partition of
     // them) refuses that many.  Any number of blocks sorts, in longer ranges.
     for (int blocks = coop_blocks(n, sms);; blocks = (blocks + 1) / 2) {
