@@ -132,7 +132,8 @@ struct Scratch {
     int64_t* info;          // [8] see tcr_count
     int32_t* num_flagged;   // [1]
     int32_t* exact_clouds;  // [1] clouds whose every pair takes the exact test
-    int32_t* num_exact;     // [1] pairs inside the count walk's band, decided exactly
+    int32_t* num_exact;     // [3] pairs inside the count walk's band: listed one by one, decided with their window;
+                            // windows listed
     int32_t* unit_cap;      // [1] queries per work unit of this search (set by the count phase)
     unsigned long long* cursor;  // [2] staging fill, staging capacity
     float4* pack;           // [max(nq,nr)] packed input points before sorting
@@ -180,7 +181,7 @@ static Scratch carve_scratch(void* buf, int64_t nq, int64_t nr, int64_t C, bool 
     s.info = c.take<int64_t>(8);
     s.num_flagged = c.take<int32_t>(1);
     s.exact_clouds = c.take<int32_t>(1);
-    s.num_exact = c.take<int32_t>(1);
+    s.num_exact = c.take<int32_t>(3);
     s.unit_cap = c.take<int32_t>(1);
     s.cursor = c.take<unsigned long long>(2);
     s.pack = c.take<float4>(nmax);
@@ -504,9 +505,12 @@ __global__ void finish_cells_kernel(int32_t* cell_start, const int32_t* num_cell
 // test; derived from the statistics by whoever reads them.
 __device__ __forceinline__ bool query_limits(const CloudParams& cp, const GridParams& g, const QueryParams& q,
                                              float& qmax) {
-    const bool has_q = cp.query_sup != nullptr && cp.mode != kScatter;
-    qmax = has_q ? key_float(q.stats.max_key) : 0.0f;
-    return (has_q && q.stats.bad) || (cp.mode != kGather && g.ref_stats.bad) || !(fabsf(qmax) <= 1e18f);
+    // (every field is read first: as short-circuits the reads waited for each other)
+    const int mode = cp.mode, qbad = q.stats.bad, rbad = g.ref_stats.bad;
+    const uint32_t key = q.stats.max_key;
+    const bool has_q = (cp.query_sup != nullptr) & (mode != kScatter);
+    qmax = has_q ? key_float(key) : 0.0f;
+    return (has_q & (qbad != 0)) | ((mode != kGather) & (rbad != 0)) | !(fabsf(qmax) <= 1e18f);
 }
 
 // Start of a count: the (last clouds of the) table; zeroes the per-search counters, the per-cloud query
@@ -530,7 +534,7 @@ __global__ void count_init_kernel(const __grid_constant__ CloudChunk<kUploadChun
         *W.num_units = 0;
         *W.num_flagged = 0;
         *W.exact_clouds = 0;
-        *W.num_exact = 0;
+        W.num_exact[0] = W.num_exact[1] = W.num_exact[2] = 0;
         *W.unit_cap = unit_cap;
         W.cursor[0] = 0ull;
         W.cursor[1] = (unsigned long long)stage_cap;
@@ -1067,6 +1071,12 @@ constexpr float kMmaSupport = 4.0f;
 constexpr float kMmaReach = 16.0f;
 constexpr float kMmaPad = 15.0f;
 constexpr float kMmaFar = 60000.0f;
+// Lanes with a pair inside the band, over the chunks of a window, from which on the window is listed as a whole, if
+// they are also one a pair of chunks; fewer list their pairs.  A random cloud's window has one at most nearly always,
+// and 0.3 on average where 32 queries meet 16 pairs of chunks (20k points in 4^3 periodic cells: 654 us when four
+// lanes there listed the window, which takes one warp 30 us); a lattice's has four even in 1D (1M points: 1.15 ms,
+// 1.45 when eight were asked for).
+constexpr int kBandLanes = 4;
 
 // The unit's cloud, as the walk kernels read it (shared memory, warp-uniform).
 struct UnitCtx {
@@ -1123,12 +1133,14 @@ struct WalkArgs {
     int32_t* stray;
     int32_t* num_stray;
     int32_t* counts;              // [nq] count output, global query order
-    int32_t* rec;                 // [units] offset of each unit's record in the staging list, -1 if not staged
+    int32_t* rec;                 // [units] offset of each unit's record in the staging list, negative if not staged
     int32_t* flagged;             // [units] units to re-walk in the emit pass
     int32_t* num_flagged;
-    int32_t* num_exact;           // pairs inside the product's band, decided after the walk
+    int32_t* num_exact;           // [3] pairs inside the product's band, listed; decided with their window; windows listed
     int32_t* exact_clouds;
     int4* band_pairs;             // [nq] (sorted query, sorted reference, mask word of the staging list, bit)
+    unsigned long long* band_windows;  // [band_cap] unit << 32 | window << 16 | its marked pairs of chunks
+    int64_t band_cap;
     unsigned long long* cursor;   // staging list fill
     int32_t* stage;               // staging list
     int64_t stage_cap;
@@ -1899,7 +1911,7 @@ __device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int3
                 const int32_t j = sm.delta[w][run] + (w0 + min(k, wn - 1));
                 return __ldg(&a.rsorted[j]);
             };
-            uint32_t marked = 0;  // the window's pairs of chunks with a pair inside the band
+            uint32_t marked = 0;  // bits 0 .. 15: the window's pairs of chunks with a pair inside the band; then: lanes with one
             // one copy of the loop per number of query tiles: a tile costs no branch
             auto pairs = [&](auto tiles) {
                 constexpr int NT = decltype(tiles)::value;
@@ -1955,7 +1967,8 @@ __device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int3
                         if (NT >= 3) p1 = mma_hits<MODE>(p1, c0, c1, cs, qb[0], qb[1], qs[2], umin);
                     }
                     redo |= far;
-                    if (__any_sync(0xffffffffu, umin <= band)) marked |= 1u << (k0 >> 6);
+                    const uint32_t close = __ballot_sync(0xffffffffu, umin <= band);
+                    if (close) marked += (1u << (k0 >> 6)) + ((uint32_t)__popc(close) << 16);
                     const bool in = k0 + 32 * half < wn;
                     const uint32_t m0 = nibble_transpose(p0, lane);
                     count += __popc(m0);
@@ -1975,9 +1988,11 @@ __device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int3
             else pairs(std::integral_constant<int, 4>());
             // rare: list the pairs inside the band among the marked chunks -- their products again, tile by
             // tile, each lane keeping its own
-            if (!stage && marked) redo = true;
+            const bool list = stage && (int32_t)(marked >> 16) < max(kBandLanes, (wn + 63) >> 6);
+            bool full = !list;
+            marked &= 0xffffu;
 #pragma unroll 1
-            for (int32_t c = 0; stage && 32 * c < wn && (marked >> (c >> 1)); ++c) {
+            for (int32_t c = 0; list && 32 * c < wn && (marked >> (c >> 1)); ++c) {
                 if (!((marked >> (c >> 1)) & 1u)) continue;
                 int32_t run;
                 const float4 v = fetch(32 * c + lane, run);
@@ -2012,10 +2027,20 @@ __device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int3
                                 a.unit_t0[unit] + q, sm.delta[w][run] + w0 + k,
                                 a.rec[unit] + kRecHeader + 2 * R + 1 + ((w0 + k) >> 5) * nb + q, k & 31);
                         else
-                            redo = true;  // the list is full
+                            full = true;  // the list is
                     }
                     __syncwarp();
                 }
+            }
+            // many of them, or no place for them: the window, to be tested again
+            if (marked && __any_sync(0xffffffffu, full) && lane == 0) {
+                // (every place that is claimed is written)
+                const bool named = w0 < (kWalkWin << 16);
+                const int32_t f = named ? atomicAdd(&a.num_exact[2], 1) : 0;
+                if (named && f < a.band_cap)
+                    a.band_windows[f] = ((unsigned long long)(uint32_t)unit << 32) | (uint32_t)(w0 / kWalkWin) << 16 | marked;
+                else
+                    redo = true;
             }
         }
         redo = __any_sync(0xffffffffu, redo);
@@ -2028,7 +2053,10 @@ __device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int3
     }
     if (n.active) a.counts[n.qorig] = (int32_t)count;
     __syncwarp();
-    if (nchunks > 0 && (!product || redo)) fix_unit<DIM, PERIODIC, MODE>(a, sm, unit, grp, lane, w);
+    if (nchunks > 0 && (!product || redo)) {
+        if (lane == 0 && a.rec[unit] < 0) a.rec[unit] = -2;  // not staged, and no listed window of it needs deciding
+        fix_unit<DIM, PERIODIC, MODE>(a, sm, unit, grp, lane, w);
+    }
 }
 
 // Class (dim * 2 + any periodic dim) of a cloud, the key of the walk kernels' template.
@@ -2529,9 +2557,30 @@ __global__ void compose_ids_kernel(const int32_t* __restrict__ rsidx, const int3
     }
 }
 
-// Serial walk for queries whose own cell differs from their group's (one thread per query).
-// After the count walk also: each pair inside the product's band decided by the reference's exact test, its
-// hit bit and its query's count corrected where the product's sign said otherwise (one thread per pair).
+// Sets hit `bit` of a mask to what the exact test found: 1 or -1 where that is a change.  (A pair may be listed by
+// itself and with its window; one of the two finds the change.)
+__device__ __forceinline__ int set_hit(uint32_t* mask, int bit, bool in) {
+    const uint32_t b = 1u << bit;
+    if (in) return (atomicOr(mask, b) & b) ? 0 : 1;
+    return (atomicAnd(mask, ~b) & b) ? -1 : 0;
+}
+
+// Where a window's runs start (at: the lane's run, relative to the window), and the rank of each chunk's first run.
+__device__ __forceinline__ void lay_window(WalkSmem& sm, int lane, int w, bool starts, int32_t at) {
+    sm.starts[w][lane] = make_uint2(0u, 0u);
+    __syncwarp();
+    if (starts && at >= 0 && at < kWalkWin) atomicOr(&sm.starts[w][at >> 5].x, 1u << (at & 31));
+    __syncwarp();
+    const int32_t before = __popc(__ballot_sync(0xffffffffu, starts && at < 0));
+    const int32_t here = __popc(sm.starts[w][lane].x);
+    const int32_t upto = before + warp_inclusive_scan(here) - 1;
+    sm.starts[w][lane].y = (uint32_t)(upto - here);
+    if (lane == 31) sm.starts[w][32] = sm.starts[w][33] = make_uint2(0u, (uint32_t)upto);
+    __syncwarp();
+}
+
+// A pair inside the product's band decided by the reference's exact test after the walk, its hit bit and its query's
+// count corrected where the product's sign said otherwise.
 __device__ __forceinline__ void decide_band_pair(const WalkArgs& a, const int4& p) {
     if (!TCR_GUARD(p.x, a.nq_total) || !TCR_GUARD(p.y, a.nr_total) || !TCR_GUARD(p.z, a.stage_cap)) return;
     const int32_t qorig = a.qsidx[p.x];
@@ -2548,26 +2597,190 @@ __device__ __forceinline__ void decide_band_pair(const WalkArgs& a, const int4& 
         const float4 q = a.qsorted[p.x], c = a.rsorted[p.y];
         in = exact_pair_test(xc, q, q.w, c, c.w);
     }
-    const uint32_t bit = 1u << (p.w & 31);
-    const bool was = (a.stage[p.z] & bit) != 0;
-    if (in == was) return;
-    atomicXor(reinterpret_cast<uint32_t*>(&a.stage[p.z]), bit);
-    atomicAdd(&a.counts[qorig], in ? 1 : -1);
+    if (const int change = set_hit(reinterpret_cast<uint32_t*>(&a.stage[p.z]), p.w & 31, in)) atomicAdd(&a.counts[qorig], change);
 }
 
+// What decide_window keeps in shared memory, in place of the second chunk's fragments.
+struct BandSmem {
+    uint32_t pair[64];   // bit 31: the product's decision, [10, 15): query, [0, 10): candidate of the window
+    int32_t change[32];  // per query: pairs found less pairs lost
+};
+static_assert(sizeof(BandSmem) <= sizeof(uint4) * 2 * 32 && kWalkWin <= 1024, "fits the fragments of one chunk");
+
+// A window of a unit's candidates with many pairs inside the product's band (points on a lattice whose spacing
+// divides the support: most queries have some): the products of its marked pairs of chunks again, the pairs
+// inside the band queued in shared memory and decided 32 at a time by the exact test, one per lane.  (Tested again
+// by fix_unit, one candidate per lane against every query, 1M lattice points took 2.75 ms, of 0.6 ms without pairs at
+// the threshold; now NNN.)  Not in the walk, whose registers and code it would share.
+template <int DIM, int MODE>
+__device__ __noinline__ void decide_window(const WalkArgs& a, WalkSmem& sm, unsigned long long entry, int lane, int w) {
+    const UnitCtx& u = sm.u[w];
+    BandSmem& near = *reinterpret_cast<BandSmem*>(&sm.cand[w][1][0][0]);
+    const int32_t unit = (int32_t)(entry >> 32), w0 = (int32_t)((entry >> 16) & 0xffffu) * kWalkWin;
+    const uint32_t marked = (uint32_t)entry & 0xffffu;
+    const int32_t t0 = a.unit_t0[unit], base = a.rec[unit];
+    if (base < -1) return;  // the unit was tested again as a whole
+    const Unit n = open_unit<DIM, true, false>(a, u, unit, a.unit_group[unit], lane);
+    const int32_t wn = min(n.M - w0, kWalkWin);
+    uint32_t* msk = nullptr;  // the window's first hit mask
+    if (base >= 0 && TCR_GUARD(base + kRecHeader, a.stage_cap))
+        msk = reinterpret_cast<uint32_t*>(a.stage + base + kRecHeader + 2 * a.stage[base + 1] + 1) + (int64_t)(w0 >> 5) * n.nb;
+    // runs, queries and scale as count_unit has them
+    const bool starts = n.cnt > 0;
+    const uint32_t smask = __ballot_sync(0xffffffffu, starts), lt = (1u << lane) - 1u;
+    const int rid = __popc(smask & lt);
+    if (starts) {
+        sm.delta[w][rid] = n.beg - n.pre;
+        for (int d = 0; d < 3; ++d) sm.shift[w][d][rid] = n.sh[d];
+    }
+    const float s = u.scale;
+    float os[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) os[d] = d < DIM ? -s * fmaf((float)n.gc[d] + 0.5f, u.hcell[d], u.dmin[d]) : 0.f;
+    const float H = n.q.w * s;
+    store_query_frag<MODE>(sm.query[w][lane], fmaf(n.q.x, s, os[0]), DIM > 1 ? fmaf(n.q.y, s, os[1]) : 0.f,
+                           DIM > 2 ? fmaf(n.q.z, s, os[2]) : 0.f, H, n.active);
+    if (MODE == kSuperSymmetric) sm.qsq[w][lane] = H * H;
+    lay_window(sm, lane, w, starts, n.pre - w0);
+    const float band = u.mma_band + (n.seam ? u.mma_seam : 0.f);
+    const int g = lane >> 2, tq = lane & 3, slot = cand_slot(lane);
+    const uint32_t crow = (uint32_t)__cvta_generic_to_shared(
+        &sm.cand[w][0][lane >> 4][cand_slot(4 * (lane & 7) + ((lane >> 3) & 1))]);
+    near.change[lane] = 0;
+    int32_t waiting = 0, decided = 0;
+    auto run_of = [&](int32_t k) -> int32_t {  // candidate k of the window
+        const uint2 st = sm.starts[w][k >> 5];
+        return (int32_t)st.y + __popc(st.x & ((2u << (k & 31)) - 1u));
+    };
+    auto decide = [&]() {  // the first 32 waiting pairs (the rest moves up)
+        __syncwarp();
+        const int32_t m = min(waiting, 32);
+        if (lane < m) {
+            const uint32_t e = near.pair[lane];
+            const int q = (e >> 10) & 31, k = e & 1023;
+            const int32_t j = sm.delta[w][run_of(k)] + w0 + k;
+            bool in;
+            if (a.f64.qpos) {
+                in = f64_pair_decide(a.f64, DIM, u.periodic_mask, MODE, a.qsidx[t0 + q] - u.qshift, j);
+            } else {
+                const float4 x = a.qsorted[t0 + q], c = a.rsorted[j];
+                in = exact_pair_test(unit_exact_ctx(u, MODE), x, x.w, c, c.w);
+            }
+            if (in != ((e >> 31) != 0)) {
+                const int change = msk ? set_hit(&msk[(k >> 5) * n.nb + q], k & 31, in) : (in ? 1 : -1);
+                if (change) atomicAdd(&near.change[q], change);
+            }
+        }
+        waiting -= m;
+        decided += m;
+        __syncwarp();
+        const uint32_t rest = near.pair[32 + lane];
+        __syncwarp();
+        if (lane < waiting) near.pair[lane] = rest;
+        __syncwarp();
+    };
+#pragma unroll 1
+    for (int32_t c = 0; 32 * c < wn; ++c) {
+        if (!((marked >> (c >> 1)) & 1u)) continue;
+        const int32_t k0 = min(32 * c + lane, wn - 1), run = run_of(k0);  // (lanes past the last candidate repeat it)
+        const float4 v = __ldg(&a.rsorted[sm.delta[w][run] + w0 + k0]);
+        float x = v.x, y = v.y, z = v.z;
+        if (n.seam) {
+            x += sm.shift[w][0][run];
+            if (DIM > 1) y += sm.shift[w][1][run];
+            if (DIM > 2) z += sm.shift[w][2][run];
+        }
+        __syncwarp();  // (the last chunk's fragments are read)
+        store_cand_frag<MODE>(&sm.cand[w][0][0][slot], &sm.cand[w][0][1][slot], fmaf(x, s, os[0]),
+                              DIM > 1 ? fmaf(y, s, os[1]) : 0.f, DIM > 2 ? fmaf(z, s, os[2]) : 0.f, v.w * s);
+        if (MODE == kSuperSymmetric) sm.csq[w][0][lane] = (v.w * s) * (v.w * s);
+        __syncwarp();
+#pragma unroll 1
+        for (int i = 0; 8 * (i >> 1) < n.nb; ++i) {  // tile i & 1 of the candidates, i >> 1 of the queries
+            uint32_t cf[4];
+            load_matrix(cf, crow ^ (32u * (i & 1)));
+            const uint32_t* qf = reinterpret_cast<const uint32_t*>(&sm.query[w][8 * (i >> 1) + g][0]);
+            float d[4];
+            mma_16x8(d, cf, qf[tq], qf[4 + tq]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int q = 8 * (i >> 1) + 2 * tq + (j & 1), k = 32 * c + 4 * g + 2 * (i & 1) + (j >> 1);
+                float r = d[j];
+                if (MODE == kSuperSymmetric) r -= fmaxf(sm.qsq[w][q], sm.csq[w][0][k & 31]);
+                const bool close = fabsf(r) <= band && q < n.nb && k < wn;
+                const uint32_t m = __ballot_sync(0xffffffffu, close);
+                if (m == 0) continue;
+                if (close) near.pair[waiting + __popc(m & lt)] = (__float_as_uint(r) & 0x80000000u) | (uint32_t)(q << 10 | k);
+                waiting += __popc(m);
+                if (waiting >= 32) decide();
+            }
+        }
+    }
+    if (waiting > 0) decide();
+    __syncwarp();
+    if (n.active && near.change[lane] != 0) atomicAdd(&a.counts[n.qorig], near.change[lane]);
+    if (lane == 0) atomicAdd(&a.num_exact[1], decided);
+    __syncwarp();
+}
+
+template <int DIM>
+__device__ __forceinline__ void decide_window_mode(const WalkArgs& a, WalkSmem& sm, unsigned long long entry, int lane, int w) {
+    switch (a.mode) {
+        case kGather: return decide_window<DIM, kGather>(a, sm, entry, lane, w);
+        case kScatter: return decide_window<DIM, kScatter>(a, sm, entry, lane, w);
+        case kSymmetric: return decide_window<DIM, kSymmetric>(a, sm, entry, lane, w);
+        default: return decide_window<DIM, kSuperSymmetric>(a, sm, entry, lane, w);
+    }
+}
+
+// The listed windows, one warp each.
+__device__ __forceinline__ void decide_windows(const WalkArgs& a) {
+    const int32_t n = (int32_t)min((int64_t)a.num_exact[2], a.band_cap);
+    if (n == 0) return;
+    __shared__ WalkSmem sm;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    sm.cand[w][0][1][lane].w = kHalfOnes;
+    const int32_t units = *a.num_units;
+    int cur = -1;
+    for (int32_t i = blockIdx.x * kWalkWarps + w; i < n; i += gridDim.x * kWalkWarps) {
+        const unsigned long long entry = a.band_windows[i];
+        if (!TCR_GUARD(entry >> 32, units)) continue;
+        const int32_t grp = a.unit_group[entry >> 32];
+        const int cloud = a.num_clouds == 1 ? 0 : a.group_cloud[grp];
+        if (cloud != cur) {
+            __syncwarp();
+            if (lane == 0) load_unit_ctx(sm.u[w], a, cloud);
+            cur = cloud;
+            __syncwarp();
+        }
+        if (sm.u[w].dim == 1) decide_window_mode<1>(a, sm, entry, lane, w);
+        else if (sm.u[w].dim == 2) decide_window_mode<2>(a, sm, entry, lane, w);
+        else decide_window_mode<3>(a, sm, entry, lane, w);
+    }
+}
+
+// Resident blocks per SM of the launch after the count walk (registers <= 65536 / (128 * blocks)): a listed window is a
+// chain of reads for one warp, so warps in flight decide (1M lattice points, 3D / 1D: 1.22 / 1.18 ms with five,
+// 1.18 / 1.13 with seven).
+constexpr int kStrayBlocks = 7;
+
+// Serial walk for queries whose own cell differs from their group's (one thread per query).  After the count
+// walk also: the pairs inside the product's band (one thread per listed pair, one warp per listed window).
 template <bool EMIT>
-__global__ void stray_kernel(WalkArgs a) {
+__global__ void __launch_bounds__(kWalkWarps * 32, EMIT ? 1 : kStrayBlocks) stray_kernel(const __grid_constant__ WalkArgs a) {
     const int32_t ns = *a.num_stray;
     // the last launch of a count or an emit leaves the work counters ready for the next emit
     if (blockIdx.x == 0 && threadIdx.x < kWorkCounters) a.work[threadIdx.x] = 0;
-    if (!EMIT) {
+    if constexpr (!EMIT) {
         for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.num_clouds; c += gridDim.x * blockDim.x) {
             float qmax;
-            if (a.table[c].n_query > 0 && query_limits(a.table[c], a.grid[c], a.qparams[c], qmax)) atomicAdd(a.exact_clouds, 1);
+            const bool any = a.table[c].n_query > 0;
+            if (query_limits(a.table[c], a.grid[c], a.qparams[c], qmax) & any) atomicAdd(a.exact_clouds, 1);
         }
         const int64_t nband = min((int64_t)*a.num_exact, a.nq_total);
         for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nband; i += (int64_t)gridDim.x * blockDim.x)
             decide_band_pair(a, a.band_pairs[i]);
+        decide_windows(a);
     }
     for (int32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
         const int32_t t = a.stray[s];
@@ -2777,7 +2990,7 @@ struct OffsetOut {
         info[3] = *exact_clouds;
         info[4] = (int64_t)*cursor;
         info[5] = *num_flagged;
-        info[6] = *num_exact;
+        info[6] = min((int64_t)num_exact[0], n) + num_exact[1];
         // incremental build: points sorted by the small sort (-1: the full sort ran); -2: no hint
         info[7] = inc_count ? ((inc_count[1] != 0 || 2 * (int64_t)inc_count[0] < n_ref) ? -1 : n_ref - inc_count[0]) : -2;
     }
@@ -3067,6 +3280,8 @@ static WalkArgs make_walk(const HostBatch& b, const Structure& S, const Scratch&
     a.num_exact = W.num_exact;
     a.exact_clouds = W.exact_clouds;
     a.band_pairs = reinterpret_cast<int4*>(W.pack);  // the packed points are sorted away by now
+    a.band_windows = reinterpret_cast<unsigned long long*>(W.keys[1]);  // and so are the keys
+    a.band_cap = std::max(b.nq, b.nr);
     a.cursor = W.cursor;
     a.query_ids = b.query_ids;
     a.ref_ids = b.ref_ids;
@@ -3294,7 +3509,7 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
         prof_mark(TCR_PROFILE_COUNT_WALK, 0, st);
         TCR_CUDA(launch_walks<CountLaunch>(b, a, dim3(walk_blocks(b, nq)), dim3(kWalkWarps * 32), 0, st));
         prof_mark(TCR_PROFILE_COUNT_WALK, 1, st);
-        stray_kernel<false><<<grid_for(nq, 128, num_sms() * 4), 128, 0, st>>>(a);
+        stray_kernel<false><<<grid_for(nq, 128, num_sms() * kStrayBlocks), kWalkWarps * 32, 0, st>>>(a);
         note_launches(1);
     }
     CountIn ci{W.counts, nq};
@@ -3357,7 +3572,7 @@ static int emit_impl(const HostBatch& b, const Structure& S, const Scratch& W, c
         note_launches(1);
     }
     TCR_CUDA(launch_walks<EmitLaunch>(b, a, dim3(walk_blocks(b, nq)), dim3(kWalkWarps * 32), 0, st));
-    stray_kernel<true><<<grid_for(nq, 128, num_sms() * 4), 128, 0, st>>>(a);
+    stray_kernel<true><<<grid_for(nq, 128, num_sms() * 4), kWalkWarps * 32, 0, st>>>(a);
     note_launches(1);
     return TCR_OK;
 }
