@@ -965,7 +965,19 @@ __global__ void pack_self_queries_kernel(const CloudParams* __restrict__ table, 
         qsorted[t] = wrap_point(p.dim, p.periodic_mask, p.dmin, p.ext, v, 1);
         qsidx[t] = i;
     }
-    block_stats(p.cloud, kmax, bad, out, stride);
+    // A warp that stayed in one cloud reduces first.  No barriers, and an atomic only where it raises the maximum:
+    // reduced by blocks, 1M periodic points took 29 us instead of 25.
+    const int c0 = __shfl_sync(0xffffffffu, p.cloud, 0);
+    const bool one = __all_sync(0xffffffffu, p.cloud < 0 || p.cloud == c0);
+    if (one) {
+        kmax = __reduce_max_sync(0xffffffffu, kmax);
+        bad = __reduce_or_sync(0xffffffffu, bad);
+    }
+    if (p.cloud >= 0 && (!one || (threadIdx.x & 31) == 0)) {
+        SupportStats* st = stats_at(out, stride, p.cloud);
+        if (kmax > *(volatile uint32_t*)&st->max_key) atomicMax(&st->max_key, kmax);
+        if (bad && *(volatile int32_t*)&st->bad == 0) atomicOr(&st->bad, 1);
+    }
 }
 
 // Group count comes from a device scalar; the scan kernels are launched over the upper bound
@@ -1796,6 +1808,89 @@ __device__ __noinline__ void fix_unit(const WalkArgs& a, WalkSmem& wsm, int32_t 
     wsm.cand[w][0][1][lane].w = wsm.cand[w][1][1][lane].w = kHalfOnes;
 }
 
+// The pairs inside the band among a window's marked chunks, listed: their products again, tile by tile, each lane
+// keeping its own.  Many of them, or no place for them: the window itself.  Returns true when there is no
+// place for that either.  Out of line, so that the walk's registers hold none of it (in line, the walk took 2 to 5%
+// longer in half of the modes).
+template <int DIM, bool PERIODIC, int MODE>
+__device__ __noinline__ bool list_band(const WalkArgs& a, WalkSmem& sm, int32_t unit, int32_t grp, int32_t w0, int32_t M,
+                                       uint32_t marked, bool seam, int lane, int w) {
+    const UnitCtx& u = sm.u[w];
+    const int32_t wn = min(M - w0, kWalkWin), nb = min(*a.unit_cap, a.group_start[grp + 1] - a.unit_t0[unit]);
+    const float s = u.scale;
+    float os[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        os[d] = d < DIM ? -s * fmaf((float)a.group_coords[3 * grp + d] + 0.5f, u.hcell[d], u.dmin[d]) : 0.f;
+    float band = u.mma_band;
+    if (PERIODIC && seam) band += u.mma_seam;
+    const int g = lane >> 2, tq = lane & 3, slot = cand_slot(lane);
+    const uint32_t crow = (uint32_t)__cvta_generic_to_shared(
+        &sm.cand[w][0][lane >> 4][cand_slot(4 * (lane & 7) + ((lane >> 3) & 1))]);
+    const int32_t base = a.rec[unit];
+    const int32_t masks = base >= 0 ? base + kRecHeader + 2 * a.stage[base + 1] + 1 : 0;
+    auto run_of = [&](int32_t k) -> int32_t {
+        const uint2 st = sm.starts[w][k >> 5];
+        return (int32_t)st.y + __popc(st.x & ((2u << (k & 31)) - 1u));
+    };
+    bool full = base < 0 || (int32_t)(marked >> 16) >= max(kBandLanes, (wn + 63) >> 6);
+    const bool list = !full;  // the pairs one by one
+    marked &= 0xffffu;
+#pragma unroll 1
+    for (int32_t c = 0; list && 32 * c < wn && (marked >> (c >> 1)); ++c) {
+        if (!((marked >> (c >> 1)) & 1u)) continue;
+        const int32_t kl = min(32 * c + lane, wn - 1), run = run_of(kl);
+        const float4 v = __ldg(&a.rsorted[sm.delta[w][run] + w0 + kl]);
+        float x = v.x, y = v.y, z = v.z;
+        if (PERIODIC && seam) {
+            x += sm.shift[w][0][run];
+            if (DIM > 1) y += sm.shift[w][1][run];
+            if (DIM > 2) z += sm.shift[w][2][run];
+        }
+        store_cand_frag<MODE>(&sm.cand[w][0][0][slot], &sm.cand[w][0][1][slot], fmaf(x, s, os[0]),
+                              DIM > 1 ? fmaf(y, s, os[1]) : 0.f, DIM > 2 ? fmaf(z, s, os[2]) : 0.f, v.w * s);
+        if (MODE == kSuperSymmetric) sm.csq[w][0][lane] = (v.w * s) * (v.w * s);
+        __syncwarp();
+#pragma unroll 1
+        for (int i = 0; 8 * (i >> 1) < nb; ++i) {  // tile i & 1 of the candidates, i >> 1 of the queries
+            uint32_t cf[4];
+            load_matrix(cf, crow ^ (32u * (i & 1)));
+            const uint32_t* qf = reinterpret_cast<const uint32_t*>(&sm.query[w][8 * (i >> 1) + g][0]);
+            float d[4];
+            mma_16x8(d, cf, qf[tq], qf[4 + tq]);
+            const int q0 = 8 * (i >> 1) + 2 * tq, k0 = 32 * c + 4 * g + 2 * (i & 1);  // of d[0]; d[j]: q0 + (j & 1), k0 + (j >> 1)
+            uint32_t close = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float r = d[j];
+                if (MODE == kSuperSymmetric) r -= fmaxf(sm.qsq[w][q0 + (j & 1)], sm.csq[w][0][(k0 + (j >> 1)) & 31]);
+                close |= (fabsf(r) <= band && q0 + (j & 1) < nb && k0 + (j >> 1) < wn ? 1u : 0u) << j;
+            }
+            for (; close; close &= close - 1) {
+                const int j = __ffs(close) - 1, q = q0 + (j & 1), k = k0 + (j >> 1);
+                const int32_t f = atomicAdd(a.num_exact, 1);
+                if (f < a.nq_total)
+                    a.band_pairs[f] = make_int4(a.unit_t0[unit] + q, sm.delta[w][run_of(k)] + w0 + k,
+                                                masks + ((w0 + k) >> 5) * nb + q, k & 31);
+                else
+                    full = true;  // the list is
+            }
+            __syncwarp();
+        }
+    }
+    bool lost = false;
+    if (__any_sync(0xffffffffu, full) && lane == 0) {
+        // (every place that is claimed is written)
+        const bool named = w0 < (kWalkWin << 16);
+        const int32_t f = named ? atomicAdd(&a.num_exact[2], 1) : 0;
+        lost = !named || f >= a.band_cap;
+        if (!lost)
+            a.band_windows[f] = ((unsigned long long)(uint32_t)unit << 32) | (uint32_t)(w0 / kWalkWin) << 16 | marked;
+    }
+    __syncwarp();
+    return lost;
+}
+
 // Count walk of one unit: test every (query, candidate) once, count, and stage the unit's record.
 //
 // The unit's candidates stream two chunks of 32 at a time, one per lane and chunk (a lane finds its
@@ -1986,62 +2081,8 @@ __device__ __forceinline__ void count_unit(const WalkArgs& a, WalkSmem& sm, int3
             else if (nb <= 16) pairs(std::integral_constant<int, 2>());
             else if (nb <= 24) pairs(std::integral_constant<int, 3>());
             else pairs(std::integral_constant<int, 4>());
-            // rare: list the pairs inside the band among the marked chunks -- their products again, tile by
-            // tile, each lane keeping its own
-            const bool list = stage && (int32_t)(marked >> 16) < max(kBandLanes, (wn + 63) >> 6);
-            bool full = !list;
-            marked &= 0xffffu;
-#pragma unroll 1
-            for (int32_t c = 0; list && 32 * c < wn && (marked >> (c >> 1)); ++c) {
-                if (!((marked >> (c >> 1)) & 1u)) continue;
-                int32_t run;
-                const float4 v = fetch(32 * c + lane, run);
-                float x = v.x, y = v.y, z = v.z;
-                if (PERIODIC && n.seam) {
-                    x += sm.shift[w][0][run];
-                    if (DIM > 1) y += sm.shift[w][1][run];
-                    if (DIM > 2) z += sm.shift[w][2][run];
-                }
-                store_cand_frag<MODE>(&sm.cand[w][0][0][slot], &sm.cand[w][0][1][slot], fmaf(x, s, os[0]),
-                                      DIM > 1 ? fmaf(y, s, os[1]) : 0.f, DIM > 2 ? fmaf(z, s, os[2]) : 0.f, v.w * s);
-                if (MODE == kSuperSymmetric) sm.csq[w][0][lane] = (v.w * s) * (v.w * s);
-                __syncwarp();
-#pragma unroll 1
-                for (int i = 0; 8 * (i >> 1) < nb; ++i) {  // tile i & 1 of the candidates, i >> 1 of the queries
-                    uint32_t cf[4];
-                    load_matrix(cf, crow ^ (32u * (i & 1)));
-                    const uint32_t* qf = reinterpret_cast<const uint32_t*>(&sm.query[w][8 * (i >> 1) + g][0]);
-                    float d[4];
-                    mma_16x8(d, cf, qf[tq], qf[4 + tq]);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int q = 8 * (i >> 1) + 2 * tq + (j & 1), k = 32 * c + 4 * g + 2 * (i & 1) + (j >> 1);
-                        float r = d[j];
-                        if (MODE == kSuperSymmetric) r -= fmaxf(sm.qsq[w][q], sm.csq[w][0][k & 31]);
-                        if (!(fabsf(r) <= band) || q >= nb || k >= wn) continue;
-                        const int32_t f = atomicAdd(a.num_exact, 1);
-                        const uint2 st = sm.starts[w][k >> 5];
-                        run = (int32_t)st.y + __popc(st.x & ((2u << (k & 31)) - 1u));
-                        if (f < a.nq_total)
-                            a.band_pairs[f] = make_int4(
-                                a.unit_t0[unit] + q, sm.delta[w][run] + w0 + k,
-                                a.rec[unit] + kRecHeader + 2 * R + 1 + ((w0 + k) >> 5) * nb + q, k & 31);
-                        else
-                            full = true;  // the list is
-                    }
-                    __syncwarp();
-                }
-            }
-            // many of them, or no place for them: the window, to be tested again
-            if (marked && __any_sync(0xffffffffu, full) && lane == 0) {
-                // (every place that is claimed is written)
-                const bool named = w0 < (kWalkWin << 16);
-                const int32_t f = named ? atomicAdd(&a.num_exact[2], 1) : 0;
-                if (named && f < a.band_cap)
-                    a.band_windows[f] = ((unsigned long long)(uint32_t)unit << 32) | (uint32_t)(w0 / kWalkWin) << 16 | marked;
-                else
-                    redo = true;
-            }
+            // rare: the pairs inside the band are listed, to be decided after the walk
+            if (marked) redo |= list_band<DIM, PERIODIC, MODE>(a, sm, unit, grp, w0, M, marked, PERIODIC && n.seam, lane, w);
         }
         redo = __any_sync(0xffffffffu, redo);
         // the two chunks of a pair were counted by different lanes; query q's count to lane q
@@ -2760,8 +2801,8 @@ __device__ __forceinline__ void decide_windows(const WalkArgs& a) {
 }
 
 // Resident blocks per SM of the launch after the count walk (registers <= 65536 / (128 * blocks)): a listed window is a
-// chain of reads for one warp, so warps in flight decide (1M lattice points, 3D / 1D: 1.22 / 1.18 ms with five,
-// 1.18 / 1.13 with seven).
+// chain of reads for one warp, so warps in flight decide (1M lattice points in 3D / 1D: 1.22 / 1.18 ms with five, 1.18 /
+// 1.13 with seven).
 constexpr int kStrayBlocks = 7;
 
 // Serial walk for queries whose own cell differs from their group's (one thread per query).  After the count
@@ -3478,7 +3519,7 @@ static int count_impl(const HostBatch& b, const Structure& S, const Scratch& W, 
         const int32_t* ngroups;
         if (b.self) {
             if (packed) {
-                pack_self_queries_kernel<<<grid_for(nq, 256, num_sms() * 8), 256, 0, st>>>(
+                pack_self_queries_kernel<<<grid_for(nq, 256), 256, 0, st>>>(
                     W.table, S.grid, W.query_prefix, C, S.rsidx, nq, W.qsorted, W.qsidx, W.qparams);
                 note_launches(1);
             }
