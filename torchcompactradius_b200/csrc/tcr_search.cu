@@ -2775,8 +2775,7 @@ __device__ __forceinline__ void decide_window_mode(const WalkArgs& a, WalkSmem& 
 }
 
 // The listed windows, one warp each.
-__device__ __forceinline__ void decide_windows(const WalkArgs& a) {
-    const int32_t n = (int32_t)min((int64_t)a.num_exact[2], a.band_cap);
+__device__ __forceinline__ void decide_windows(const WalkArgs& a, int32_t n) {
     if (n == 0) return;
     __shared__ WalkSmem sm;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -2809,19 +2808,20 @@ constexpr int kStrayBlocks = 7;
 // walk also: the pairs inside the product's band (one thread per listed pair, one warp per listed window).
 template <bool EMIT>
 __global__ void __launch_bounds__(kWalkWarps * 32, EMIT ? 1 : kStrayBlocks) stray_kernel(const __grid_constant__ WalkArgs a) {
-    const int32_t ns = *a.num_stray;
+    // (read together: as they are used, each would wait for the work before it)
+    const int32_t ns = *a.num_stray, listed = a.num_exact[0], windows = a.num_exact[2];
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
     // the last launch of a count or an emit leaves the work counters ready for the next emit
     if (blockIdx.x == 0 && threadIdx.x < kWorkCounters) a.work[threadIdx.x] = 0;
     if constexpr (!EMIT) {
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.num_clouds; c += gridDim.x * blockDim.x) {
+        for (int64_t c = threads - 1 - first; c < a.num_clouds; c += threads) {  // (from the end: the first have pairs)
             float qmax;
             const bool any = a.table[c].n_query > 0;
             if (query_limits(a.table[c], a.grid[c], a.qparams[c], qmax) & any) atomicAdd(a.exact_clouds, 1);
         }
-        const int64_t nband = min((int64_t)*a.num_exact, a.nq_total);
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nband; i += (int64_t)gridDim.x * blockDim.x)
-            decide_band_pair(a, a.band_pairs[i]);
-        decide_windows(a);
+        const int64_t nband = min((int64_t)listed, a.nq_total);
+        for (int64_t i = first; i < nband; i += threads) decide_band_pair(a, a.band_pairs[i]);
+        decide_windows(a, (int32_t)min((int64_t)windows, a.band_cap));
     }
     for (int32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
         const int32_t t = a.stray[s];
