@@ -60,8 +60,8 @@ typedef struct tcr_search_desc {
                                  skipped, wrapped stencil cells on periodic dims with < 3 cells visited
                                  once (the reference visits them twice and reports those pairs twice) */
     /* Tuning of this search (no reference counterpart; 0 keeps the default; no setting changes a
-     * result): queries per work unit of the walks -- 32, 16 or 8 -- and resident walk blocks per
-     * SM (1..64).  tcr_count and tcr_emit of one search must be given the same unit_queries. */
+     * result): queries per work unit of the walks -- 32, 16 or 8 -- and blocks per SM of
+     * the walks' grid (1..64).  tcr_count and tcr_emit of one search must be given the same unit_queries. */
     int32_t unit_queries;
     int32_t walk_blocks_per_sm;
     int32_t reserved;
@@ -165,7 +165,8 @@ int tcr_search_sizes(int64_t n_query, int64_t n_ref, int32_t dim, int64_t* struc
  *   CELL_COORDS   int32 [3*C] integer cell coordinates
  *   CELL_BUCKET   int32 [C] reference hash of the coordinates mod hashMapLength
  *   MAP           uint64 [cap] entries (lin << 32 | cell), empty = ~0: at slot lin when every point lies in a
- *                 grid of no more cells than slots, else an open-addressing table */
+ *                 grid of no more cells than slots, else an open-addressing table.  The placement is the
+ *                 search's own and may change; to look a cell up, search CELL_LIN, which ascends */
 #define TCR_STRUCT_GRID 0
 #define TCR_STRUCT_NUM_CELLS 1
 #define TCR_STRUCT_SORTED_POINTS 2

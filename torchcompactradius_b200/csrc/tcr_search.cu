@@ -60,13 +60,13 @@ static inline int64_t hash_capacity(int64_t n_ref, int64_t min_cap) {
 constexpr int64_t kSingleMapMin = 1024;  // one search
 constexpr int64_t kBatchMapMin = 64;     // per cloud of a batch
 // Work counters: [0] count walk, [1] emit walk, [2 + cls] / [8 + cls] the count / emit walk of
-// one cloud class (cls = dim * 2 + periodic, 2..7) in a batch that mixes classes, [16 + the same]
-// for the count walk of the units recorded window by window.
+// one cloud class (cls = dim * 2 + periodic, 2..7) in a batch that mixes classes, [30] the expansion.
 constexpr int kWorkCounters = 32;
 constexpr int kExpandCounter = 30;  // the record expansion
 
 // Default tuning of a search (tcr_search_desc / tcr_batch_desc unit_queries and walk_blocks_per_sm):
-// queries per work unit and resident walk blocks per SM.  Neither changes a result: a query's
+// queries per work unit and blocks per SM of the walk's grid (the count walk has six or seven of them
+// resident; the others take over as those end).  Neither changes a result: a query's
 // candidates and their order do not depend on how queries are grouped into units.
 constexpr int kDefaultUnitQueries = 32;
 constexpr int kDefaultWalkBlocksPerSM = 12;
@@ -1086,7 +1086,7 @@ constexpr float kMmaFar = 60000.0f;
 // Lanes with a pair inside the band, over the chunks of a window, from which on the window is listed as a whole, if
 // they are also one a pair of chunks; fewer list their pairs.  A random cloud's window has one at most nearly always,
 // and 0.3 on average where 32 queries meet 16 pairs of chunks (20k points in 4^3 periodic cells: 654 us when four
-// lanes there listed the window, which takes one warp 30 us); a lattice's has four even in 1D (1M points: 1.15 ms,
+// lanes there listed the window, which takes one warp 30 us); a lattice's has four even in 1D (1M points: 1.18 ms,
 // 1.45 when eight were asked for).
 constexpr int kBandLanes = 4;
 
@@ -1381,13 +1381,12 @@ constexpr int kWalkMinBlocks = TCR_WALK_MIN_BLOCKS;
 constexpr int kWalkMinBlocksPeriodic = TCR_WALK_MIN_BLOCKS_PERIODIC;
 
 // Record of a staged unit in the staging list (int32 words):
-//   [0] chunks of 32 candidates   [1] R, candidate runs   [2] nb, queries   [3] 0
+//   [0] chunks of 32 candidates   [1] R, candidate runs   [2] nb, queries   [3] 0 (unused)
 //   [4, 4 + R)          first sorted index of each run
 //   [4 + R, 5 + 2R)     candidate prefix of each run; entry R is the unit's candidate count M
 //   [5 + 2R, ...)       hit masks, chunk-major: word c * nb + q, bit j set when query q meets
 //                       candidate 32 c + j
-// A run is a stretch of consecutive sorted points: stencil cells whose ranges continue each other
-// (the row neighbours of a linear-order grid) merge into one.
+// A run is a stretch of consecutive sorted points: one non-empty stencil cell, so R is at most 27.
 constexpr int kRecHeader = 4;
 __host__ __device__ __forceinline__ int64_t record_words(int32_t runs, int32_t nchunks, int32_t nb) {
     return kRecHeader + 2 * (int64_t)runs + 1 + (int64_t)nchunks * nb;
@@ -1513,7 +1512,7 @@ __device__ __forceinline__ uint32_t chunk_hits(const WrapCtx& wc, const float4* 
 // products, each at most E = (|Q| + thr + ..)^2, aligned and summed in about 24 bits (<= 16 * 2^-24 E;
 // measured 2^-21.4 of the largest product), dropped lo*lo terms and the halves' rounding (<= 8e-7 E).
 // kMmaBand = 4e-6 covers the sum twice (measured over random cells: 1.7e-7 E).  The pairs inside the band
-// (three in a thousand queries have one) are listed and decided exactly after the walk.
+// (three in a thousand queries have one) are listed, alone or as a window, and decided exactly after the walk.
 __device__ __forceinline__ uint32_t h2bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 // (a, b) as float16 pairs: hi = fl16(a, b), lo = fl16((a, b) - hi).
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
@@ -1731,7 +1730,7 @@ struct FixSmem {
 static_assert(sizeof(FixSmem) <= sizeof(uint4) * 2 * 2 * 32, "fits the fragments of one warp");
 
 // A unit the product did not take: a periodic cloud with so few cells that differences wrap, supports
-// outside the fast test's range, points far outside their cell.  One candidate per lane against every
+// outside the fast test's range, points far outside their cell, more windows at the threshold than can be listed.  One candidate per lane against every
 // query in float32; a chunk with a pair inside the float32 band once more with those pairs decided by
 // the reference's exact test; the hit bits transposed into the masks.  Out of line, at the unit's end, so
 // that its registers do not cost the main loop spills.
@@ -3058,7 +3057,7 @@ struct HostBatch {
     int32_t* lin_out = nullptr;         // receives the linear cell of every sorted reference point
     int32_t* order_out = nullptr;       // receives the input index of every sorted reference point
     int unit_cap = kDefaultUnitQueries;           // queries per work unit
-    int walk_bps = kDefaultWalkBlocksPerSM;       // resident walk blocks per SM
+    int walk_bps = kDefaultWalkBlocksPerSM;       // blocks per SM of the walk's grid
 };
 
 // The descriptors' tuning fields (0: default).

@@ -55,7 +55,7 @@ def _to_host(tensors):
 _warned_f64 = False
 
 
-def _as_f32(t, device, shape=None):
+def _as_f32(t, device):
     """Positions and supports as contiguous float32 on the device.  The search computes in float32
     (the reference's float path); a float64 input is rounded to float32 first, with one warning per
     process, since the reference searches float64 inputs in double and pairs whose distance lies

@@ -6,7 +6,7 @@ their order do not depend on them):
 * queries per work unit -- 32, 16 or 8.  A unit is one warp; with fewer queries per unit each
   query gets 2 or 4 lanes (the candidate streams of the walk), which pays for sparse clouds whose
   cells hold few points and costs more stencil look-ups for dense ones;
-* resident walk blocks per SM -- the size of the persistent walk grid;
+* walk blocks per SM -- the size of the persistent walk grid;
 * the cell-size multiplier of single searches (``cell_scales``): cells m times the largest
   threshold on the exact clamped grid, which pays for sparse clouds whose reference-size cells hold
   few points.  Its pair set is the reference's whenever every point lies inside the domain on its
