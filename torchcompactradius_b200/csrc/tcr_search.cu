@@ -2625,6 +2625,7 @@ __device__ __forceinline__ void decide_band_pair(const WalkArgs& a, const int4& 
     if (!TCR_GUARD(p.x, a.nq_total) || !TCR_GUARD(p.y, a.nr_total) || !TCR_GUARD(p.z, a.stage_cap)) return;
     const int32_t qorig = a.qsidx[p.x];
     const CloudParams& cp = a.table[cloud_of(a.query_prefix, a.num_clouds, qorig)];
+    const bool was = ((uint32_t)a.stage[p.z] >> (p.w & 31)) & 1u;
     bool in;
     if (a.f64.qpos) {
         in = f64_pair_decide(a.f64, cp.dim, cp.periodic_mask, a.mode, qorig - (a.local_index ? cp.query_base : 0), p.y);
@@ -2637,6 +2638,7 @@ __device__ __forceinline__ void decide_band_pair(const WalkArgs& a, const int4& 
         const float4 q = a.qsorted[p.x], c = a.rsorted[p.y];
         in = exact_pair_test(xc, q, q.w, c, c.w);
     }
+    if (in == was) return;  // (nearly always)
     if (const int change = set_hit(reinterpret_cast<uint32_t*>(&a.stage[p.z]), p.w & 31, in)) atomicAdd(&a.counts[qorig], change);
 }
 
